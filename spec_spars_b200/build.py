@@ -17,7 +17,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler",
           "--expt-relaxed-constexpr", "-Xptxas", "-O3"]
 # Translation units whose results must be bit-identical to the CPU oracle: no FMA contraction.
 EXACT = {"ssp_graph.cu", "ssp_sketch.cu", "ssp_factor.cu", "ssp_sample.cu", "ssp_noalloc.cu"}
-SOURCES = ["ssp_util.cu", "ssp_graph.cu", "ssp_sketch.cu", "ssp_factor.cu", "ssp_pcg.cu", "ssp_sample.cu",
+SOURCES = ["ssp_util.cu", "ssp_graph.cu", "ssp_sketch.cu", "ssp_factor.cu", "ssp_tail.cu", "ssp_pcg.cu", "ssp_sample.cu",
            "ssp_autotune.cu", "ssp_noalloc.cu", "ssp_quality.cu", "ssp_mtxio.cu", "ssp_api.cu", "ssp_host.cpp",
            "ssp_server.cpp"]
 HEADERS = ["ssp_internal.cuh", "ssp_sort.cuh", "ssp_host.h", "ssp_decimal.cuh"]

@@ -638,106 +638,6 @@ __global__ void k_collect_live_range(int64_t v0, int64_t v1, const int32_t* leve
         if (level[v] < 0) rem[atomicAdd((unsigned long long*)cnt, 1ull)] = (int32_t)v;
 }
 
-// ---------------------------------------------------------------- solve schedule
-// Thin-level runs (DevFactor::SolveRun) and their step schedules.  Row t of a run depends, in the forward
-// solve, on the rows of the same run that its L row reads (lower levels), and in the backward solve on the
-// rows its L column reaches (higher levels); its step is one more than the deepest of those (0 if none).
-// Steps list the run's storage rows by (step, storage row).  Built on the host from the runs' own rows.
-static void build_solve_schedule(Context& C, DevFactor& out, const std::vector<int64_t>& lp, const std::string& tag) {
-    const int32_t NL = out.num_levels;
-    out.runs.clear();
-    for (int32_t l = 0; l < NL;) {
-        int32_t r = l;
-        while (r < NL && lp[r + 1] - lp[r] <= THIN_ROWS) r++;
-        if (r - l >= 2) {
-            out.runs.push_back({l, r, 0, 0, 0, 0});
-            l = r;
-        } else {
-            l++;
-        }
-    }
-    if (out.runs.empty()) return;
-    // the runs' vertices, row pointers and entries
-    struct Host {
-        std::vector<int32_t> vert, fidx, bidx;
-        std::vector<int64_t> fptr, bptr;
-    };
-    std::vector<Host> h(out.runs.size());
-    auto get = [&](void* dst, const void* src, size_t bytes) {
-        if (bytes) SSP_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, C.stream));
-    };
-    for (size_t u = 0; u < out.runs.size(); u++) {
-        const int64_t r0 = lp[out.runs[u].l0], r1 = lp[out.runs[u].l1];
-        h[u].vert.resize(r1 - r0);
-        h[u].fptr.resize(r1 - r0 + 1);
-        h[u].bptr.resize(r1 - r0 + 1);
-        get(h[u].vert.data(), out.level_rows + r0, sizeof(int32_t) * (r1 - r0));
-        get(h[u].fptr.data(), out.prow_ptr + r0, sizeof(int64_t) * (r1 - r0 + 1));
-        get(h[u].bptr.data(), out.pcol_ptr + r0, sizeof(int64_t) * (r1 - r0 + 1));
-    }
-    SSP_CUDA(cudaStreamSynchronize(C.stream));
-    for (auto& x : h) {
-        x.fidx.resize(x.fptr.back() - x.fptr.front());
-        x.bidx.resize(x.bptr.back() - x.bptr.front());
-        get(x.fidx.data(), out.prow_idx + x.fptr.front(), sizeof(int32_t) * x.fidx.size());
-        get(x.bidx.data(), out.pcol_idx + x.bptr.front(), sizeof(int32_t) * x.bidx.size());
-    }
-    SSP_CUDA(cudaStreamSynchronize(C.stream));
-    std::vector<int32_t> fsched, bsched, fstep{0}, bstep{0};
-    std::vector<int32_t> where(out.n, -1);  // vertex -> local row of the run being scheduled
-    // depth of every local row, then a counting sort by depth
-    auto schedule = [&](const Host& x, int64_t r0, bool fwd, std::vector<int32_t>& sched, std::vector<int32_t>& step,
-                        int32_t& s0, int32_t& s1) {
-        const int32_t R = (int32_t)x.vert.size();
-        const auto& ptr = fwd ? x.fptr : x.bptr;
-        const auto& idx = fwd ? x.fidx : x.bidx;
-        std::vector<int32_t> d(R, 0);
-        int32_t depth = 0;
-        for (int32_t k = 0; k < R; k++) {
-            const int32_t t = fwd ? k : R - 1 - k;  // dependencies come first in this order
-            int32_t dt = 0;
-            for (int64_t e = ptr[t] - ptr[0]; e < ptr[t + 1] - ptr[0]; e++) {
-                const int32_t j = where[idx[e]];
-                if (j < 0) continue;
-                if (fwd ? j >= t : j <= t) throw Error(SSP_ERR_INVALID, "factor: solve schedule out of order");
-                dt = std::max(dt, d[j] + 1);
-            }
-            d[t] = dt;
-            depth = std::max(depth, dt + 1);
-        }
-        std::vector<int32_t> cnt(depth + 1, 0);
-        for (int32_t t = 0; t < R; t++) cnt[d[t] + 1]++;
-        for (int32_t s = 0; s < depth; s++) cnt[s + 1] += cnt[s];
-        const size_t base = sched.size();
-        sched.resize(base + R);
-        for (int32_t t = 0; t < R; t++) sched[base + cnt[d[t]]++] = (int32_t)(r0 + t);
-        s0 = (int32_t)step.size() - 1;
-        int32_t acc = (int32_t)base;
-        std::vector<int32_t> sz(depth, 0);
-        for (int32_t t = 0; t < R; t++) sz[d[t]]++;
-        for (int32_t s = 0; s < depth; s++) step.push_back(acc += sz[s]);
-        s1 = (int32_t)step.size() - 1;
-    };
-    for (size_t u = 0; u < out.runs.size(); u++) {
-        auto& run = out.runs[u];
-        const int64_t r0 = lp[run.l0];
-        for (int32_t t = 0; t < (int32_t)h[u].vert.size(); t++) where[h[u].vert[t]] = t;
-        schedule(h[u], r0, true, fsched, fstep, run.fs0, run.fs1);
-        schedule(h[u], r0, false, bsched, bstep, run.bs0, run.bs1);
-        for (int32_t v : h[u].vert) where[v] = -1;
-    }
-    auto put = [&](const std::vector<int32_t>& v, const char* name) {
-        int32_t* d = C.ws.get_t<int32_t>(tag + "_" + name, v.size());
-        SSP_CUDA(cudaMemcpyAsync(d, v.data(), sizeof(int32_t) * v.size(), cudaMemcpyHostToDevice, C.stream));
-        return d;
-    };
-    out.fsched = put(fsched, "fsched");
-    out.fstep = put(fstep, "fstep");
-    out.bsched = put(bsched, "bsched");
-    out.bstep = put(bstep, "bstep");
-    SSP_CUDA(cudaStreamSynchronize(C.stream));
-}
-
 // ---------------------------------------------------------------- dense tail
 __global__ void k_collect_live(int64_t n, const int32_t* level, int32_t* rem, int64_t* cnt) {
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
@@ -978,11 +878,12 @@ __global__ void k_level_count(int64_t n, const int32_t* level, int32_t* lvcnt) {
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
         atomicAdd(&lvcnt[level[v]], 1);
 }
-__global__ void k_level_scatter(int64_t n, const int32_t* level, const int64_t* lvptr, int32_t* cursor,
-                                int32_t* rows) {
+// sort key of a vertex: its level, then the length of its row (or column) of L, longest first
+__global__ void k_level_keys(int64_t n, const int32_t* level, const int64_t* ptr, uint64_t* key, int32_t* v_out) {
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-        int32_t l = level[v];
-        rows[lvptr[l] + atomicAdd(&cursor[l], 1)] = (int32_t)v;
+        const int64_t len = ptr[v + 1] - ptr[v];
+        key[v] = ((uint64_t)(uint32_t)level[v] << 8) | (uint64_t)(255 - (len < 255 ? len : 255));
+        v_out[v] = (int32_t)v;
     }
 }
 __global__ void k_i64_to_i32(int64_t n, const int64_t* a, int32_t* b) {
@@ -1050,15 +951,20 @@ __global__ void k_perm_count(int64_t n, const int32_t* perm, const int64_t* ptr,
     }
 }
 __global__ void k_perm_copy(int64_t n, const int32_t* perm, const int64_t* ptr, const int32_t* idx, const double* val,
-                            const int64_t* pptr, int32_t* pidx, double* pval) {
+                            const int64_t* pptr, int32_t* pidx, double* pval, FactorRow* prow,
+                            FactorEnt<double>* pent) {
     const int lane = threadIdx.x & 31;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nw) {
         const int32_t v = perm[i];
         const int64_t s = ptr[v], d = pptr[i], c = ptr[v + 1] - s;
+        if (lane == 0) prow[i] = FactorRow{v, (int32_t)c, d};
         for (int64_t q = lane; q < c; q += 32) {
-            pidx[d + q] = idx[s + q];
-            pval[d + q] = val[s + q];
+            const int32_t u = idx[s + q];
+            const double x = val[s + q];
+            pidx[d + q] = u;
+            pval[d + q] = x;
+            pent[d + q] = FactorEnt<double>{x, u};
         }
     }
 }
@@ -1505,15 +1411,28 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
     // level lists
     const int32_t NL = out.num_levels;
     int32_t* lvcnt = W.get_t<int32_t>(nm("lvcnt"), NL + 1);
-    int32_t* lvcur = W.get_t<int32_t>(nm("lvcur"), NL + 1);
     SSP_CUDA(cudaMemsetAsync(lvcnt, 0, sizeof(int32_t) * (NL + 1), C.stream));
-    SSP_CUDA(cudaMemsetAsync(lvcur, 0, sizeof(int32_t) * (NL + 1), C.stream));
     k_level_count<<<grid_for(n, T256), T256, 0, C.stream>>>(n, F.level, lvcnt);
     SSP_CHECK_LAUNCH();
     int64_t* lvptr = W.get_t<int64_t>(nm("lvptr64"), NL + 1);
     exclusive_scan_i32_to_i64(C, lvcnt, lvptr, NL + 1, nullptr);
     out.level_rows = W.get_t<int32_t>(nm("level_rows"), n);
-    k_level_scatter<<<grid_for(n, T256), T256, 0, C.stream>>>(n, F.level, lvptr, lvcur, out.level_rows);
+    // a level's vertices by the length of their rows (columns) and then by id: neighbours in the order have about as much
+    // work, and everything laid out from here on (and the order in which the solves add a row up) is the same in every run
+    out.level_cols = W.get_t<int32_t>(nm("level_cols"), n);
+    {
+        uint64_t* key = W.get_t<uint64_t>(nm("lvkey"), n);
+        uint64_t* tkey = W.get_t<uint64_t>(nm("lvkey2"), n);
+        int32_t* tval = W.get_t<int32_t>(nm("lvval2"), n);
+        int bits = 9;
+        while (bits < 40 && (int64_t(256) << (bits - 8)) < (int64_t)NL * 256) bits++;
+        for (int f = 0; f < 2; f++) {
+            int32_t* order = f == 0 ? out.level_rows : out.level_cols;
+            k_level_keys<<<grid_for(n, T256), T256, 0, C.stream>>>(n, F.level, f == 0 ? out.row_ptr : out.col_ptr, key, order);
+            SSP_CHECK_LAUNCH();
+            radix_sort_u64(C, key, order, n, bits, tkey, tval);
+        }
+    }
     out.level_ptr_d = W.get_t<int32_t>(nm("level_ptr"), NL + 1);
     k_i64_to_i32<<<grid_for(NL + 1, T256), T256, 0, C.stream>>>(NL + 1, lvptr, out.level_ptr_d);
     SSP_CHECK_LAUNCH();
@@ -1528,20 +1447,22 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
     // storage-order row and column forms + per-level chunk lists
     {
         int32_t* cnt = W.get_t<int32_t>(nm("permcnt"), n + 1);
-        auto build = [&](const int64_t* ptr, const int32_t* idx, const double* val, const char* tagp,
+        auto build = [&](const int32_t* order, const int64_t* ptr, const int32_t* idx, const double* val, const char* tagp,
                          int64_t** pptr, int32_t** pidx, double** pval, int32_t** chunks,
-                         std::vector<int32_t>& chunk_lvl) {
+                         std::vector<int32_t>& chunk_lvl, std::vector<int64_t>& hp, FactorRow** prow, FactorEnt<double>** pent) {
             *pptr = W.get_t<int64_t>(nm(tagp) + "_ptr", n + 1);
-            k_perm_count<<<grid_for(n, T256), T256, 0, C.stream>>>(n, out.level_rows, ptr, cnt);
+            k_perm_count<<<grid_for(n, T256), T256, 0, C.stream>>>(n, order, ptr, cnt);
             SSP_CUDA(cudaMemsetAsync(cnt + n, 0, sizeof(int32_t), C.stream));
             exclusive_scan_i32_to_i64(C, cnt, *pptr, n + 1, nullptr);
             *pidx = W.get_t<int32_t>(nm(tagp) + "_idx", out.nnz + 1);
             *pval = W.get_t<double>(nm(tagp) + "_val", out.nnz + 1);
-            k_perm_copy<<<grid_for(n * 32, T256, 148 * 64), T256, 0, C.stream>>>(n, out.level_rows, ptr, idx, val,
-                                                                                *pptr, *pidx, *pval);
+            *prow = W.get_t<FactorRow>(nm(tagp) + "_row", n);
+            *pent = W.get_t<FactorEnt<double>>(nm(tagp) + "_ent", out.nnz + 1);
+            k_perm_copy<<<grid_for(n * 32, T256, 148 * 64), T256, 0, C.stream>>>(n, order, ptr, idx, val,
+                                                                                *pptr, *pidx, *pval, *prow, *pent);
             SSP_CHECK_LAUNCH();
             C.kernels_launched += 2;
-            std::vector<int64_t> hp(n + 1);
+            hp.resize(n + 1);
             SSP_CUDA(cudaMemcpyAsync(hp.data(), *pptr, sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToHost, C.stream));
             SSP_CUDA(cudaStreamSynchronize(C.stream));
             const int64_t last_nnz = NL > 0 ? hp[lp[NL]] - hp[lp[NL - 1]] : 0;
@@ -1560,12 +1481,12 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
                                      C.stream));
             SSP_CUDA(cudaStreamSynchronize(C.stream));
         };
-        build(out.row_ptr, out.row_idx, out.row_val, "prow", &out.prow_ptr, &out.prow_idx, &out.prow_val,
-              &out.fchunk, out.fchunk_lvl);
-        build(out.col_ptr, out.col_idx, out.col_val, "pcol", &out.pcol_ptr, &out.pcol_idx, &out.pcol_val,
-              &out.bchunk, out.bchunk_lvl);
+        build(out.level_rows, out.row_ptr, out.row_idx, out.row_val, "prow", &out.prow_ptr, &out.prow_idx, &out.prow_val,
+              &out.fchunk, out.fchunk_lvl, out.hfptr, &out.frow, &out.fent);
+        build(out.level_cols, out.col_ptr, out.col_idx, out.col_val, "pcol", &out.pcol_ptr, &out.pcol_idx, &out.pcol_val,
+              &out.bchunk, out.bchunk_lvl, out.hbptr, &out.brow, &out.bent);
     }
-    build_solve_schedule(C, out, lp, tag);
+    build_tail(C, out, T, T > 0 ? W.get_t<double>(nm("W"), (size_t)T * T) : nullptr, tag);
 }
 
 }  // namespace ssp

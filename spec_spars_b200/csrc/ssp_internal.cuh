@@ -339,6 +339,16 @@ void sketch_device_part(Context& C, const DevGraph& G, int64_t v0, int64_t nv, i
                         uint64_t seed, int uniform, double* Y, int64_t ldy, int tile_major, int32_t col_lo = 0);
 
 // a7: factor
+// a row of the factor's storage order and an entry with its value beside it, each one aligned load
+struct __align__(16) FactorRow {
+    int32_t u, cnt;  // vertex, entries
+    int64_t e0;      // first entry
+};
+template <class T>
+struct __align__(2 * sizeof(T)) FactorEnt {
+    T v;
+    int32_t idx;
+};
 struct DevFactor {
     int64_t n = 0;
     int64_t nnz = 0;
@@ -353,7 +363,9 @@ struct DevFactor {
     double* D = nullptr;
     int32_t* level = nullptr;       // [n]
     int32_t* level_ptr_d = nullptr; // [num_levels+1] (device)
-    int32_t* level_rows = nullptr;  // [n] vertices grouped by level ("storage order")
+    int32_t* level_rows = nullptr;  // [n] vertices grouped by level ("storage order"), a level's by the length of
+                                    // their L rows, longest first, then by id
+    int32_t* level_cols = nullptr;  // the same by the length of their columns (storage order of the column form)
     std::vector<int32_t> level_ptr; // host copy
     // L rows (forward solve) and columns (backward solve) re-laid in storage order, so that the rows of
     // a level are contiguous; chunk lists split each level into row-aligned pieces of bounded size
@@ -363,6 +375,10 @@ struct DevFactor {
     int64_t* pcol_ptr = nullptr;
     int32_t* pcol_idx = nullptr;
     double* pcol_val = nullptr;
+    FactorRow* frow = nullptr;           // the same rows, entries and values for the walked levels of the solves
+    FactorRow* brow = nullptr;
+    FactorEnt<double>* fent = nullptr;
+    FactorEnt<double>* bent = nullptr;
     int32_t* fchunk = nullptr;           // device chunk starts (storage rows) for the forward solve
     int32_t* bchunk = nullptr;           // ... for the backward solve
     std::vector<int32_t> fchunk_lvl;     // [num_levels+1] chunk index range per level
@@ -379,23 +395,25 @@ struct DevFactor {
     // forward solve of that level finish its rows (z = y / D) and the backward solve skip it.
     int64_t last_fwd_nnz = -1;
     int64_t last_bwd_nnz = -1;
-    // Solve schedule.  Maximal runs of consecutive thin levels (at most THIN_ROWS rows each, two or more
-    // levels) are solved by one launch that walks "steps": the run's rows grouped by their dependency depth
-    // inside the run (a row's depth is one more than the deepest row of the same run it reads), which is
-    // often far smaller than the run's level count (the dense tail eliminates one vertex per level).  The
-    // factor and its levels are unchanged; only the order rows are solved in differs, and each row's own
-    // sum is formed the same way whatever step it lands in.
-    struct SolveRun {
-        int32_t l0, l1;  // levels [l0, l1)
-        int32_t fs0, fs1, bs0, bs1;  // step ranges of the forward and backward schedules
-    };
-    std::vector<SolveRun> runs;
-    int32_t* fsched = nullptr;  // storage rows of all runs, forward step order
-    int32_t* fstep = nullptr;   // step pointers into fsched
-    int32_t* bsched = nullptr;
-    int32_t* bstep = nullptr;
+    std::vector<int64_t> hfptr, hbptr;  // prow_ptr and pcol_ptr on the host
+    // The dense tail (dense_levels > 0): the last tail_rows storage rows, one per level from level tail_l0 on.  linv is
+    // the inverse of their unit lower triangular block of L (row-major, tail_rows x tail_rows); tin_* are the
+    // entries of their rows in earlier levels, with their own row pointers and chunks (ssp_tail.cu).
+    int32_t tail_rows = 0, tail_l0 = 0;
+    double* linv = nullptr;
+    int64_t* tin_ptr = nullptr;
+    int32_t* tin_idx = nullptr;
+    double* tin_val = nullptr;
+    int64_t tin_nnz = 0;
+    int32_t* tchunk = nullptr;
+    int32_t ntchunk = 0;
 };
-constexpr int THIN_ROWS = 64;  // a level with at most this many rows is "thin"
+// the tail's inverse and split rows from the storage-order row form; X: scratch of T x T doubles
+void build_tail(Context& C, DevFactor& F, int64_t T, double* X, const std::string& tag);
+// the tail of one application in y (tile-major), its rows already reduced by the earlier levels; tmp: T x ld values.
+// Returns the kernels launched.
+template <class T>
+int64_t launch_tail(Context& C, const DevFactor& F, const T* linv, const T* D, T* y, T* tmp, int64_t ntiles);
 struct FactorOptions {
     uint64_t seed = 0;
     int64_t dense_threshold = 4096;

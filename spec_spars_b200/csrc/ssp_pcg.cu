@@ -370,6 +370,13 @@ __global__ void k_f2d(int64_t count, const float* __restrict__ src, double* __re
         dst[i] = (double)src[i];
 }
 
+__global__ void k_ent_f32(int64_t count, const FactorEnt<double>* __restrict__ src, FactorEnt<float>* __restrict__ dst) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
+        const FactorEnt<double> e = src[i];
+        dst[i] = FactorEnt<float>{(float)e.v, e.idx};
+    }
+}
+
 // inner right-hand side: the FP64 residual of the columns still active, rounded to T; zero elsewhere
 // (runs in place when T is double)
 template <class T>
@@ -570,12 +577,9 @@ struct LoopGraph {
 enum { M_SPMM = 0, M_FWD = 1, M_BWD = 2, M_SPMM_ACC = 3, M_FWD_LAST = 4 };
 constexpr int CH_THREADS = 256;
 // independent gathers in flight per lane in the chunk kernels (powers of two).  Measured on B200 at ER n = 1M,
-// k = 1327: 8 for the SpMM takes it from 48 to 38 ms; the level solves are faster with 4 (19 against 22 ms).
+// k = 1327: 8 for the SpMM takes it from 48 to 38 ms.
 #ifndef SSP_GATHER_UNROLL_SPMM
 #define SSP_GATHER_UNROLL_SPMM 8
-#endif
-#ifndef SSP_GATHER_UNROLL_SOLVE
-#define SSP_GATHER_UNROLL_SOLVE 4
 #endif
 constexpr int CH_WARPS = CH_THREADS / 32;
 constexpr int MINB_SPMM = 6, MINB_FWD = 6, MINB_BWD = 5;
@@ -601,6 +605,69 @@ __device__ __forceinline__ void chunk_epilogue(T* out, const T* aux, const T* xt
         const T yu = out[o];
         out[o] = (d != (T)0 ? yu / d : yu) - acc;
     }
+}
+
+// Row sums of the triangular solves.  A row's entries are summed in segments of ROW_SEG: entry i of a segment goes to
+// accumulator i mod 4 (in entry order), the four are combined as (a0 + a1) + (a2 + a3), and the segments' sums are
+// added in order.  Every launch width forms a row this way -- one lane per (row, column), or the entry slots of a warp
+// for a row longer than a chunk -- so the values do not depend on it.
+constexpr int ROW_SEG = 64;
+
+// one lane, entries [q0, q1) of staged or global index and value arrays.  The last entries of a row are loaded under
+// predicates, all at once: a row of three entries costs one gather latency, not three.
+template <class T, class I>
+__device__ __forceinline__ T row_sum_lane(const int32_t* si, const T* sv, I q0, I q1, const T* xt) {
+    T tot = 0;
+    for (I s = q0; s < q1; s += ROW_SEG) {
+        const I e = min(s + (I)ROW_SEG, q1);
+        T a[4] = {0, 0, 0, 0};
+        I q = s;
+        for (; q + 3 < e; q += 4) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) a[u] += sv[q + u] * xt[(int64_t)si[q + u] * TILE];
+        }
+        if (q < e) {
+            T x[3];
+#pragma unroll
+            for (int u = 0; u < 3; u++) x[u] = q + u < e ? xt[(int64_t)si[q + u] * TILE] : (T)0;
+#pragma unroll
+            for (int u = 0; u < 3; u++)
+                if (q + u < e) a[u] += sv[q + u] * x[u];
+        }
+        tot += (a[0] + a[1]) + (a[2] + a[3]);
+    }
+    return tot;
+}
+
+// one segment [s, e) of staged entries by the 32 / W slots of a full warp (W = 8, 16 or 32); every lane of a column
+// gets the sum
+template <class T, int W>
+__device__ __forceinline__ T seg_sum_slots(const int32_t* si, const T* sv, int s, int e, const T* xt, int slot) {
+    constexpr int SLOTS = 32 / W, NA = 4 / SLOTS, U = NA == 1 ? 4 : 4 / NA;
+    static_assert(SLOTS <= 4, "columns per row below 8");
+    T a[NA];
+#pragma unroll
+    for (int j = 0; j < NA; j++) a[j] = 0;
+    for (int q = s + slot; q < e; q += 4 * U) {
+        T x[U * NA];
+#pragma unroll
+        for (int u = 0; u < U * NA; u++) {
+            const int p = q + SLOTS * u;
+            x[u] = p < e ? xt[(int64_t)si[p] * TILE] : (T)0;
+        }
+#pragma unroll
+        for (int u = 0; u < U * NA; u++) {
+            const int p = q + SLOTS * u;
+            if (p < e) a[u % NA] += sv[p] * x[u];
+        }
+    }
+#pragma unroll
+    for (int o = W; o < 32; o <<= 1)
+#pragma unroll
+        for (int j = 0; j < NA; j++) a[j] += __shfl_xor_sync(0xffffffffu, a[j], o);
+    if constexpr (NA == 4) return (a[0] + a[1]) + (a[2] + a[3]);
+    else if constexpr (NA == 2) return a[0] + a[1];
+    else return a[0];
 }
 
 // Grid: x over chunks, y over (tile, sub-tile): a tile's TILE columns are covered by nsub = TILE / W warps'
@@ -630,7 +697,6 @@ __global__ void __launch_bounds__(CH_THREADS, MINB)
     T* sv = s_val[w];
     int32_t* sp = s_ptr[w];
     int32_t* sr = s_row[w];
-    constexpr int SLOTS_W = 32 / W;
     constexpr bool SPMM = MODE == M_SPMM || MODE == M_SPMM_ACC;
     const bool want_dot = SPMM && part != nullptr;
     double dot = 0.0;  // SpMM: per-lane partial of p.q for column (lane % W)
@@ -656,62 +722,79 @@ __global__ void __launch_bounds__(CH_THREADS, MINB)
                 const bool on = row_on(ra, vrow, t);
                 const bool live = on && t * TILE + col < kcols;
                 const int32_t q0 = sp[rr], q1 = live ? sp[rr + 1] : q0;
-                // GATHER_UNROLL independent accumulators, summed as a pairwise tree
-                constexpr int GATHER_UNROLL = SPMM ? SSP_GATHER_UNROLL_SPMM : SSP_GATHER_UNROLL_SOLVE;
-                T a[GATHER_UNROLL];
+                T sum;
+                if constexpr (SPMM) {
+                    // GATHER_UNROLL independent accumulators, summed as a pairwise tree
+                    constexpr int GATHER_UNROLL = SSP_GATHER_UNROLL_SPMM;
+                    T a[GATHER_UNROLL];
 #pragma unroll
-                for (int u = 0; u < GATHER_UNROLL; u++) a[u] = 0;
-                int32_t q = q0;
-                for (; q + GATHER_UNROLL - 1 < q1; q += GATHER_UNROLL) {
+                    for (int u = 0; u < GATHER_UNROLL; u++) a[u] = 0;
+                    int32_t q = q0;
+                    for (; q + GATHER_UNROLL - 1 < q1; q += GATHER_UNROLL) {
 #pragma unroll
-                    for (int u = 0; u < GATHER_UNROLL; u++) a[u] += sv[q + u] * xt[(int64_t)si[q + u] * TILE + col];
+                        for (int u = 0; u < GATHER_UNROLL; u++)
+                            a[u] += sv[q + u] * xt[(int64_t)si[q + u] * TILE + col];
+                    }
+                    if (GATHER_UNROLL > 4 && q + 3 < q1) {  // short rows (a slab's share of a row) still get 4 in flight
+#pragma unroll
+                        for (int u = 0; u < 4; u++) a[u] += sv[q + u] * xt[(int64_t)si[q + u] * TILE + col];
+                        q += 4;
+                    }
+                    for (; q < q1; q++) a[0] += sv[q] * xt[(int64_t)si[q] * TILE + col];
+#pragma unroll
+                    for (int h = 1; h < GATHER_UNROLL; h <<= 1)
+#pragma unroll
+                        for (int u = 0; u < GATHER_UNROLL; u += 2 * h) a[u] += a[u + h];
+                    sum = a[0];
+                } else {
+                    sum = row_sum_lane<T>(si, sv, q0, q1, xt + col);
                 }
-                if (GATHER_UNROLL > 4 && q + 3 < q1) {  // short rows (a slab's share of a row) still get 4 in flight
-#pragma unroll
-                    for (int u = 0; u < 4; u++) a[u] += sv[q + u] * xt[(int64_t)si[q + u] * TILE + col];
-                    q += 4;
-                }
-                for (; q < q1; q++) a[0] += sv[q] * xt[(int64_t)si[q] * TILE + col];
-#pragma unroll
-                for (int h = 1; h < GATHER_UNROLL; h <<= 1)
-#pragma unroll
-                    for (int u = 0; u < GATHER_UNROLL; u += 2 * h) a[u] += a[u + h];
-                if (on) chunk_epilogue<MODE, T>(out, aux, xt, toff, vrow, col, a[0], dot, want_dot, dlast);
+                if (on) chunk_epilogue<MODE, T>(out, aux, xt, toff, vrow, col, sum, dot, want_dot, dlast);
             }
             __syncwarp();
         } else {
-            // One long row: (32 / W) entry slots x W columns per step.  The sum does not depend on W: entry i
-            // of the row goes to virtual accumulator i mod LONG_ACC (each summed in entry order), and the
-            // accumulators are combined by a fixed tree, highest index bit first.  A lane of slot s holds the
-            // accumulators s + SLOTS_W j; it combines their high bits itself, the slot bits are combined
-            // across lanes afterwards (offset 16 first), so a level solved with any column width W gives
-            // the same values bit for bit -- which lets the launch shapes be chosen by measurement.
-            constexpr int LONG_ACC = 4, NA = LONG_ACC / SLOTS_W;
-            static_assert(NA >= 1 && LONG_ACC % SLOTS_W == 0, "column width below 8");
+            // one long row: (32 / W) entry slots x W columns
             const int slot = lane / W, col = c0 + lane % W;
             const int64_t vr0 = rowmap ? rowmap[r0] : r0;
             const bool on = row_on(ra, vr0, t);
-            const int64_t qe = on && t * TILE + col < kcols ? e1 : e0;
-            T a[NA];
+            const bool live = t * TILE + col < kcols;
+            T acc = 0;
+            if constexpr (SPMM) {
+                constexpr int SLOTS_W = 32 / W, NA = 4 / SLOTS_W;
+                const int64_t qe = on && live ? e1 : e0;
+                T a[NA];
 #pragma unroll
-            for (int j = 0; j < NA; j++) a[j] = 0;
-            int64_t q = e0 + slot;
-            for (; q + (NA - 1) * SLOTS_W < qe; q += NA * SLOTS_W) {
+                for (int j = 0; j < NA; j++) a[j] = 0;
+                int64_t q = e0 + slot;
+                for (; q + (NA - 1) * SLOTS_W < qe; q += NA * SLOTS_W) {
 #pragma unroll
-                for (int j = 0; j < NA; j++)
-                    a[j] += __ldcs(val + q + j * SLOTS_W) * xt[(int64_t)__ldcs(idx + q + j * SLOTS_W) * TILE + col];
+                    for (int j = 0; j < NA; j++)
+                        a[j] += __ldcs(val + q + j * SLOTS_W) * xt[(int64_t)__ldcs(idx + q + j * SLOTS_W) * TILE + col];
+                }
+#pragma unroll
+                for (int j = 0; j < NA - 1; j++)
+                    if (q + j * SLOTS_W < qe)
+                        a[j] += __ldcs(val + q + j * SLOTS_W) * xt[(int64_t)__ldcs(idx + q + j * SLOTS_W) * TILE + col];
+#pragma unroll
+                for (int h = NA / 2; h >= 1; h >>= 1)
+#pragma unroll
+                    for (int j = 0; j < h; j++) a[j] += a[j + h];
+                acc = a[0];
+#pragma unroll
+                for (int o = 16; o >= W; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            } else {
+                for (int64_t base = e0; on && base < e1; base += CHUNK_CAP) {  // warp-uniform
+                    const int m = (int)min((int64_t)CHUNK_CAP, e1 - base);
+                    for (int i = lane; i < m; i += 32) {
+                        si[i] = __ldcs(idx + base + i);
+                        sv[i] = __ldcs(val + base + i);
+                    }
+                    __syncwarp();
+                    for (int q = 0; q < m; q += ROW_SEG)
+                        acc += seg_sum_slots<T, W>(si, sv, q, live ? min(q + ROW_SEG, m) : q, xt + col, slot);
+                    __syncwarp();
+                }
             }
-#pragma unroll
-            for (int j = 0; j < NA - 1; j++)
-                if (q + j * SLOTS_W < qe)
-                    a[j] += __ldcs(val + q + j * SLOTS_W) * xt[(int64_t)__ldcs(idx + q + j * SLOTS_W) * TILE + col];
-#pragma unroll
-            for (int h = NA / 2; h >= 1; h >>= 1)
-#pragma unroll
-                for (int j = 0; j < h; j++) a[j] += a[j + h];
-            T acc = a[0];
-#pragma unroll
-            for (int o = 16; o >= W; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
             if (lane < W && on) chunk_epilogue<MODE, T>(out, aux, xt, toff, vr0, col, acc, dot, want_dot, dlast);
         }
     }
@@ -829,102 +912,155 @@ static int chunk_blocks(int32_t nchunks) {
     return std::max(1, std::min((nchunks + CH_WARPS - 1) / CH_WARPS, 148 * 6));
 }
 
-// Runs of thin levels: the k columns are independent, so one block per column tile walks the run's steps
-// (rows grouped by dependency depth, DevFactor::SolveRun) on its own, with only block barriers between
-// steps (its own writes are the only values it reads back).  y is read and written in place: no read-only
-// cache path.  A step with fewer rows than warps splits each row's entries over several warps (partial sums
-// added in warp order), so a lone row costs about one gather latency instead of one per entry.
-constexpr int RUN_THREADS = 512;
-constexpr int RUN_WARPS = RUN_THREADS / 32;
+// Levels walked inside one launch: the k columns are independent, so one block per sub-tile of W columns goes through
+// consecutive levels on its own, with only block barriers between them (it reads back nothing but its own writes).
+// A level then costs the chain barrier -> gather -> sum -> store instead of a launch.  Its rows, ordered by length, are
+// taken in rounds (TrsvPlan): a slot of W / 2 lanes (two columns each, 16-byte gathers) works on a row, or 2^lg slots of a
+// warp share it.  The next round's rows, their own values and first entries are loaded while the current one is
+// summed, across level boundaries too.  y is read and written in place: no read-only cache path.
+// What bounds it is the issue of one SM per sub-tile (a round costs every warp about a hundred instructions, however few
+// columns it carries: the time is the same with 4 blocks and with 112) and the latency of its chain, not bandwidth.
+// Measured on B200, one FP64 application, all levels launched one by one with the thin ones in dependency runs -> here:
+// 2-D grid n = 10,000, 885 columns 1.34 -> 0.42 ms; geometric graph n = 20,011, 2642 columns 6.7 -> 4.2 ms; 3-D grid
+// n = 80,840, 1085 columns 9.2 -> 4.6 ms; union of 20 graphs, n = 29K, 726 columns 3.5 -> 1.5 ms; ER n = 20,000, degree
+// 200, 951 columns 2.0 -> 0.68 ms; geometric graph n = 30,011, 60 columns 9.7 -> 1.8 ms.
+// Slower: a row per lane without ordering rows by length (1.3x to 1.6x); rows and entries staged through shared memory
+// by cp.async, by warp or by block (1.3x to 2.2x: more instructions per round than the latency they hide).
+template <class T>
+struct WalkPair;
+template <>
+struct WalkPair<double> {
+    using V = double2;
+};
+template <>
+struct WalkPair<float> {
+    using V = float2;
+};
 
-// one warp's share of a row: entries ptr[row] + sub * SLOTS_W + slot, stepping g * SLOTS_W, four in flight,
-// summed over the slots; every lane returns its column's partial
-template <class T, int W>
-__device__ __forceinline__ T warp_row_share(const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-                                            const T* __restrict__ val, int64_t row, const T* xt, int lane,
-                                            bool live, int sub, int g) {
-    constexpr int SLOTS_W = 32 / W;
-    const int slot = lane / W, c = lane % W;
-    const int64_t e = live ? ptr[row + 1] : 0;
-    const int64_t st = (int64_t)g * SLOTS_W;
-    int64_t p = live ? ptr[row] + (int64_t)sub * SLOTS_W + slot : 0;
-    T a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-    for (; p + 3 * st < e; p += 4 * st) {
-        const int32_t i0 = idx[p], i1 = idx[p + st], i2 = idx[p + 2 * st], i3 = idx[p + 3 * st];
-        const T v0 = val[p], v1 = val[p + st], v2 = val[p + 2 * st], v3 = val[p + 3 * st];
-        a0 += v0 * xt[(int64_t)i0 * TILE + c];
-        a1 += v1 * xt[(int64_t)i1 * TILE + c];
-        a2 += v2 * xt[(int64_t)i2 * TILE + c];
-        a3 += v3 * xt[(int64_t)i3 * TILE + c];
-    }
-    for (; p < e; p += st) a0 += val[p] * xt[(int64_t)idx[p] * TILE + c];
-    T acc = (a0 + a1) + (a2 + a3);
+// Rows row .. row + nr of the storage order, 2^lg slots per row; last: the level's last round
+struct WalkRound {
+    int32_t row;
+    uint16_t nr;
+    uint8_t lg, last;
+};
+constexpr int WALK_MAX_ROUNDS = 4096;  // of one launch (kept in shared memory)
+
+template <class T, int W, int NT, bool FWD, bool CLUSTER>
+__global__ void __launch_bounds__(NT, 1024 / NT)
+    k_trsv_walk(int64_t n, const WalkRound* __restrict__ rounds, int32_t nrounds, const FactorRow* __restrict__ rows,
+                const FactorEnt<T>* __restrict__ ent, const T* __restrict__ aux, T* y, int32_t kcols, int nsub, int cl,
+                RowAct ra) {
+    using V = typename WalkPair<T>::V;
+    constexpr int LPS = W / 2, B = 4;
+    extern __shared__ WalkRound s_rounds[];
+    for (int i = threadIdx.x; i < nrounds; i += NT) s_rounds[i] = rounds[i];
+    __syncthreads();
+    // a cluster of cl blocks shares a sub-tile's rows
+    const int sub = CLUSTER ? blockIdx.x / cl : blockIdx.x;
+    const int slot = (CLUSTER ? blockIdx.x % cl : 0) * (NT / LPS) + threadIdx.x / LPS;
+    const int64_t t = sub / nsub;
+    const int c0 = sub % nsub * W;
+    // a block of padding columns only keeps them at zero (r is zero there): no gathers
+    const bool dead = t * TILE + c0 >= kcols;
+    T* yt = y + t * n * TILE + c0 + 2 * (threadIdx.x % LPS);
+    const T* rt = FWD ? aux + t * n * TILE + c0 + 2 * (threadIdx.x % LPS) : nullptr;
+    auto at = [](const T* p, int32_t u) -> V { return *reinterpret_cast<const V*>(p + (int64_t)u * TILE); };
+    // this slot's share of a row: vertex u (-1: none), cnt entries from e on, stride 2^lg
+    int32_t u, cnt;
+    const FactorEnt<T>* e;
+    FactorEnt<T> en[B];
+    V o;
+    T d = (T)0;
+    auto load_row = [&](const WalkRound& w) -> FactorRow {
+        FactorRow r;
+        r.u = -1;
+        const int q = slot >> w.lg;
+        if (q < w.nr) r = rows[w.row + q];
+        return r;
+    };
+    auto take = [&](const FactorRow& r, int lg) {
+        u = r.u;
+        cnt = 0;
+        if (u >= 0) {
+            if (!row_on(ra, u, t)) {
+                u = -1;
+            } else {
+                const int g = slot & ((1 << lg) - 1);
+                if (!dead) cnt = (r.cnt - g + (1 << lg) - 1) >> lg;
+                e = ent + r.e0 + g;
+                o = at(FWD ? rt : yt, u);
+                if (!FWD) d = aux[u];
 #pragma unroll
-    for (int o = W; o < 32; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    return acc;
-}
-
-// FWD: y_u = r_u - L[u, :] y (row form).  BWD: y_u = y_u / D_u (D_u != 0) - L[:, u]^T y (column form).
-template <class T, bool FWD>
-__device__ __forceinline__ void run_finish(const int32_t* __restrict__ rows, const T* __restrict__ aux, T* y,
-                                           int64_t toff, int c, int32_t i, T acc) {
-    const int64_t u = rows[i];
-    const int64_t o = toff + u * TILE + c;
-    if (FWD) {
-        y[o] = aux[o] - acc;
-    } else {
-        const T d = aux[u];
-        const T yu = y[o];
-        y[o] = (d != (T)0 ? yu / d : yu) - acc;
-    }
-}
-
-template <class T, int W, bool FWD>
-__global__ void __launch_bounds__(RUN_THREADS) k_trsv_run(int64_t n, const int32_t* __restrict__ rows,
-                                                          const int32_t* __restrict__ sched,
-                                                          const int32_t* __restrict__ step, int32_t s0, int32_t s1,
-                                                          const int64_t* __restrict__ ptr,
-                                                          const int32_t* __restrict__ idx,
-                                                          const T* __restrict__ val, const T* __restrict__ aux, T* y,
-                                                          int32_t kcols, int nsub, RowAct ra) {
-    __shared__ T s_part[RUN_WARPS][W];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t t = blockIdx.x / nsub;
-    const int c0 = (int)(blockIdx.x % nsub) * W;  // first column of this block's sub-tile
-    const int64_t toff = t * n * TILE;
-    const bool live = t * TILE + c0 + lane % W < kcols;
-    for (int32_t s = s0; s < s1; s++) {
-        const int32_t a = step[s], b = step[s + 1];
-        const int g = RUN_WARPS / max(1, b - a);  // warps per row
-        if (g <= 1) {
-            for (int32_t q = a + warp; q < b; q += RUN_WARPS) {
-                const int32_t i = sched[q];
-                const bool on = row_on(ra, rows[i], t);
-                const T acc = warp_row_share<T, W>(ptr, idx, val, i, y + toff + c0, lane, live && on, 0, 1);
-                if (lane < W && on) run_finish<T, FWD>(rows, aux, y, toff, c0 + lane, i, acc);
-            }
-        } else {
-            const int q = warp / g, sub = warp % g;
-            const bool mine = a + q < b && row_on(ra, rows[sched[a + q]], t);
-            const T acc = mine ? warp_row_share<T, W>(ptr, idx, val, sched[a + q], y + toff + c0, lane, live, sub, g)
-                               : (T)0;
-            if (lane < W) s_part[warp][lane] = acc;
-            __syncthreads();
-            if (mine && sub == 0 && lane < W) {
-                T tot = s_part[warp][lane];
-                for (int u = 1; u < g; u++) tot += s_part[warp + u][lane];
-                run_finish<T, FWD>(rows, aux, y, toff, c0 + lane, sched[a + q], tot);
+                for (int k = 0; k < B; k++)
+                    if (k < cnt) en[k] = e[k << lg];
             }
         }
-        __syncthreads();
+    };
+    WalkRound w = s_rounds[0];
+    take(load_row(w), w.lg);
+    for (int32_t i = 0; i < nrounds; i++) {
+        WalkRound nw = s_rounds[min(i + 1, nrounds - 1)];
+        if (i + 1 == nrounds) nw.nr = 0;
+        if (!__any_sync(0xffffffffu, u >= 0)) {
+            take(load_row(nw), nw.lg);
+        } else {
+            V acc{(T)0, (T)0}, x[B];
+#pragma unroll
+            for (int k = 0; k < B; k++)
+                if (k < cnt) x[k] = at(yt, en[k].idx);
+            const FactorRow nr = load_row(nw);
+#pragma unroll
+            for (int k = 0; k < B; k++)
+                if (k < cnt) {
+                    acc.x += en[k].v * x[k].x;
+                    acc.y += en[k].v * x[k].y;
+                }
+            for (int done = B; done < cnt; done += B) {
+                e += B << w.lg;
+#pragma unroll
+                for (int k = 0; k < B; k++)
+                    if (done + k < cnt) en[k] = e[k << w.lg];
+#pragma unroll
+                for (int k = 0; k < B; k++)
+                    if (done + k < cnt) x[k] = at(yt, en[k].idx);
+#pragma unroll
+                for (int k = 0; k < B; k++)
+                    if (done + k < cnt) {
+                        acc.x += en[k].v * x[k].x;
+                        acc.y += en[k].v * x[k].y;
+                    }
+            }
+            __syncwarp();
+            for (int f = LPS; f < (LPS << w.lg); f <<= 1) {
+                acc.x += __shfl_xor_sync(0xffffffffu, acc.x, f);
+                acc.y += __shfl_xor_sync(0xffffffffu, acc.y, f);
+            }
+            if (u >= 0 && (slot & ((1 << w.lg) - 1)) == 0) {
+                // FWD: y_u = r_u - L[u, :] y.  BWD: y_u = y_u / D_u (D_u != 0) - L[:, u]^T y.
+                if (!FWD && d != (T)0) {
+                    o.x /= d;
+                    o.y /= d;
+                }
+                o.x -= acc.x;
+                o.y -= acc.y;
+                *reinterpret_cast<V*>(yt + (int64_t)u * TILE) = o;
+            }
+            take(nr, nw.lg);
+        }
+        if (w.last) {
+            // the level's rows are written, for this block or, released and acquired, for the cluster's others
+            if (!CLUSTER) __syncthreads();
+            else asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+        }
+        w = nw;
     }
 }
 
 // ---------------------------------------------------------------- the last forward level, finished
 // The rows of a factor's last level are read by no later forward level, and their columns of L are empty
 // (nothing is eliminated after them; a level's rows never reference each other), so the backward solve's
-// whole work on them is z_u = y_u / D_u - 0.  When the last level is a level of its own (not part of a
-// thin-level run), its forward launch (M_FWD_LAST) does this too and its backward launch is skipped; each
+// whole work on them is z_u = y_u / D_u - 0.  When there is no dense tail, the last level is a launch of its own and
+// its forward launch (M_FWD_LAST) does this too and its backward launch is skipped; each
 // value is formed by the same operations in the same order as in the two launches.  At ER n = 1M the
 // truncated factor's last level holds 855K of the 1M rows, and its backward launch took 5.5 ms of a 21 ms
 // application.  (A kernel that gave each warp several of these short rows at once, with all their loads
@@ -937,6 +1073,11 @@ struct FactorVals {
     const T* prow_val;
     const T* pcol_val;
     const T* D;
+    const T* tin_val;  // the dense tail's entries in earlier levels, and its inverse
+    const T* linv;
+    T* tail_tmp;       // tail rows x ld scratch
+    const FactorEnt<T>* fent;  // the entries of both forms with their values beside them (walked levels)
+    const FactorEnt<T>* bent;
 };
 
 // Column layouts of the triangular-solve launches.  A level launch gives each warp row a width of W columns
@@ -944,13 +1085,20 @@ struct FactorVals {
 // (256-byte gathers); with W = 8 a warp works on four rows at once, with four times the blocks, which suits
 // latency-bound levels of few rows.  Every width gives the same values bit for bit (each (row, column) sum is
 // formed the same way, see k_chunked), so the width is a pure launch-shape choice: the fixed rule below, or
-// widths measured level by level (tune_trsv_shapes).  Runs of thin levels always use 8 columns.  With no more
+// widths measured level by level (tune_trsv_shapes).  Walked levels have their own layout (WalkShape).  With no more
 // than 8 real columns (the factor autotuner's probe) every launch uses 8 columns and one sub-tile; the padding
 // columns of y must then be zero.
 constexpr int NARROW_W = 8;
-constexpr int SPLIT_LEVEL_ROWS = 1024;
+constexpr int SPLIT_LEVEL_ROWS = 28 * 1024;
 constexpr int TRSV_NWIDTH = TILE >= 32 ? 3 : TILE >= 16 ? 2 : 1;  // widths 8, 16, 32 that fit a tile
 static inline int trsv_width(int code) { return 8 << code; }
+// The fixed rule: 8 columns per warp row up to SPLIT_LEVEL_ROWS (row, column tile) pairs -- 1024 rows at 900 columns --
+// and 32 above: a small solve's levels need the four times as many warps up to more rows.
+static int rule_code(const DevFactor& F, int32_t l, int ntiles, bool narrow) {
+    if (narrow) return 0;
+    const int64_t rows = F.level_ptr[l + 1] - F.level_ptr[l];
+    return std::min(rows * ntiles <= SPLIT_LEVEL_ROWS ? 0 : 2, TRSV_NWIDTH - 1);
+}
 
 // CUDA events around each level launch of a preconditioner application (measurement only)
 struct LevelEvents {
@@ -998,34 +1146,181 @@ static void launch_level_w(int code, dim3 grid, cudaStream_t s, int64_t n, const
     }
 }
 
+// ---------------------------------------------------------------- which levels are walked
+// A walk's blocks: W columns and NT threads each, one of 1024 threads per SM, or smaller ones so that all of them are
+// resident at once.  Where the columns leave SMs idle, a cluster of cl blocks shares a sub-tile's rows.
+struct WalkShape {
+    int W = 8, NT = 1024, nsub = 1, cl = 1;  // nsub sub-tiles per column tile
+    int64_t blocks = 0;
+    int slots() const { return 2 * NT / W * cl; }
+};
+static WalkShape walk_shape(int ntiles, bool narrow, int cl) {
+    const int64_t cols = narrow ? NARROW_W : (int64_t)ntiles * TILE;
+    WalkShape w;
+    w.W = narrow ? 2 : 8;
+    w.nsub = (narrow ? NARROW_W : TILE) / w.W;
+    w.cl = cl;
+    w.blocks = cols / w.W * cl;
+    w.NT = w.blocks <= 148 ? 1024 : w.blocks <= 2 * 148 ? 512 : 256;
+    return w;
+}
+// One direction's segments [l0, l1) of the levels before the dense tail, in level order.
+struct TrsvSeg {
+    int32_t l0, l1;
+    const WalkRound* rounds = nullptr;  // device; null: a launch of its own
+    int32_t nrounds = 0;
+};
+struct TrsvPlan {
+    std::vector<TrsvSeg> fw, bw;
+    bool fuse_last = false;
+    WalkShape walk;
+};
+
+template <class T, int W, int NT, bool CLUSTER>
+static void launch_walk_fb(Context& C, bool fwd, const TrsvPlan& P, const TrsvSeg& S, const DevFactor& F,
+                           const FactorVals<T>& V, int64_t n, const T* r, T* y, int32_t kcols, const RowAct& ra) {
+    auto kern = fwd ? k_trsv_walk<T, W, NT, true, CLUSTER> : k_trsv_walk<T, W, NT, false, CLUSTER>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)P.walk.blocks);
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = sizeof(WalkRound) * S.nrounds;  // at most 32 KB
+    cfg.stream = C.stream;
+    cudaLaunchAttribute cluster;
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = (unsigned)P.walk.cl;
+    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    cfg.attrs = &cluster;
+    cfg.numAttrs = CLUSTER ? 1 : 0;
+    const WalkRound* rounds = S.rounds;
+    const FactorRow* rows = fwd ? F.frow : F.brow;
+    const FactorEnt<T>* ent = fwd ? V.fent : V.bent;
+    const T* aux = fwd ? r : V.D;
+    SSP_CUDA(cudaLaunchKernelEx(&cfg, kern, n, rounds, S.nrounds, rows, ent, aux, y, kcols, P.walk.nsub, P.walk.cl, ra));
+}
+template <class T>
+static void launch_walk(Context& C, bool fwd, const TrsvPlan& P, const TrsvSeg& S, const DevFactor& F,
+                        const FactorVals<T>& V, int64_t n, const T* r, T* y, int32_t kcols, const RowAct& ra) {
+    const WalkShape& w = P.walk;
+    auto launch = w.W == 2 ? (w.cl > 1 ? launch_walk_fb<T, 2, 1024, true> : launch_walk_fb<T, 2, 1024, false>)
+                  : w.cl > 1 ? launch_walk_fb<T, 8, 1024, true>
+                  : w.NT == 1024 ? launch_walk_fb<T, 8, 1024, false>
+                  : w.NT == 512 ? launch_walk_fb<T, 8, 512, false> : launch_walk_fb<T, 8, 256, false>;
+    launch(C, fwd, P, S, F, V, n, r, y, kcols, ra);
+}
+
+// The plan for a solve's columns; the rounds go to workspace buffers named after tag.
+static TrsvPlan make_trsv_plan(Context& C, const DevFactor& F, int ntiles, bool narrow, size_t elem,
+                               const std::string& tag) {
+    TrsvPlan P;
+    const int32_t NL = F.tail_rows ? F.tail_l0 : F.num_levels;
+    // the last level finished by its forward launch (M_FWD_LAST); SSP_PRECOND_FUSE_LAST=0 keeps the level's two
+    // launches (the same values, bit for bit; for comparisons)
+    const char* fuse_env = getenv("SSP_PRECOND_FUSE_LAST");
+    P.fuse_last = !(fuse_env && fuse_env[0] == '0') && F.tail_rows == 0 && F.num_levels > 0 && F.last_bwd_nnz == 0;
+    const double cols = narrow ? NARROW_W : (double)ntiles * TILE;
+    // The costs (us, bytes per us) that decide between a launch and a walk, fitted on B200 to the graphs above.  A
+    // level's launch takes 13-18 us where it is small (five dependent loads per chunk, most blocks with one chunk) and
+    // moves gathered rows at 5.5 TB/s where it is large; a walk costs a round's issue, a cycle of its SM's cache tags per
+    // gathered row, or its traffic in 64-byte pieces, whichever is most.
+    const double c_launch = 20.0, bw_launch = 5.5e6;
+    const double c_round = 0.6, bw_walk = 3.9e6, c_level = 0.5, c_cluster = 0.9;
+    const double per_slot = 16.0;
+    // The rounds of level l in storage-row order (longest rows first).  2^lg slots share a row: per_slot entries of the
+    // round's longest row each, or all the slots there are.
+    auto level_rounds = [&](const std::vector<int64_t>& ptr, const WalkShape& w, int32_t l, std::vector<WalkRound>& out) {
+        const int slots = w.slots(), max_lg = w.W == 8 ? 3 : 5;  // slots of a warp
+        const int64_t a = F.level_ptr[l], b = F.level_ptr[l + 1];
+        for (int64_t r = a; r < b;) {
+            const int64_t len = ptr[r + 1] - ptr[r];
+            int lg = 0;
+            while (lg < max_lg && (((b - r) << (lg + 1)) <= slots || (double)len > per_slot * (double)(1 << lg))) lg++;
+            const int64_t e = std::min(b, r + (slots >> lg));
+            out.push_back(WalkRound{(int32_t)r, (uint16_t)(e - r), (uint8_t)lg, (uint8_t)(e == b)});
+            r = e;
+        }
+    };
+    // us of level l walked (rounds: how many) and launched
+    auto walk_us = [&](const std::vector<int64_t>& ptr, const WalkShape& w, int32_t l, size_t rounds) {
+        const double E = (double)(ptr[F.level_ptr[l + 1]] - ptr[F.level_ptr[l]]), R = F.level_ptr[l + 1] - F.level_ptr[l];
+        const double per_sm = (double)ceil_div<int64_t>(w.blocks, 148);
+        return c_level + (w.cl > 1 ? c_cluster : 0.0) +
+               std::max({per_sm * c_round * rounds, per_sm * E / w.cl / 1900.0, (E + 2 * R) * cols * elem / bw_walk});
+    };
+    auto launch_us = [&](const std::vector<int64_t>& ptr, int32_t l) {
+        const double E = (double)(ptr[F.level_ptr[l + 1]] - ptr[F.level_ptr[l]]), R = F.level_ptr[l + 1] - F.level_ptr[l];
+        return c_launch + (E + 2 * R) * cols * elem / bw_launch;
+    };
+    // the factor's last level is a launch of its own (M_FWD_LAST when it can be)
+    const int32_t alone = F.tail_rows ? NL : NL - 1;
+    std::vector<WalkRound> tmp;
+    double best = 0;
+    for (int cl = 1; cl <= 8; cl *= 2) {
+        const WalkShape w = walk_shape(ntiles, narrow, cl);
+        if (cl > 1 && w.blocks > 128) break;
+        double us = 0;
+        for (int32_t l = 0; l < alone; l++)
+            for (const auto* ptr : {&F.hfptr, &F.hbptr}) {
+                tmp.clear();
+                level_rounds(*ptr, w, l, tmp);
+                us += std::min(launch_us(*ptr, l), walk_us(*ptr, w, l, tmp.size()));
+            }
+        if (cl == 1 || us < best) {
+            best = us;
+            P.walk = w;
+        }
+    }
+    std::vector<WalkRound> all;
+    auto plan = [&](bool fwd) {
+        const std::vector<int64_t>& ptr = fwd ? F.hfptr : F.hbptr;
+        std::vector<TrsvSeg> seg;
+        std::vector<double> gain(NL, -1.0);
+        std::vector<size_t> cnt(NL, 0);
+        for (int32_t l = 0; l < alone; l++) {
+            tmp.clear();
+            level_rounds(ptr, P.walk, l, tmp);
+            cnt[l] = tmp.size();
+            gain[l] = launch_us(ptr, l) - walk_us(ptr, P.walk, l, tmp.size());
+        }
+        for (int32_t l = 0; l < NL;) {
+            int32_t r = l;
+            double g = -c_launch;
+            size_t nrd = 0;
+            while (r < NL && gain[r] > 0 && nrd + cnt[r] <= WALK_MAX_ROUNDS) nrd += cnt[r], g += gain[r++];
+            if (r - l >= 2 && g > 0) {
+                const size_t at = all.size();
+                for (int32_t i = 0; i < r - l; i++) level_rounds(ptr, P.walk, fwd ? l + i : r - 1 - i, all);
+                seg.push_back(TrsvSeg{l, r, (const WalkRound*)nullptr + at, (int32_t)(all.size() - at)});
+                l = r;
+            } else {
+                for (r = std::max(r, l + 1); l < r; l++) seg.push_back(TrsvSeg{l, l + 1});
+            }
+        }
+        return seg;
+    };
+    P.fw = plan(true);
+    P.bw = plan(false);
+    WalkRound* d = C.ws.get_t<WalkRound>(tag + "_rounds", all.size() + 1);
+    if (!all.empty()) {
+        SSP_CUDA(cudaMemcpyAsync(d, all.data(), sizeof(WalkRound) * all.size(), cudaMemcpyHostToDevice, C.stream));
+        SSP_CUDA(cudaStreamSynchronize(C.stream));
+    }
+    for (auto* v : {&P.fw, &P.bw})
+        for (TrsvSeg& g : *v) g.rounds = g.nrounds ? d + (g.rounds - (const WalkRound*)nullptr) : nullptr;
+    return P;
+}
+
 // sh: per-level widths (nullptr: the fixed rule); lev: events around each level launch (nullptr: none)
 template <class T>
-static int64_t launch_precond(Context& C, const DevFactor& F, const FactorVals<T>& V, int64_t n, const T* r, T* y,
-                              int64_t ld, int32_t kcols, const RowAct& ra = RowAct(),
+static int64_t launch_precond(Context& C, const DevFactor& F, const TrsvPlan& P, const FactorVals<T>& V, int64_t n,
+                              const T* r, T* y, int64_t ld, int32_t kcols, const RowAct& ra = RowAct(),
                               const TrsvShapes* sh = nullptr, LevelEvents* lev = nullptr) {
     const int ntiles = (int)(ld / TILE);
     const bool narrow = TILE > NARROW_W && kcols <= NARROW_W;
-    const int nsub = narrow ? 1 : TILE / NARROW_W;  // sub-tiles of the 8-column layout (runs)
     int64_t launches = 0;
-    // segments in level order: the thin-level runs (by index into F.runs) and single wide levels (-1)
-    std::vector<std::pair<int32_t, int32_t>> seg;  // (level, run or -1)
-    for (int32_t l = 0, u = 0; l < F.num_levels;) {
-        if (u < (int32_t)F.runs.size() && F.runs[u].l0 == l) {
-            seg.push_back({l, u});
-            l = F.runs[u++].l1;
-        } else {
-            seg.push_back({l++, -1});
-        }
-    }
-    // the last level finished by its forward launch (M_FWD_LAST) when it is a level of its own;
-    // SSP_PRECOND_FUSE_LAST=0 keeps the level's two launches (the same values, bit for bit; for comparisons)
     const int32_t L_last = F.num_levels - 1;
-    const char* fuse_env = getenv("SSP_PRECOND_FUSE_LAST");
-    const bool fuse_last = !(fuse_env && fuse_env[0] == '0') && !seg.empty() && seg.back().second < 0 &&
-                           F.last_bwd_nnz == 0 && L_last >= 0;
     auto width_code = [&](bool fwd, int32_t l) -> int {
         if (narrow) return 0;
-        int c = F.level_ptr[l + 1] - F.level_ptr[l] <= SPLIT_LEVEL_ROWS ? 0 : 2;
+        int c = rule_code(F, l, ntiles, narrow);
         if (sh) {
             const auto& v = fwd ? sh->fw : sh->bw;
             if ((size_t)l < v.size()) c = v[l];
@@ -1040,7 +1335,7 @@ static int64_t launch_precond(Context& C, const DevFactor& F, const FactorVals<T
         const int ns = narrow ? 1 : TILE / trsv_width(code);
         const dim3 grid((unsigned)chunk_blocks(nc), (unsigned)(ntiles * ns));
         const int32_t* ch = (fwd ? F.fchunk : F.bchunk) + c0;
-        const bool last = fwd && fuse_last && l == L_last;
+        const bool last = fwd && P.fuse_last && l == L_last;
         if (lev) lev->begin(C.stream, fwd, l);
         if (last)
             launch_level_w<M_FWD_LAST, T, MINB_FWD>(code, grid, C.stream, n, ch, nc, F.prow_ptr, F.prow_idx,
@@ -1050,32 +1345,35 @@ static int64_t launch_precond(Context& C, const DevFactor& F, const FactorVals<T
                                                F.level_rows, y, r, ld, kcols, ns, nullptr, ra);
         else
             launch_level_w<M_BWD, T, MINB_BWD>(code, grid, C.stream, n, ch, nc, F.pcol_ptr, F.pcol_idx, V.pcol_val,
-                                               F.level_rows, y, V.D, ld, kcols, ns, nullptr, ra);
+                                               F.level_cols, y, V.D, ld, kcols, ns, nullptr, ra);
         if (lev) lev->end(C.stream);
         launches++;
     };
-    const unsigned rgrid = (unsigned)(ntiles * nsub);
-    for (size_t i = 0; i < seg.size(); i++) {
-        if (seg[i].second < 0) {
-            level(true, seg[i].first);
+    for (const auto& s : P.fw) {
+        if (!s.rounds) {
+            level(true, s.l0);
             continue;
         }
-        const auto& run = F.runs[seg[i].second];
-        k_trsv_run<T, NARROW_W, true><<<rgrid, RUN_THREADS, 0, C.stream>>>(
-            n, F.level_rows, F.fsched, F.fstep, run.fs0, run.fs1, F.prow_ptr, F.prow_idx, V.prow_val, r, y, kcols,
-            nsub, ra);
+        launch_walk<T>(C, true, P, s, F, V, n, r, y, kcols, ra);
         launches++;
     }
-    for (size_t i = seg.size(); i-- > 0;) {
-        if (fuse_last && i + 1 == seg.size()) continue;  // finished by its forward launch (M_FWD_LAST)
-        if (seg[i].second < 0) {
-            level(false, seg[i].first);
+    if (F.tail_rows) {
+        // the tail's rows less their entries in earlier levels (one launch, as a level), then its block
+        const int code = width_code(true, F.tail_l0);
+        const int ns = narrow ? 1 : TILE / trsv_width(code);
+        launch_level_w<M_FWD, T, MINB_FWD>(code, dim3((unsigned)chunk_blocks(F.ntchunk), (unsigned)(ntiles * ns)),
+                                           C.stream, n, F.tchunk, F.ntchunk, F.tin_ptr, F.tin_idx, V.tin_val,
+                                           F.level_rows + (F.n - F.tail_rows), y, r, ld, kcols, ns, nullptr, ra);
+        launches += 1 + launch_tail<T>(C, F, V.linv, V.D, y, V.tail_tmp, ntiles);
+    }
+    for (size_t i = P.bw.size(); i-- > 0;) {
+        const auto& s = P.bw[i];
+        if (P.fuse_last && s.l1 == F.num_levels) continue;  // finished by its forward launch (M_FWD_LAST)
+        if (!s.rounds) {
+            level(false, s.l0);
             continue;
         }
-        const auto& run = F.runs[seg[i].second];
-        k_trsv_run<T, NARROW_W, false><<<rgrid, RUN_THREADS, 0, C.stream>>>(
-            n, F.level_rows, F.bsched, F.bstep, run.bs0, run.bs1, F.pcol_ptr, F.pcol_idx, V.pcol_val, V.D, y, kcols,
-            nsub, ra);
+        launch_walk<T>(C, false, P, s, F, V, n, r, y, kcols, ra);
         launches++;
     }
     SSP_CHECK_LAUNCH();
@@ -1120,30 +1418,22 @@ static uint64_t trsv_signature(const DevFactor& F, int64_t n, int64_t ld, int32_
     mix((uint64_t)F.last_fwd_nnz);
     mix((uint64_t)F.last_bwd_nnz);
     for (int32_t v : F.level_ptr) mix((uint64_t)(uint32_t)v);
-    for (const auto& r : F.runs) mix(((uint64_t)(uint32_t)r.l0 << 32) | (uint32_t)r.l1);
+    mix((uint64_t)F.tail_rows);
     return h;
 }
 
-static void count_trsv_widths(const DevFactor& F, const TrsvShapes& sh, PcgReport& rep) {
+static void count_trsv_widths(const DevFactor& F, const TrsvShapes& sh, const TrsvPlan& P, PcgReport& rep) {
     for (int i = 0; i < 3; i++) rep.trsv_levels[i] = 0;
-    std::vector<bool> in_run(F.num_levels, false);
-    for (const auto& r : F.runs)
-        for (int32_t l = r.l0; l < r.l1; l++) in_run[l] = true;
-    for (int32_t l = 0; l < F.num_levels; l++) {
-        if (in_run[l]) continue;
-        if (F.fchunk_lvl[l + 1] > F.fchunk_lvl[l]) rep.trsv_levels[sh.fw[l]]++;
-        if (F.bchunk_lvl[l + 1] > F.bchunk_lvl[l]) rep.trsv_levels[sh.bw[l]]++;
-    }
+    for (const auto& s : P.fw)
+        if (!s.rounds && F.fchunk_lvl[s.l1] > F.fchunk_lvl[s.l0]) rep.trsv_levels[sh.fw[s.l0]]++;
+    for (const auto& s : P.bw)
+        if (!s.rounds && F.bchunk_lvl[s.l1] > F.bchunk_lvl[s.l0]) rep.trsv_levels[sh.bw[s.l0]]++;
 }
 
-static int rule_code(const DevFactor& F, int32_t l, bool narrow) {
-    if (narrow) return 0;
-    return std::min(F.level_ptr[l + 1] - F.level_ptr[l] <= SPLIT_LEVEL_ROWS ? 0 : 2, TRSV_NWIDTH - 1);
-}
-static TrsvShapes rule_shapes(const DevFactor& F, bool narrow) {
+static TrsvShapes rule_shapes(const DevFactor& F, int ntiles, bool narrow) {
     TrsvShapes s;
     s.fw.resize(F.num_levels);
-    for (int32_t l = 0; l < F.num_levels; l++) s.fw[l] = (uint8_t)rule_code(F, l, narrow);
+    for (int32_t l = 0; l < F.num_levels; l++) s.fw[l] = (uint8_t)rule_code(F, l, ntiles, narrow);
     s.bw = s.fw;
     return s;
 }
@@ -1156,7 +1446,7 @@ static TrsvShapes forced_shapes(const DevFactor& F, int code) {
 
 // per level and direction, the width with the smallest time in ev[c] (one measured application per width
 // code c); the rule's width unless another is faster
-static void shapes_from_events(const DevFactor& F, const LevelEvents* ev, int nw, TrsvShapes& out) {
+static void shapes_from_events(const DevFactor& F, int ntiles, const LevelEvents* ev, int nw, TrsvShapes& out) {
     const float INF = 3.0e38f;
     std::vector<float> best(2 * (size_t)F.num_levels * nw, INF);
     for (int c = 0; c < nw; c++) {
@@ -1173,7 +1463,7 @@ static void shapes_from_events(const DevFactor& F, const LevelEvents* ev, int nw
     for (int dir = 0; dir < 2; dir++)
         for (int32_t l = 0; l < F.num_levels; l++) {
             const float* b = &best[((size_t)dir * F.num_levels + l) * nw];
-            int pick = rule_code(F, l, false);
+            int pick = rule_code(F, l, ntiles, false);
             for (int c = 0; c < nw; c++)
                 if (b[c] < b[pick]) pick = c;
             (dir == 0 ? out.fw : out.bw)[l] = (uint8_t)pick;
@@ -1209,22 +1499,22 @@ static void cache_shapes(Context& C, uint64_t key, const TrsvShapes& s) {
     E.push_back({key, s});
 }
 
-static void report_shapes(PcgReport& rep, int32_t source, const DevFactor& F, const TrsvShapes& s) {
+static void report_shapes(PcgReport& rep, int32_t source, const DevFactor& F, const TrsvShapes& s, const TrsvPlan& P) {
     rep.trsv_shapes = source;
-    count_trsv_widths(F, s, rep);
+    count_trsv_widths(F, s, P, rep);
 }
 
 // Three applications, one per width, then the per-level choice (the stage entry point's measurement).
 template <class T>
-static void tune_trsv_shapes(Context& C, const DevFactor& F, const FactorVals<T>& V, int64_t n, const T* r, T* y,
-                             int64_t ld, int32_t kcols, const RowAct& ra, TrsvShapes& out) {
+static void tune_trsv_shapes(Context& C, const DevFactor& F, const TrsvPlan& P, const FactorVals<T>& V, int64_t n,
+                             const T* r, T* y, int64_t ld, int32_t kcols, const RowAct& ra, TrsvShapes& out) {
     LevelEvents ev[3];
     for (int c = 0; c < TRSV_NWIDTH; c++) {
         const TrsvShapes f = forced_shapes(F, c);
-        C.kernels_launched += launch_precond<T>(C, F, V, n, r, y, ld, kcols, ra, &f, &ev[c]);
+        C.kernels_launched += launch_precond<T>(C, F, P, V, n, r, y, ld, kcols, ra, &f, &ev[c]);
     }
     SSP_CUDA(cudaStreamSynchronize(C.stream));
-    shapes_from_events(F, ev, TRSV_NWIDTH, out);
+    shapes_from_events(F, (int)(ld / TILE), ev, TRSV_NWIDTH, out);
 }
 
 // The preconditioner application as a CUDA graph, with its level shapes.  measure: the shapes are still to be
@@ -1236,6 +1526,7 @@ struct Precond {
     bool has_shapes = false;
     bool measure = false;
     uint64_t key = 0;
+    TrsvPlan plan;                 // which levels are walked
     int mstep = 0;                 // widths measured so far
     LevelEvents mev[3];            // their level launches
     cudaEvent_t m0 = nullptr, m1 = nullptr;  // around the measured applications
@@ -1463,13 +1754,14 @@ static void build_precond_graph(Context& C, const DevFactor& F, int64_t n, int64
     uint64_t key = 0;
     const bool narrow = TILE > NARROW_W && kcols <= NARROW_W;
     const ShapeSource src = trsv_shape_source(C, F, n, ld, kcols, elem, ra.act != nullptr, store, key);
+    P.plan = make_trsv_plan(C, F, (int)(ld / TILE), narrow, elem, elem == sizeof(float) ? "pcg32" : "pcg");
     P.measure = false;
     P.has_shapes = src == ShapeSource::Forced || src == ShapeSource::Cached;
     if (P.has_shapes) {
         P.shapes = store;
-        report_shapes(rep, src == ShapeSource::Forced ? SSP_TRSV_FORCED : SSP_TRSV_CACHED, F, store);
+        report_shapes(rep, src == ShapeSource::Forced ? SSP_TRSV_FORCED : SSP_TRSV_CACHED, F, store, P.plan);
     } else {
-        report_shapes(rep, SSP_TRSV_RULE, F, rule_shapes(F, narrow));
+        report_shapes(rep, SSP_TRSV_RULE, F, rule_shapes(F, (int)(ld / TILE), narrow), P.plan);
         if (src == ShapeSource::Measure) {
             P.measure = true;
             P.key = key;
@@ -1479,7 +1771,36 @@ static void build_precond_graph(Context& C, const DevFactor& F, int64_t n, int64
     capture_precond(C, P, launches, pc);
 }
 
-static FactorVals<double> fp64_vals(const DevFactor& F) { return FactorVals<double>{F.prow_val, F.pcol_val, F.D}; }
+static FactorVals<double> fp64_vals(Context& C, const DevFactor& F, int64_t ld) {
+    double* tmp = F.tail_rows ? C.ws.get_t<double>("pcg_tail", (size_t)F.tail_rows * ld) : nullptr;
+    return FactorVals<double>{F.prow_val, F.pcol_val, F.D, F.tin_val, F.linv, tmp, F.fent, F.bent};
+}
+// the factor's values rounded to FP32, in workspace buffers named after tag
+static FactorVals<float> fp32_vals(Context& C, const DevFactor& F, int64_t n, int64_t ld, const std::string& tag) {
+    const int64_t T = F.tail_rows;
+    const int64_t cnt[5] = {F.nnz, F.nnz, n, T ? F.tin_nnz : 0, T * T};
+    const double* src[5] = {F.prow_val, F.pcol_val, F.D, F.tin_val, F.linv};
+    float* f = C.ws.get_t<float>(tag + "_fval", 2 * F.nnz + n + cnt[3] + cnt[4] + 1);
+    int64_t at[5], o = 0;
+    for (int i = 0; i < 5; i++) {
+        at[i] = o;
+        o += cnt[i];
+        if (cnt[i] <= 0) continue;
+        k_d2f<<<grid_for(cnt[i], 256, 148 * 16), 256, 0, C.stream>>>(cnt[i], src[i], f + at[i]);
+        SSP_CHECK_LAUNCH();
+        C.kernels_launched++;
+    }
+    float* tmp = T ? C.ws.get_t<float>(tag + "_tail", (size_t)T * ld) : nullptr;
+    FactorEnt<float>* e = C.ws.get_t<FactorEnt<float>>(tag + "_ent", 2 * F.nnz + 1);
+    if (F.nnz > 0) {
+        const int g = grid_for(F.nnz, 256, 148 * 16);
+        k_ent_f32<<<g, 256, 0, C.stream>>>(F.nnz, F.fent, e);
+        k_ent_f32<<<g, 256, 0, C.stream>>>(F.nnz, F.bent, e + F.nnz);
+        SSP_CHECK_LAUNCH();
+        C.kernels_launched += 2;
+    }
+    return FactorVals<float>{f + at[0], f + at[1], f + at[2], f + at[3], f + at[4], tmp, e, e + F.nnz};
+}
 
 // apply M^{-1} to R into Z once (tile-major n x ld blocks; stage entry point).  When the shapes are to be
 // measured, one application per width measures them first (each writes the same Z).
@@ -1487,15 +1808,17 @@ void precond_apply_device(Context& C, const DevFactor& F, const double* R, doubl
     TrsvShapes store;
     uint64_t key = 0;
     const ShapeSource src = trsv_shape_source(C, F, F.n, ld, (int32_t)ld, sizeof(double), false, store, key);
+    const TrsvPlan P = make_trsv_plan(C, F, (int)(ld / TILE), TILE > NARROW_W && ld <= NARROW_W, sizeof(double), "pcg");
+    const FactorVals<double> V = fp64_vals(C, F, ld);
     const TrsvShapes* sh = nullptr;
     if (src == ShapeSource::Forced || src == ShapeSource::Cached) {
         sh = &store;
     } else if (src == ShapeSource::Measure) {
-        tune_trsv_shapes<double>(C, F, fp64_vals(F), F.n, R, Z, ld, (int32_t)ld, RowAct(), store);
+        tune_trsv_shapes<double>(C, F, P, V, F.n, R, Z, ld, (int32_t)ld, RowAct(), store);
         cache_shapes(C, key, store);
         sh = &store;
     }
-    int64_t l = launch_precond<double>(C, F, fp64_vals(F), F.n, R, Z, ld, (int32_t)ld, RowAct(), sh);
+    int64_t l = launch_precond<double>(C, F, P, V, F.n, R, Z, ld, (int32_t)ld, RowAct(), sh);
     C.kernels_launched += l;
 }
 
@@ -1603,14 +1926,14 @@ static int32_t pcg_solve(Context& C, int64_t n, int32_t k, int64_t ld, const Spm
     // cache it, and rebuild the graph with it
     auto finish_measure = [&]() {
         if (!P.measure || P.mstep < TRSV_NWIDTH) return;
-        shapes_from_events(F, P.mev, TRSV_NWIDTH, P.shapes);
+        shapes_from_events(F, (int)ntiles, P.mev, TRSV_NWIDTH, P.shapes);
         float ms = 0;
         SSP_CUDA(cudaEventElapsedTime(&ms, P.m0, P.m1));
         rep.ms_trsv_tune += ms;
         P.has_shapes = true;
         P.measure = false;
         cache_shapes(C, P.key, P.shapes);
-        report_shapes(rep, SSP_TRSV_TUNED, F, P.shapes);
+        report_shapes(rep, SSP_TRSV_TUNED, F, P.shapes, P.plan);
         capture_precond(C, P, pc_launches, pc);
     };
     int64_t active = read_i64(C, S.nactive);
@@ -1843,34 +2166,25 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
             size_t elem = sizeof(double);
             if (opt.precision == SSP_PRECISION_PC32 && !(TILE > NARROW_W && k <= NARROW_W)) {
                 // FP64 PCG with the triangular solves in FP32: r rounded on the way in, z widened on the way out
-                float* fv = W.get_t<float>("pcgp_fval", 2 * F.nnz + n + 1);
-                const int64_t fcount[3] = {F.nnz, F.nnz, n};
-                const double* fsrc[3] = {F.prow_val, F.pcol_val, F.D};
-                int64_t at = 0;
-                for (int i = 0; i < 3; i++) {
-                    if (fcount[i] > 0)
-                        k_d2f<<<grid_for(fcount[i], 256, 148 * 16), 256, 0, C.stream>>>(fcount[i], fsrc[i], fv + at);
-                    at += fcount[i];
-                }
-                SSP_CHECK_LAUNCH();
-                C.kernels_launched += 3;
-                const FactorVals<float> V32{fv, fv + F.nnz, fv + 2 * F.nnz};
+                const FactorVals<float> V32 = fp32_vals(C, F, n, ld, "pcgp");
                 // r32 and z32 live in q's memory: q (= A p) is dead from the r update to the next Laplacian
                 // product, and the preconditioner runs in between, so this mode needs no more memory than FP64
                 float* r32 = reinterpret_cast<float*>(q);
                 float* z32 = r32 + total;
                 const int cgrid = grid_for(total, 256, 148 * 16);
-                pc = [&C, &F, V32, n, r32, z32, r, z, ld, k, ra, total, cgrid](const TrsvShapes* sh, LevelEvents* lev) {
+                pc = [&C, &F, &P, V32, n, r32, z32, r, z, ld, k, ra, total, cgrid](const TrsvShapes* sh, LevelEvents* lev) {
                     k_d2f<<<cgrid, 256, 0, C.stream>>>(total, r, r32);
-                    const int64_t l = launch_precond<float>(C, F, V32, n, r32, z32, ld, k, ra, sh, lev);
+                    const int64_t l = launch_precond<float>(C, F, P.plan, V32, n, r32, z32, ld, k, ra, sh, lev);
                     k_f2d<<<cgrid, 256, 0, C.stream>>>(total, z32, z);
                     SSP_CHECK_LAUNCH();
                     return l + 2;
                 };
                 elem = sizeof(float);
             } else {
-                pc = [&C, &F, n, r, z, ld, k, ra](const TrsvShapes* sh, LevelEvents* lev) {
-                    return launch_precond<double>(C, F, fp64_vals(F), n, r, z, ld, k, ra, sh, lev);
+                // (its scratch is allocated here: the applications are captured into graphs)
+                const FactorVals<double> V64 = fp64_vals(C, F, ld);
+                pc = [&C, &F, &P, V64, n, r, z, ld, k, ra](const TrsvShapes* sh, LevelEvents* lev) {
+                    return launch_precond<double>(C, F, P.plan, V64, n, r, z, ld, k, ra, sh, lev);
                 };
             }
             build_precond_graph(C, F, n, ld, k, elem, P, pc_launches, rep, ra, pc);
@@ -1880,7 +2194,6 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
     } else {
         // FP32 copies of the Laplacian and factor values, and the FP32 inner vectors
         float* aval32 = W.get_t<float>("pcgm_aval", lap_nnz + 1);
-        float* fval32 = W.get_t<float>("pcgm_fval", 2 * F.nnz + n + 1);
         auto to_f32 = [&](int64_t count, const double* src, float* dst) {
             if (count <= 0) return;
             k_d2f<<<grid_for(count, 256, 148 * 16), 256, 0, C.stream>>>(count, src, dst);
@@ -1888,10 +2201,7 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
             C.kernels_launched++;
         };
         to_f32(lap_nnz, A.val, aval32);
-        to_f32(F.nnz, F.prow_val, fval32);
-        to_f32(F.nnz, F.pcol_val, fval32 + F.nnz);
-        to_f32(n, F.D, fval32 + 2 * F.nnz);
-        const FactorVals<float> V32{fval32, fval32 + F.nnz, fval32 + 2 * F.nnz};
+        const FactorVals<float> V32 = fp32_vals(C, F, n, ld, "pcgm");
         float* e32 = W.get_t<float>("pcgm_e", total);
         float* r32 = W.get_t<float>("pcgm_r", total);
         float* z32 = W.get_t<float>("pcgm_z", total);
@@ -1916,8 +2226,9 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
                 k_cols_init_inner<<<cg, 256, 0, C.stream>>>(ld, k, MIXED_INNER_REDUCTION, S.thr, Si, R.G);
                 SSP_CHECK_LAUNCH();
                 C.kernels_launched += 2;
-                const PcApply pc32f = [&C, &F, V32, n, r32, z32, ld, k, ra](const TrsvShapes* sh, LevelEvents* lev) {
-                    return launch_precond<float>(C, F, V32, n, r32, z32, ld, k, ra, sh, lev);
+                const PcApply pc32f = [&C, &F, &P32, V32, n, r32, z32, ld, k, ra](const TrsvShapes* sh,
+                                                                                   LevelEvents* lev) {
+                    return launch_precond<float>(C, F, P32.plan, V32, n, r32, z32, ld, k, ra, sh, lev);
                 };
                 if (!P32.exec) build_precond_graph(C, F, n, ld, k, sizeof(float), P32, pc32, rep, ra, pc32f);
                 int32_t cap = opt.max_iters - it;
@@ -1940,8 +2251,9 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
                 k_cols_init_inner<<<cg, 256, 0, C.stream>>>(ld, k, 0.0, S.thr, Si, R.G);
                 SSP_CHECK_LAUNCH();
                 C.kernels_launched += 2;
-                const PcApply pc64f = [&C, &F, n, r, z, ld, k, ra](const TrsvShapes* sh, LevelEvents* lev) {
-                    return launch_precond<double>(C, F, fp64_vals(F), n, r, z, ld, k, ra, sh, lev);
+                const FactorVals<double> V64 = fp64_vals(C, F, ld);
+                const PcApply pc64f = [&C, &F, &P64, V64, n, r, z, ld, k, ra](const TrsvShapes* sh, LevelEvents* lev) {
+                    return launch_precond<double>(C, F, P64.plan, V64, n, r, z, ld, k, ra, sh, lev);
                 };
                 if (!P64.exec) build_precond_graph(C, F, n, ld, k, sizeof(double), P64, pc64, rep, ra, pc64f);
                 its = pcg_solve<double>(C, n, k, ld, A, A.val, F, pc64f, P64, pc64,
