@@ -574,26 +574,16 @@ struct LoopGraph {
 // evict the gathered slab from L2), then every (row, column) lane pair sums its row with independent
 // gathers from the tile slab.  Warps never wait for each other.  Modes: SpMM (+ p.q partials), SpMM
 // adding into its output (the second and later column slabs of the matrix), forward solve, backward solve.
-enum { M_SPMM = 0, M_FWD = 1, M_BWD = 2, M_SPMM_ACC = 3, M_FWD_LAST = 4 };
+enum { M_FWD = 1, M_BWD = 2, M_FWD_LAST = 4 };
 constexpr int CH_THREADS = 256;
-// independent gathers in flight per lane in the chunk kernels (powers of two).  Measured on B200 at ER n = 1M,
-// k = 1327: 8 for the SpMM takes it from 48 to 38 ms.
-#ifndef SSP_GATHER_UNROLL_SPMM
-#define SSP_GATHER_UNROLL_SPMM 8
-#endif
 constexpr int CH_WARPS = CH_THREADS / 32;
-constexpr int MINB_SPMM = 6, MINB_FWD = 6, MINB_BWD = 5;
+constexpr int MINB_FWD = 6, MINB_BWD = 5;
 
 template <int MODE, class T>
-__device__ __forceinline__ void chunk_epilogue(T* out, const T* aux, const T* xt, int64_t toff, int64_t v, int col,
-                                               T acc, double& dot, bool want_dot, const T* dlast) {
+__device__ __forceinline__ void chunk_epilogue(T* out, const T* aux, int64_t toff, int64_t v, int col, T acc,
+                                               const T* dlast) {
     const int64_t o = toff + v * TILE + col;
-    if (MODE == M_SPMM || MODE == M_SPMM_ACC) {
-        // q streams out (evict-first), so it does not push the gathered slab out of L2
-        if (MODE == M_SPMM_ACC) acc += __ldcs(out + o);
-        __stcs(out + o, acc);
-        if (want_dot) dot += (double)acc * (double)xt[v * TILE + col];
-    } else if (MODE == M_FWD) {
+    if (MODE == M_FWD) {
         out[o] = aux[o] - acc;
     } else if (MODE == M_FWD_LAST) {
         // the forward value, then the backward solve's step for a row with an empty column
@@ -672,22 +662,18 @@ __device__ __forceinline__ T seg_sum_slots(const int32_t* si, const T* sv, int s
 
 // Grid: x over chunks, y over (tile, sub-tile): a tile's TILE columns are covered by nsub = TILE / W warps'
 // column ranges (nsub = 1 for the full-width layout, or for the narrow one when only W columns are real).
-// MINB: resident blocks per SM asked of the compiler.  The SpMM asks for six (its registers would otherwise
-// allow five: FP32 SpMM 29.7 -> 22.6 ms at ER n = 1M); the level solves ask for what their own register
-// choice gives (forward 6, backward 5; forcing six on the backward solve cost the preconditioner 7 %).
-// Keeping the body in the kernel itself matters: moved into a __device__ function holding the shared
-// arrays, the FP32 SpMM took 39 ms instead of 22.6 (twice the long-scoreboard stalls per issue).
+// MINB: resident blocks per SM asked of the compiler, what each direction's own register choice gives (forward 6,
+// backward 5; forcing six on the backward solve cost the preconditioner 7 %).
 template <int MODE, class T, int W, int MINB>
 __global__ void __launch_bounds__(CH_THREADS, MINB)
     k_chunked(int64_t n, const int32_t* __restrict__ cstart, int32_t nchunks, const int64_t* __restrict__ ptr,
               const int32_t* __restrict__ idx, const T* __restrict__ val, const int32_t* __restrict__ rowmap,
-              const T* xsrc, T* out, const T* __restrict__ aux, int64_t ld, double* __restrict__ part,
-              int32_t kcols, int nsub, const T* __restrict__ dlast = nullptr, RowAct ra = RowAct()) {
+              const T* xsrc, T* out, const T* __restrict__ aux, int32_t kcols, int nsub,
+              const T* __restrict__ dlast = nullptr, RowAct ra = RowAct()) {
     __shared__ int32_t s_idx[CH_WARPS][CHUNK_CAP];
     __shared__ T s_val[CH_WARPS][CHUNK_CAP];
     __shared__ int32_t s_ptr[CH_WARPS][CHUNK_ROWS + 1];
     __shared__ int32_t s_row[CH_WARPS][CHUNK_ROWS];
-    __shared__ double s_red[CH_THREADS];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t t = blockIdx.y / nsub;
     const int c0 = (int)(blockIdx.y % nsub) * W;  // first column of this block's sub-tile
@@ -697,9 +683,6 @@ __global__ void __launch_bounds__(CH_THREADS, MINB)
     T* sv = s_val[w];
     int32_t* sp = s_ptr[w];
     int32_t* sr = s_row[w];
-    constexpr bool SPMM = MODE == M_SPMM || MODE == M_SPMM_ACC;
-    const bool want_dot = SPMM && part != nullptr;
-    double dot = 0.0;  // SpMM: per-lane partial of p.q for column (lane % W)
     for (int32_t c = blockIdx.x * CH_WARPS + w; c < nchunks; c += gridDim.x * CH_WARPS) {
         const int32_t r0 = cstart[c], r1 = cstart[c + 1];
         const int64_t e0 = ptr[r0], e1 = ptr[r1];
@@ -709,10 +692,10 @@ __global__ void __launch_bounds__(CH_THREADS, MINB)
                 si[i] = __ldcs(idx + e0 + i);
                 sv[i] = __ldcs(val + e0 + i);
             }
-            // the chunk's row pointers and vertex ids (level solves: storage row -> vertex) staged together
+            // the chunk's row pointers and vertex ids staged together
             for (int32_t i = lane; i <= r1 - r0; i += 32) {
                 sp[i] = (int32_t)(ptr[r0 + i] - e0);
-                if (i < r1 - r0) sr[i] = rowmap ? rowmap[r0 + i] : r0 + i;
+                if (i < r1 - r0) sr[i] = rowmap[r0 + i];
             }
             __syncwarp();
             const int32_t pairs = (r1 - r0) * W;
@@ -722,83 +705,127 @@ __global__ void __launch_bounds__(CH_THREADS, MINB)
                 const bool on = row_on(ra, vrow, t);
                 const bool live = on && t * TILE + col < kcols;
                 const int32_t q0 = sp[rr], q1 = live ? sp[rr + 1] : q0;
-                T sum;
-                if constexpr (SPMM) {
-                    // GATHER_UNROLL independent accumulators, summed as a pairwise tree
-                    constexpr int GATHER_UNROLL = SSP_GATHER_UNROLL_SPMM;
-                    T a[GATHER_UNROLL];
-#pragma unroll
-                    for (int u = 0; u < GATHER_UNROLL; u++) a[u] = 0;
-                    int32_t q = q0;
-                    for (; q + GATHER_UNROLL - 1 < q1; q += GATHER_UNROLL) {
-#pragma unroll
-                        for (int u = 0; u < GATHER_UNROLL; u++)
-                            a[u] += sv[q + u] * xt[(int64_t)si[q + u] * TILE + col];
-                    }
-                    if (GATHER_UNROLL > 4 && q + 3 < q1) {  // short rows (a slab's share of a row) still get 4 in flight
-#pragma unroll
-                        for (int u = 0; u < 4; u++) a[u] += sv[q + u] * xt[(int64_t)si[q + u] * TILE + col];
-                        q += 4;
-                    }
-                    for (; q < q1; q++) a[0] += sv[q] * xt[(int64_t)si[q] * TILE + col];
-#pragma unroll
-                    for (int h = 1; h < GATHER_UNROLL; h <<= 1)
-#pragma unroll
-                        for (int u = 0; u < GATHER_UNROLL; u += 2 * h) a[u] += a[u + h];
-                    sum = a[0];
-                } else {
-                    sum = row_sum_lane<T>(si, sv, q0, q1, xt + col);
-                }
-                if (on) chunk_epilogue<MODE, T>(out, aux, xt, toff, vrow, col, sum, dot, want_dot, dlast);
+                const T sum = row_sum_lane<T>(si, sv, q0, q1, xt + col);
+                if (on) chunk_epilogue<MODE, T>(out, aux, toff, vrow, col, sum, dlast);
             }
             __syncwarp();
         } else {
             // one long row: (32 / W) entry slots x W columns
             const int slot = lane / W, col = c0 + lane % W;
-            const int64_t vr0 = rowmap ? rowmap[r0] : r0;
+            const int64_t vr0 = rowmap[r0];
             const bool on = row_on(ra, vr0, t);
             const bool live = t * TILE + col < kcols;
             T acc = 0;
-            if constexpr (SPMM) {
-                constexpr int SLOTS_W = 32 / W, NA = 4 / SLOTS_W;
-                const int64_t qe = on && live ? e1 : e0;
-                T a[NA];
-#pragma unroll
-                for (int j = 0; j < NA; j++) a[j] = 0;
-                int64_t q = e0 + slot;
-                for (; q + (NA - 1) * SLOTS_W < qe; q += NA * SLOTS_W) {
-#pragma unroll
-                    for (int j = 0; j < NA; j++)
-                        a[j] += __ldcs(val + q + j * SLOTS_W) * xt[(int64_t)__ldcs(idx + q + j * SLOTS_W) * TILE + col];
+            for (int64_t base = e0; on && base < e1; base += CHUNK_CAP) {  // warp-uniform
+                const int m = (int)min((int64_t)CHUNK_CAP, e1 - base);
+                for (int i = lane; i < m; i += 32) {
+                    si[i] = __ldcs(idx + base + i);
+                    sv[i] = __ldcs(val + base + i);
                 }
-#pragma unroll
-                for (int j = 0; j < NA - 1; j++)
-                    if (q + j * SLOTS_W < qe)
-                        a[j] += __ldcs(val + q + j * SLOTS_W) * xt[(int64_t)__ldcs(idx + q + j * SLOTS_W) * TILE + col];
-#pragma unroll
-                for (int h = NA / 2; h >= 1; h >>= 1)
-#pragma unroll
-                    for (int j = 0; j < h; j++) a[j] += a[j + h];
-                acc = a[0];
-#pragma unroll
-                for (int o = 16; o >= W; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            } else {
-                for (int64_t base = e0; on && base < e1; base += CHUNK_CAP) {  // warp-uniform
-                    const int m = (int)min((int64_t)CHUNK_CAP, e1 - base);
-                    for (int i = lane; i < m; i += 32) {
-                        si[i] = __ldcs(idx + base + i);
-                        sv[i] = __ldcs(val + base + i);
-                    }
-                    __syncwarp();
-                    for (int q = 0; q < m; q += ROW_SEG)
-                        acc += seg_sum_slots<T, W>(si, sv, q, live ? min(q + ROW_SEG, m) : q, xt + col, slot);
-                    __syncwarp();
-                }
+                __syncwarp();
+                for (int q = 0; q < m; q += ROW_SEG)
+                    acc += seg_sum_slots<T, W>(si, sv, q, live ? min(q + ROW_SEG, m) : q, xt + col, slot);
+                __syncwarp();
             }
-            if (lane < W && on) chunk_epilogue<MODE, T>(out, aux, xt, toff, vr0, col, acc, dot, want_dot, dlast);
+            if (lane < W && on) chunk_epilogue<MODE, T>(out, aux, toff, vr0, col, acc, dlast);
         }
     }
-    if (want_dot) {
+}
+
+// ---------------------------------------------------------------- q = A p
+// A warp's item is a chunk (as above) or a segment of CHUNK_CAP entries of a longer row.  A segment's sums go to
+// lpart[segment][column], and k_spmm_long adds a row's segments up: a hub's row, walked by one warp, kept a whole launch
+// waiting.  The lanes of a row have eight gathers in flight, its last entries (under predicates) among them, in four
+// accumulators: a grid's row of seven entries costs one gather latency, where a loop over the last three added three.
+// Bound by random 256-byte row gathers through L2 (51 GB in 5.0 ms at ER n = 250,000).  Measured on B200, one FP64 product,
+// with the long rows walked whole and serial last entries -> here: R-MAT n = 24,281, 883K entries, 2693 columns 4.21 ->
+// 1.60 ms; 3-D grid n = 80,840, 1085 columns 1.05 -> 0.58; ER n = 250,000, degree 20, 1194 columns 6.4 -> 5.0; ER n = 1M, 80
+// columns 2.70 -> 2.10.  FP32 stays at 3.1 ms at ER n = 229,373, 1185 columns.  Slower: 16-column halves of a tile, whose
+// gathered rows then fit L2 (2.89 against 2.75 ms at ER n = 1M); sixteen gathers in flight in FP32 (3.14 against 3.07).
+// Six resident blocks per SM (five ran slower: FP32 29.7 against 22.6 ms at ER n = 1M, 1327 columns).
+struct SpmmItems {
+    const int32_t* chunks = nullptr;  // nchunks + 1 row starts (a row of more than CHUNK_CAP entries is skipped there)
+    int32_t nchunks = 0;
+    int32_t nseg = 0;
+    const int64_t* seg = nullptr;     // first entry of each segment (its end: CHUNK_CAP further, or the row's)
+    const int32_t* segrow = nullptr;  // row of each segment
+    int32_t nlong = 0;
+    const int32_t* lrow = nullptr;    // rows of more than CHUNK_CAP entries
+    const int32_t* lseg = nullptr;    // nlong + 1 first segments
+};
+template <class T>
+__device__ __forceinline__ T spmm_row(const int32_t* si, const T* sv, int32_t q, int32_t q1, const T* xt) {
+    T a[4] = {0, 0, 0, 0};
+    for (; q + 7 < q1; q += 8) {
+        T x[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) x[u] = xt[(int64_t)si[q + u] * TILE];
+#pragma unroll
+        for (int u = 0; u < 8; u++) a[u & 3] += sv[q + u] * x[u];
+    }
+    if (q < q1) {
+        T x[7];
+#pragma unroll
+        for (int u = 0; u < 7; u++) x[u] = q + u < q1 ? xt[(int64_t)si[q + u] * TILE] : (T)0;
+#pragma unroll
+        for (int u = 0; u < 7; u++)
+            if (q + u < q1) a[u & 3] += sv[q + u] * x[u];
+    }
+    return (a[0] + a[1]) + (a[2] + a[3]);
+}
+
+// W: columns per warp row (TILE, or 8 when at most 8 are real); ACC adds into q (the second and later column slabs)
+template <class T, int W, bool ACC>
+__global__ void __launch_bounds__(CH_THREADS, 6)
+    k_spmm(int64_t n, SpmmItems S, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+           const T* __restrict__ val, const T* __restrict__ p, T* __restrict__ q, int64_t ld, T* __restrict__ lpart,
+           double* __restrict__ part, int32_t kcols, RowAct ra) {
+    __shared__ int32_t s_idx[CH_WARPS][CHUNK_CAP];
+    __shared__ T s_val[CH_WARPS][CHUNK_CAP];
+    __shared__ int32_t s_ptr[CH_WARPS][CHUNK_ROWS + 1];
+    __shared__ double s_red[CH_THREADS];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t t = blockIdx.y;
+    const int64_t toff = t * n * TILE;
+    const T* xt = p + toff;
+    int32_t* si = s_idx[w];
+    T* sv = s_val[w];
+    int32_t* sp = s_ptr[w];
+    double dot = 0.0;  // per-lane partial of p.q for column (lane % W)
+    for (int32_t c = blockIdx.x * CH_WARPS + w; c < S.nseg + S.nchunks; c += gridDim.x * CH_WARPS) {
+        const bool seg = c < S.nseg;  // segments, the larger items, first
+        const int32_t r0 = seg ? S.segrow[c] : S.chunks[c - S.nseg], r1 = seg ? r0 + 1 : S.chunks[c - S.nseg + 1];
+        const int64_t e0 = seg ? S.seg[c] : ptr[r0];
+        const int64_t e1 = seg ? min(e0 + CHUNK_CAP, ptr[r1]) : ptr[r1];
+        const int32_t ne = (int32_t)(e1 - e0);
+        if (ne > CHUNK_CAP) continue;  // a long row: its segments
+        for (int32_t i = lane; i < ne; i += 32) {
+            si[i] = __ldcs(idx + e0 + i);
+            sv[i] = __ldcs(val + e0 + i);
+        }
+        for (int32_t i = lane; i <= r1 - r0; i += 32) sp[i] = seg ? i * ne : (int32_t)(ptr[r0 + i] - e0);
+        __syncwarp();
+        const int32_t pairs = (r1 - r0) * W;
+        for (int32_t pr = lane; pr < pairs; pr += 32) {
+            const int32_t rr = pr / W, col = pr % W;
+            const int64_t row = r0 + rr;
+            const bool on = row_on(ra, row, t);
+            const int32_t q0 = sp[rr], q1 = on && t * TILE + col < kcols ? sp[rr + 1] : q0;
+            T acc = spmm_row<T>(si, sv, q0, q1, xt + col);
+            if (!on) continue;
+            if (seg) {
+                lpart[(int64_t)c * ld + t * TILE + col] = acc;
+            } else {
+                // q streams out (evict-first), so it does not push the gathered slab out of L2
+                const int64_t o = toff + row * TILE + col;
+                if (ACC) acc += __ldcs(q + o);
+                __stcs(q + o, acc);
+                if (part) dot += (double)acc * (double)xt[row * TILE + col];
+            }
+        }
+        __syncwarp();
+    }
+    if (part) {
         s_red[threadIdx.x] = dot;
         __syncthreads();
         if (threadIdx.x < TILE) {
@@ -810,19 +837,64 @@ __global__ void __launch_bounds__(CH_THREADS, MINB)
     }
 }
 
+// the long rows: their segments' sums in order into q, and their share of p.q (grid: x over rows, y over tiles)
+template <class T, bool ACC>
+__global__ void __launch_bounds__(CH_THREADS) k_spmm_long(int64_t n, SpmmItems S, const T* __restrict__ lpart,
+                                                          const T* __restrict__ p, T* __restrict__ q, int64_t ld,
+                                                          double* __restrict__ part, int32_t kcols, RowAct ra) {
+    __shared__ double s_red[CH_THREADS];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t t = blockIdx.y, toff = t * n * TILE;
+    const bool live = t * TILE + lane < kcols;  // a narrow product leaves the other columns' partials unset
+    double dot = 0.0;
+    for (int32_t i = blockIdx.x * CH_WARPS + w; i < S.nlong; i += gridDim.x * CH_WARPS) {
+        const int64_t row = S.lrow[i];
+        if (!row_on(ra, row, t)) continue;
+        T acc = 0;
+#pragma unroll 4
+        for (int32_t g = S.lseg[i]; g < S.lseg[i + 1] && live; g++) acc += lpart[(int64_t)g * ld + t * TILE + lane];
+        const int64_t o = toff + row * TILE + lane;
+        if (ACC) acc += q[o];
+        q[o] = acc;
+        dot += (double)acc * (double)p[o];
+    }
+    if (part) {
+        s_red[threadIdx.x] = dot;
+        __syncthreads();
+        if (threadIdx.x < TILE) {
+            double tt = 0.0;
+            for (int i = 0; i < CH_WARPS; i++) tt += s_red[i * 32 + threadIdx.x];
+            part[(int64_t)blockIdx.x * ld + t * TILE + threadIdx.x] = tt;
+        }
+    }
+}
+
+// Four squared differences' sums over a warp, each as the xor butterfly over offsets 16, 8, 4, 2, 1 would form it (the
+// same operands added in the same order), in 6 shuffles of a double instead of 20: the first two steps hand half
+// of the values to the other half of the lanes.  Lane 8 v gets value v.
+__device__ __forceinline__ double warp_sum4(double s0, double s1, double s2, double s3, int lane) {
+    const bool h = lane & 16, g = lane & 8;
+    const double a = __dadd_rn(h ? s2 : s0, __shfl_xor_sync(0xffffffffu, h ? s0 : s2, 16));
+    const double b = __dadd_rn(h ? s3 : s1, __shfl_xor_sync(0xffffffffu, h ? s1 : s3, 16));
+    double c = __dadd_rn(g ? b : a, __shfl_xor_sync(0xffffffffu, g ? a : b, 8));
+#pragma unroll
+    for (int o = 4; o >= 1; o >>= 1) c = __dadd_rn(c, __shfl_xor_sync(0xffffffffu, c, o));
+    return c;
+}
+
 // The final product of a solve, one tile per launch, also forming the squared diff norms of the edges from
 // the rows it gathers: the edge of an entry with row < column (eid >= 0) gets, per tile, the xor-butterfly
 // sum over the tile's 32 columns of (x[row] - x[col])^2 (0 for columns past k), added to d2 in tile order
-// (first: stored) -- diff_norms_device's order.  All 32 lanes of a warp walk the same row and entry, so the
-// eid test and the butterfly are warp-uniform.  q with four accumulators (eight gathers in flight with
-// interleaved butterflies need 64 registers and ran slower: 1260 against 1231 ms per ER 1M step).
-__global__ void __launch_bounds__(CH_THREADS) k_spmm_diff(int64_t n, const int32_t* __restrict__ cstart,
-                                                          int32_t nchunks, const int64_t* __restrict__ ptr,
+// (first: stored) -- diff_norms_device's order.  All 32 lanes of a warp walk the same row, eight gathers in flight; a
+// group of four entries without an edge skips the sums.  Long rows are cut into segments as in k_spmm.  With four gathers
+// in flight, 20 shuffles per edge and whole rows a launch took 0.38 ms at ER n = 250,000, 1.38 at ER n = 1M and 1.15 on
+// k_spmm's R-MAT graph (its hubs); here 0.32, 1.25 and 0.08.
+__global__ void __launch_bounds__(CH_THREADS) k_spmm_diff(int64_t n, SpmmItems S, const int64_t* __restrict__ ptr,
                                                           const int32_t* __restrict__ idx,
                                                           const double* __restrict__ val,
                                                           const int32_t* __restrict__ eid, const double* xt,
                                                           double* qt, int32_t kcols, double* __restrict__ d2,
-                                                          int first) {
+                                                          int first, double* __restrict__ lpart, int64_t ld) {
     __shared__ int32_t s_idx[CH_WARPS][CHUNK_CAP];
     __shared__ double s_val[CH_WARPS][CHUNK_CAP];
     __shared__ int32_t s_eid[CH_WARPS][CHUNK_CAP];
@@ -833,76 +905,56 @@ __global__ void __launch_bounds__(CH_THREADS) k_spmm_diff(int64_t n, const int32
     double* sv = s_val[w];
     int32_t* se = s_eid[w];
     int32_t* sp = s_ptr[w];
-    // one entry: its gathered value g, and the squared difference into d2 when the entry names an edge
-    auto edge = [&](int32_t e, double xo, double g) {
-        if (e < 0) return;  // warp-uniform
-        const double dx = live ? __dsub_rn(xo, g) : 0.0;
-        double sq = __dmul_rn(dx, dx);
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) sq = __dadd_rn(sq, __shfl_xor_sync(0xffffffffu, sq, o));
-        if (lane == 0) d2[e] = first ? sq : __dadd_rn(d2[e], sq);
-    };
-    for (int32_t c = blockIdx.x * CH_WARPS + w; c < nchunks; c += gridDim.x * CH_WARPS) {
-        const int32_t r0 = cstart[c], r1 = cstart[c + 1];
-        const int64_t e0 = ptr[r0], e1 = ptr[r1];
-        const int64_t ne = e1 - e0;
-        if (ne <= CHUNK_CAP) {
-            for (int64_t i = lane; i < ne; i += 32) {
-                si[i] = __ldcs(idx + e0 + i);
-                sv[i] = __ldcs(val + e0 + i);
-                se[i] = __ldcs(eid + e0 + i);
-            }
-            for (int32_t i = lane; i <= r1 - r0; i += 32) sp[i] = (int32_t)(ptr[r0 + i] - e0);
-            __syncwarp();
-            for (int32_t rr = 0; rr < r1 - r0; rr++) {
-                const int64_t row = r0 + rr;
-                const double xo = live ? xt[row * TILE + lane] : 0.0;
-                const int32_t q0 = sp[rr], q1 = sp[rr + 1];
-                double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-                int32_t q = q0;
-                for (; q + 3 < q1; q += 4) {
-                    const double g0 = live ? xt[(int64_t)si[q] * TILE + lane] : 0.0;
-                    const double g1 = live ? xt[(int64_t)si[q + 1] * TILE + lane] : 0.0;
-                    const double g2 = live ? xt[(int64_t)si[q + 2] * TILE + lane] : 0.0;
-                    const double g3 = live ? xt[(int64_t)si[q + 3] * TILE + lane] : 0.0;
-                    a0 += sv[q] * g0;
-                    a1 += sv[q + 1] * g1;
-                    a2 += sv[q + 2] * g2;
-                    a3 += sv[q + 3] * g3;
-                    edge(se[q], xo, g0);
-                    edge(se[q + 1], xo, g1);
-                    edge(se[q + 2], xo, g2);
-                    edge(se[q + 3], xo, g3);
-                }
-                for (; q < q1; q++) {
-                    const double g = live ? xt[(int64_t)si[q] * TILE + lane] : 0.0;
-                    a0 += sv[q] * g;
-                    edge(se[q], xo, g);
-                }
-                __stcs(qt + row * TILE + lane, (a0 + a1) + (a2 + a3));
-            }
-            __syncwarp();
-        } else {
-            // one long row, lane = column
-            const double xo = live ? xt[(int64_t)r0 * TILE + lane] : 0.0;
-            double a0 = 0, a1 = 0;
-            int64_t q = e0;
-            for (; q + 1 < e1; q += 2) {
-                const int32_t i0 = __ldcs(idx + q), i1 = __ldcs(idx + q + 1);
-                const double g0 = live ? xt[(int64_t)i0 * TILE + lane] : 0.0;
-                const double g1 = live ? xt[(int64_t)i1 * TILE + lane] : 0.0;
-                a0 += __ldcs(val + q) * g0;
-                a1 += __ldcs(val + q + 1) * g1;
-                edge(__ldcs(eid + q), xo, g0);
-                edge(__ldcs(eid + q + 1), xo, g1);
-            }
-            if (q < e1) {
-                const double g = live ? xt[(int64_t)__ldcs(idx + q) * TILE + lane] : 0.0;
-                a0 += __ldcs(val + q) * g;
-                edge(__ldcs(eid + q), xo, g);
-            }
-            __stcs(qt + (int64_t)r0 * TILE + lane, a0 + a1);
+    for (int32_t c = blockIdx.x * CH_WARPS + w; c < S.nseg + S.nchunks; c += gridDim.x * CH_WARPS) {
+        const bool seg = c < S.nseg;
+        const int32_t r0 = seg ? S.segrow[c] : S.chunks[c - S.nseg], r1 = seg ? r0 + 1 : S.chunks[c - S.nseg + 1];
+        const int64_t e0 = seg ? S.seg[c] : ptr[r0];
+        const int64_t e1 = seg ? min(e0 + CHUNK_CAP, ptr[r1]) : ptr[r1];
+        const int32_t ne = (int32_t)(e1 - e0);
+        if (ne > CHUNK_CAP) continue;
+        for (int32_t i = lane; i < ne; i += 32) {
+            si[i] = __ldcs(idx + e0 + i);
+            sv[i] = __ldcs(val + e0 + i);
+            se[i] = __ldcs(eid + e0 + i);
         }
+        for (int32_t i = lane; i <= r1 - r0; i += 32) sp[i] = seg ? i * ne : (int32_t)(ptr[r0 + i] - e0);
+        __syncwarp();
+        for (int32_t rr = 0; rr < r1 - r0; rr++) {
+            const int64_t row = r0 + rr;
+            const double xo = live ? xt[row * TILE + lane] : 0.0;
+            const int32_t q0 = sp[rr], q1 = sp[rr + 1];
+            double a[4] = {0, 0, 0, 0};
+            for (int32_t q = q0; q < q1; q += 8) {
+                double g[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) g[u] = live && q + u < q1 ? xt[(int64_t)si[q + u] * TILE + lane] : 0.0;
+#pragma unroll
+                for (int h = 0; h < 8; h += 4) {
+                    int32_t any = -1;
+#pragma unroll
+                    for (int u = h; u < h + 4; u++)
+                        if (q + u < q1) {
+                            a[u & 3] += sv[q + u] * g[u];
+                            any = max(any, se[q + u]);
+                        }
+                    if (any < 0) continue;  // warp-uniform
+                    double sq[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const double dx = live ? __dsub_rn(xo, g[h + u]) : 0.0;
+                        sq[u] = __dmul_rn(dx, dx);
+                    }
+                    const double sum = warp_sum4(sq[0], sq[1], sq[2], sq[3], lane);
+                    const int v = h + (lane >> 3);
+                    const int32_t e = (lane & 7) == 0 && q + v < q1 ? se[q + v] : -1;
+                    if (e >= 0) d2[e] = first ? sum : __dadd_rn(d2[e], sum);
+                }
+            }
+            const double sum = (a[0] + a[1]) + (a[2] + a[3]);
+            if (seg) lpart[(int64_t)c * ld + lane] = sum;
+            else __stcs(qt + row * TILE + lane, sum);
+        }
+        __syncwarp();
     }
 }
 
@@ -1129,19 +1181,20 @@ struct LevelEvents {
 template <int MODE, class T, int MINB>
 static void launch_level_w(int code, dim3 grid, cudaStream_t s, int64_t n, const int32_t* ch, int32_t nc,
                            const int64_t* ptr, const int32_t* idx, const T* val, const int32_t* rowmap, T* y,
-                           const T* aux, int64_t ld, int32_t kcols, int nsub, const T* dlast, const RowAct& ra) {
+                           const T* aux, int32_t kcols, int nsub, const T* dlast, const RowAct& ra) {
     switch (code) {
     case 0:
-        k_chunked<MODE, T, 8, MINB><<<grid, CH_THREADS, 0, s>>>(n, ch, nc, ptr, idx, val, rowmap, y, y, aux, ld,
-                                                                nullptr, kcols, nsub, dlast, ra);
+        k_chunked<MODE, T, 8, MINB><<<grid, CH_THREADS, 0, s>>>(n, ch, nc, ptr, idx, val, rowmap, y, y, aux, kcols,
+                                                                nsub, dlast, ra);
         break;
     case 1:
         k_chunked<MODE, T, (TILE >= 16 ? 16 : 8), MINB><<<grid, CH_THREADS, 0, s>>>(
-            n, ch, nc, ptr, idx, val, rowmap, y, y, aux, ld, nullptr, kcols, nsub, dlast, ra);
+            n, ch, nc, ptr, idx, val, rowmap, y, y, aux, kcols,
+                                                                nsub, dlast, ra);
         break;
     default:
-        k_chunked<MODE, T, TILE, MINB><<<grid, CH_THREADS, 0, s>>>(n, ch, nc, ptr, idx, val, rowmap, y, y, aux, ld,
-                                                                   nullptr, kcols, nsub, dlast, ra);
+        k_chunked<MODE, T, TILE, MINB><<<grid, CH_THREADS, 0, s>>>(n, ch, nc, ptr, idx, val, rowmap, y, y, aux, kcols,
+                                                                nsub, dlast, ra);
         break;
     }
 }
@@ -1339,13 +1392,13 @@ static int64_t launch_precond(Context& C, const DevFactor& F, const TrsvPlan& P,
         if (lev) lev->begin(C.stream, fwd, l);
         if (last)
             launch_level_w<M_FWD_LAST, T, MINB_FWD>(code, grid, C.stream, n, ch, nc, F.prow_ptr, F.prow_idx,
-                                                    V.prow_val, F.level_rows, y, r, ld, kcols, ns, V.D, ra);
+                                                    V.prow_val, F.level_rows, y, r, kcols, ns, V.D, ra);
         else if (fwd)
             launch_level_w<M_FWD, T, MINB_FWD>(code, grid, C.stream, n, ch, nc, F.prow_ptr, F.prow_idx, V.prow_val,
-                                               F.level_rows, y, r, ld, kcols, ns, nullptr, ra);
+                                               F.level_rows, y, r, kcols, ns, nullptr, ra);
         else
             launch_level_w<M_BWD, T, MINB_BWD>(code, grid, C.stream, n, ch, nc, F.pcol_ptr, F.pcol_idx, V.pcol_val,
-                                               F.level_cols, y, V.D, ld, kcols, ns, nullptr, ra);
+                                               F.level_cols, y, V.D, kcols, ns, nullptr, ra);
         if (lev) lev->end(C.stream);
         launches++;
     };
@@ -1363,7 +1416,7 @@ static int64_t launch_precond(Context& C, const DevFactor& F, const TrsvPlan& P,
         const int ns = narrow ? 1 : TILE / trsv_width(code);
         launch_level_w<M_FWD, T, MINB_FWD>(code, dim3((unsigned)chunk_blocks(F.ntchunk), (unsigned)(ntiles * ns)),
                                            C.stream, n, F.tchunk, F.ntchunk, F.tin_ptr, F.tin_idx, V.tin_val,
-                                           F.level_rows + (F.n - F.tail_rows), y, r, ld, kcols, ns, nullptr, ra);
+                                           F.level_rows + (F.n - F.tail_rows), y, r, kcols, ns, nullptr, ra);
         launches += 1 + launch_tail<T>(C, F, V.linv, V.D, y, V.tail_tmp, ntiles);
     }
     for (size_t i = P.bw.size(); i-- > 0;) {
@@ -1567,9 +1620,12 @@ struct SpmmPlan {
     const int64_t* ptr = nullptr;  // nslabs * n + 1 row pointers
     const int32_t* idx = nullptr;
     const double* val = nullptr;  // FP64 values in this entry order
-    const int32_t* chunks[MAX_SLABS] = {};
-    int32_t nchunks[MAX_SLABS] = {};
-    dim3 grid;
+    SpmmItems items[MAX_SLABS];   // of each slab
+    dim3 grid;                    // of k_spmm
+    unsigned long_blocks = 0;     // x blocks of k_spmm_long for the last slab (p.q partials follow the grid's)
+    int nparts = 0;               // partials of p.q per column
+    int launches = 0;             // of one product
+    double* lpart = nullptr;      // sums of the long rows' segments (both precisions)
     double* part = nullptr;
 };
 
@@ -1682,23 +1738,70 @@ static SpmmPlan make_spmm_plan(Context& C, int64_t n, const int64_t* lap_ptr, co
     }
     SSP_CUDA(cudaMemcpyAsync(hp.data(), A.ptr, sizeof(int64_t) * hp.size(), cudaMemcpyDeviceToHost, C.stream));
     SSP_CUDA(cudaStreamSynchronize(C.stream));
-    std::vector<int32_t> all;
-    std::vector<size_t> off(m);
-    int32_t most = 0;
+    // per slab: the chunks, and the segments of the rows longer than one
+    std::vector<int32_t> i32;
+    std::vector<int64_t> i64;
+    struct Off {
+        size_t chunks, segrow, lrow, lseg, seg;
+    };
+    std::vector<Off> off(m);
+    int32_t most = 0, most_seg = 0;
     for (int32_t b = 0; b < m; b++) {
-        off[b] = all.size();
-        const size_t before = all.size();
-        make_chunks(hp.data() + (size_t)b * n, 0, (int32_t)n, all);
-        A.nchunks[b] = (int32_t)(all.size() - before);
-        most = std::max(most, A.nchunks[b]);
-        all.push_back((int32_t)n);
+        const int64_t* bp = hp.data() + (size_t)b * n;
+        SpmmItems& I = A.items[b];
+        std::vector<int32_t> ch, segrow, lrow, lseg;
+        make_chunks(bp, 0, (int32_t)n, ch);
+        I.nchunks = (int32_t)ch.size();
+        ch.push_back((int32_t)n);
+        off[b].seg = i64.size();
+        for (int32_t c = 0; c < I.nchunks; c++) {
+            const int64_t e0 = bp[ch[c]], e1 = bp[ch[c + 1]];
+            if (e1 - e0 <= CHUNK_CAP) continue;
+            lrow.push_back(ch[c]);
+            lseg.push_back((int32_t)segrow.size());
+            for (int64_t e = e0; e < e1; e += CHUNK_CAP) {
+                segrow.push_back(ch[c]);
+                i64.push_back(e);
+            }
+        }
+        lseg.push_back((int32_t)segrow.size());
+        I.nseg = (int32_t)segrow.size();
+        I.nlong = (int32_t)lrow.size();
+        auto add = [&](const std::vector<int32_t>& v) {
+            const size_t at = i32.size();
+            i32.insert(i32.end(), v.begin(), v.end());
+            return at;
+        };
+        off[b].chunks = add(ch);
+        off[b].segrow = add(segrow);
+        off[b].lrow = add(lrow);
+        off[b].lseg = add(lseg);
+        most = std::max(most, I.nchunks + I.nseg);
+        most_seg = std::max(most_seg, I.nseg);
     }
-    int32_t* d = W.get_t<int32_t>("pcg_achunks", all.size());
-    SSP_CUDA(cudaMemcpyAsync(d, all.data(), sizeof(int32_t) * all.size(), cudaMemcpyHostToDevice, C.stream));
-    for (int32_t b = 0; b < m; b++) A.chunks[b] = d + off[b];
+    int32_t* d = W.get_t<int32_t>("pcg_achunks", i32.size());
+    int64_t* d64 = W.get_t<int64_t>("pcg_aseg", i64.size() + 1);
+    SSP_CUDA(cudaMemcpyAsync(d, i32.data(), sizeof(int32_t) * i32.size(), cudaMemcpyHostToDevice, C.stream));
+    if (!i64.empty())
+        SSP_CUDA(cudaMemcpyAsync(d64, i64.data(), sizeof(int64_t) * i64.size(), cudaMemcpyHostToDevice, C.stream));
+    SSP_CUDA(cudaStreamSynchronize(C.stream));
+    for (int32_t b = 0; b < m; b++) {
+        SpmmItems& I = A.items[b];
+        I.chunks = d + off[b].chunks;
+        I.segrow = d + off[b].segrow;
+        I.lrow = d + off[b].lrow;
+        I.lseg = d + off[b].lseg;
+        I.seg = d64 + off[b].seg;
+    }
     const int bx = chunk_blocks(most);
     A.grid = dim3((unsigned)bx, (unsigned)(ld / TILE));
-    A.part = W.get_t<double>("pcg_spmm_part", (size_t)bx * ld);
+    const int32_t nl = A.items[m - 1].nlong;
+    A.long_blocks = nl ? (unsigned)std::min(ceil_div(nl, CH_WARPS), 64) : 0;
+    A.nparts = bx + (int)A.long_blocks;
+    A.launches = m;
+    for (int32_t b = 0; b < m; b++) A.launches += A.items[b].nlong > 0;
+    A.lpart = most_seg ? W.get_t<double>("pcg_lpart", (size_t)most_seg * ld) : nullptr;
+    A.part = W.get_t<double>("pcg_spmm_part", (size_t)A.nparts * ld);
     return A;
 }
 
@@ -1707,21 +1810,19 @@ template <class T>
 static void launch_spmm(Context& C, int64_t n, const SpmmPlan& A, const T* aval, const T* p, T* q, int64_t ld,
                         bool dot, int32_t kcols, const RowAct& ra = RowAct()) {
     const bool narrow = TILE > NARROW_W && kcols <= NARROW_W;
+    T* lpart = reinterpret_cast<T*>(A.lpart);
     for (int32_t b = 0; b < A.nslabs; b++) {
+        const SpmmItems& I = A.items[b];
         const int64_t* ptr = A.ptr + (int64_t)b * n;
         double* part = dot && b == A.nslabs - 1 ? A.part : nullptr;
-#define SSP_SPMM_LAUNCH(MODE, W_)                                                                                  \
-    k_chunked<MODE, T, W_, MINB_SPMM><<<A.grid, CH_THREADS, 0, C.stream>>>(n, A.chunks[b], A.nchunks[b], ptr, A.idx,  \
-                                                                            aval, nullptr, p, q, nullptr, ld, part,    \
-                                                                            kcols, 1, nullptr, ra)
-        if (b == 0) {
-            if (narrow) SSP_SPMM_LAUNCH(M_SPMM, NARROW_W);
-            else SSP_SPMM_LAUNCH(M_SPMM, TILE);
-        } else {
-            if (narrow) SSP_SPMM_LAUNCH(M_SPMM_ACC, NARROW_W);
-            else SSP_SPMM_LAUNCH(M_SPMM_ACC, TILE);
-        }
-#undef SSP_SPMM_LAUNCH
+        auto kern = narrow ? (b == 0 ? k_spmm<T, NARROW_W, false> : k_spmm<T, NARROW_W, true>)
+                           : (b == 0 ? k_spmm<T, TILE, false> : k_spmm<T, TILE, true>);
+        kern<<<A.grid, CH_THREADS, 0, C.stream>>>(n, I, ptr, A.idx, aval, p, q, ld, lpart, part, kcols, ra);
+        if (I.nlong == 0) continue;
+        const dim3 grid(part ? A.long_blocks : (unsigned)std::min(ceil_div(I.nlong, CH_WARPS), 64), A.grid.y);
+        auto fin = b == 0 ? k_spmm_long<T, false> : k_spmm_long<T, true>;
+        fin<<<grid, CH_THREADS, 0, C.stream>>>(n, I, lpart, p, q, ld, part ? part + (int64_t)A.grid.x * ld : nullptr, kcols,
+                                               ra);
     }
 }
 
@@ -1894,7 +1995,7 @@ static int32_t pcg_solve(Context& C, int64_t n, int32_t k, int64_t ld, const Spm
     // with several graphs the SpMM's blocks straddle graphs, so p.q is a segmented reduction of its own
     auto pq_dot = [&]() {
         if (G.nseg > 1) R.run<OP_DOT, T>(B.p, B.q, S.pq);
-        else colred_final(C, ld, (int)A.grid.x, A.part, S.pq);
+        else colred_final(C, ld, A.nparts, A.part, S.pq);
     };
     // which (graph, tile) pairs still have an active column: the row kernels skip the others
     auto update_act = [&]() {
@@ -1953,7 +2054,7 @@ static int32_t pcg_solve(Context& C, int64_t n, int32_t k, int64_t ld, const Spm
         k_axpy_r_rr<T><<<dim3((unsigned)R.nparts, (unsigned)ntiles), RED_THREADS, 0, C.stream>>>(
             n, S.alpha, B.q, B.r, R.rows_per_blk, ld, R.part, G);
         SSP_CHECK_LAUNCH();
-        C.kernels_launched += 3 + A.nslabs;
+        C.kernels_launched += 3 + A.launches;
         R.finish(S.rr);
         it++;
         SSP_CUDA(cudaMemsetAsync(S.nactive, 0, sizeof(int64_t), C.stream));
@@ -2053,7 +2154,7 @@ static int32_t pcg_solve(Context& C, int64_t n, int32_t k, int64_t ld, const Spm
             SSP_CHECK_LAUNCH();
         });
         // the helpers count theirs; with several graphs p.q is a reduction (counted) instead of a final pass
-        body_kernels += (C.kernels_launched - k_before) + 9 + A.nslabs - (G.nseg > 1 ? 1 : 0);
+        body_kernels += (C.kernels_launched - k_before) + 9 + A.launches - (G.nseg > 1 ? 1 : 0);
         C.kernels_launched = k_before;
         SSP_CUDA(cudaGraphInstantiate(&L.exec, L.graph, 0));
         SSP_CUDA(cudaGraphLaunch(L.exec, C.stream));
@@ -2273,7 +2374,7 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
             k_true_resid<<<dim3((unsigned)R.nparts, (unsigned)ntiles), RED_THREADS, 0, C.stream>>>(
                 n, k, Y, mean, q, r, R.rows_per_blk, ld, R.part, R.G);
             SSP_CHECK_LAUNCH();
-            C.kernels_launched += 1 + A.nslabs;
+            C.kernels_launched += 1 + A.launches;
             R.finish(relres);
             SSP_CUDA(cudaMemsetAsync(S.nactive, 0, sizeof(int64_t), C.stream));
             SSP_CUDA(cudaMemsetAsync(worst, 0, sizeof(double), C.stream));
@@ -2294,15 +2395,21 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
     if (lap_eid && d2 && A.nslabs == 1) {
         for (int64_t t = 0; t < ntiles; t++)
             k_spmm_diff<<<dim3(A.grid.x, 1), CH_THREADS, 0, C.stream>>>(
-                n, A.chunks[0], A.nchunks[0], A.ptr, A.idx, A.val, lap_eid, x + t * n * TILE, q + t * n * TILE,
-                (int32_t)(k - t * TILE), d2, (t == 0 && !d2_accumulate) ? 1 : 0);
+                n, A.items[0], A.ptr, A.idx, A.val, lap_eid, x + t * n * TILE, q + t * n * TILE,
+                (int32_t)(k - t * TILE), d2, (t == 0 && !d2_accumulate) ? 1 : 0, A.lpart ? A.lpart + t * TILE : nullptr, ld);
         SSP_CHECK_LAUNCH();
         C.kernels_launched += ntiles;
+        if (A.items[0].nlong) {
+            k_spmm_long<double, false><<<dim3(A.long_blocks, (unsigned)ntiles), CH_THREADS, 0, C.stream>>>(
+                n, A.items[0], A.lpart, x, q, ld, nullptr, k, RowAct());
+            SSP_CHECK_LAUNCH();
+            C.kernels_launched++;
+        }
         rep.diff_fused = true;
     } else {
         launch_spmm<double>(C, n, A, A.val, x, q, ld, false, k);
         SSP_CHECK_LAUNCH();
-        C.kernels_launched += A.nslabs;
+        C.kernels_launched += A.launches;
     }
     R.run<OP_SQDIFF_CENTERED, double>(Y, q, relres, mean);
     std::vector<double> hb(ns), hr(ns);
