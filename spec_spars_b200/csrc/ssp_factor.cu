@@ -62,6 +62,8 @@ struct FDev {
     int32_t* fill_a;
     int32_t* fill_b;
     double* fill_w;
+    int32_t* incoming;  // [vertex] fill entries of this level for its bag (0 between levels)
+    int32_t* owners;    // the vertices of the level's fill
 };
 
 __device__ __forceinline__ bool key_less(const uint64_t* prio, int32_t a, int32_t b) {
@@ -134,11 +136,10 @@ __global__ void k_init_count(FDev F, int32_t* frontier) {
 }
 
 // warp per frontier vertex: live entries, L and fill reservations, tier lists
-__global__ void k_live_count(FDev F, const int32_t* frontier, int32_t* live_cnt, int32_t* list_b, int32_t* list_g) {
-    int64_t nf = F.ctr[C_NEXT];
-    int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+__device__ void live_count(const FDev& F, const int32_t* frontier, int32_t* live_cnt, int32_t* list_b, int32_t* list_g,
+                           int64_t warp, int64_t nw) {
+    const int64_t nf = F.ctr[C_NEXT];
+    const int lane = threadIdx.x & 31;
     for (int64_t i = warp; i < nf; i += nw) {
         int32_t v = frontier[i];
         int64_t s = F.bag_start[v];
@@ -161,6 +162,11 @@ __global__ void k_live_count(FDev F, const int32_t* frontier, int32_t* live_cnt,
                 list_g[atomicAdd((unsigned long long*)&F.ctr[C_NG], 1ull)] = (int32_t)i;
         }
     }
+}
+
+#define SSP_WARP_OF_GRID ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, ((int64_t)gridDim.x * blockDim.x) >> 5
+__global__ void k_live_count(FDev F, const int32_t* frontier, int32_t* live_cnt, int32_t* list_b, int32_t* list_g) {
+    live_count(F, frontier, live_cnt, list_b, list_g, SSP_WARP_OF_GRID);
 }
 
 // ---------------------------------------------------------------- elimination (shared tail)
@@ -190,25 +196,31 @@ __device__ __forceinline__ void emit_slot(const FDev& F, int32_t v, int64_t fidx
             F.fill_b[fp] = b;
             F.fill_w[fp] = wf;
             atomicAdd(&F.count[key_less(F.prio, b, a) ? a : b], 1);
+            if (atomicAdd(&F.incoming[a], 1) == 0) F.owners[atomicAdd((unsigned long long*)&F.ctr[C_OWNERS], 1ull)] = a;
+            if (atomicAdd(&F.incoming[b], 1) == 0) F.owners[atomicAdd((unsigned long long*)&F.ctr[C_OWNERS], 1ull)] = b;
         }
     }
 }
 
+// One entry of an eliminated vertex' bag: its live neighbour u loses a predecessor.  A vertex comes here after all of
+// its fill is counted, so a count that reaches 0 has seen all of the level's fill at u: u is free.
+__device__ __forceinline__ void release_entry(const FDev& F, int32_t u, int32_t* next) {
+    if (atomicSub(&F.count[u], 1) == 1) next[atomicAdd((unsigned long long*)&F.ctr[C_NEXT], 1ull)] = u;
+}
+
 // Warp tier: <= 32 live entries, all in registers.
-__global__ void __launch_bounds__(128) k_elim_warp(FDev F, const int32_t* frontier, const int32_t* live_cnt) {
+// s_mu, s_mw, s_c: 32 slots for each warp of the block.
+__device__ void elim_warp(const FDev& F, const int32_t* frontier, int32_t* next, int32_t lvl, const int32_t* live_cnt,
+                          int32_t (*s_mu)[32], double (*s_mw)[32], double (*s_c)[32], int64_t warp, int64_t nw) {
     const int64_t nf = F.ctr[C_REM];  // frontier size of this level
     const int lane = threadIdx.x & 31;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t fi = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; fi < nf; fi += nw) {
+    for (int64_t fi = warp; fi < nf; fi += nw) {
         const int32_t L = live_cnt[fi];
         if (L > 32) continue;
         const int32_t v = frontier[fi];
         const int64_t s = F.bag_start[v];
         const int32_t len = F.bag_len[v];
         // gather live entries (order irrelevant: sorted next) through a per-warp staging area
-        __shared__ int32_t s_mu[4][32];
-        __shared__ double s_mw[4][32];
-        __shared__ double s_c[4][32];
         const int wib = threadIdx.x >> 5;
         int32_t got = 0;
         for (int32_t q0 = 0; q0 < len; q0 += 32) {
@@ -243,6 +255,7 @@ __global__ void __launch_bounds__(128) k_elim_warp(FDev F, const int32_t* fronti
                 F.D[v] = 0.0;
                 F.Lcnt[v] = 0;
                 F.fcnt[fi] = 0;
+                F.level[v] = lvl;
             }
             continue;
         }
@@ -257,6 +270,7 @@ __global__ void __launch_bounds__(128) k_elim_warp(FDev F, const int32_t* fronti
             int32_t ou = __shfl_down_sync(0xffffffffu, u, t);
             if (cont && lane + t < got && ou == u) sum = sum + ow;
             else cont = false;
+            if (!__any_sync(0xffffffffu, cont)) break;  // few entries come twice
         }
         const unsigned hmask = __ballot_sync(0xffffffffu, head);
         const int32_t cnt = __popc(hmask);
@@ -291,8 +305,55 @@ __global__ void __launch_bounds__(128) k_elim_warp(FDev F, const int32_t* fronti
             if (cnt > 1) atomicAdd((unsigned long long*)&F.ctr[C_NFILL], (unsigned long long)(cnt - 1));
             if (cnt > 1 && F.vseg)
                 atomicAdd((unsigned long long*)&F.gctr[3 * F.vseg[v] + GC_NFILL], (unsigned long long)(cnt - 1));
+            F.level[v] = lvl;
         }
         __syncwarp();
+        if (lane < got) release_entry(F, u, next);
+    }
+}
+
+__global__ void __launch_bounds__(128)
+    k_elim_warp(FDev F, const int32_t* frontier, int32_t* next, int32_t lvl, const int32_t* live_cnt) {
+    __shared__ int32_t s_mu[4][32];
+    __shared__ double s_mw[4][32];
+    __shared__ double s_c[4][32];
+    elim_warp(F, frontier, next, lvl, live_cnt, s_mu, s_mw, s_c, SSP_WARP_OF_GRID);
+}
+
+// Sorts the entries (mu, mw)[0 .. cnt) into (ou, ow), by (u, w) or by (w, u): 2^lg threads per entry count the entries
+// before it, one barrier instead of the bitonic network's one per stage.  Weights compare by their bits, a total order
+// (equal entries keep theirs), so the positions are a permutation for NaN too.
+constexpr int RANK_SORT_MAX = 512;  // entries; at most one for each thread
+template <bool W_FIRST>
+__device__ __forceinline__ void block_rank_sort(const int32_t* mu, const double* mw, int32_t cnt, int32_t* ou, double* ow) {
+    auto key = [](double w) {
+        const long long x = __double_as_longlong(w);
+        return x ^ ((x >> 63) & 0x7fffffffffffffffll);
+    };
+    int lg = 0;
+    while (lg < 5 && (cnt << (lg + 1)) <= (int)blockDim.x) lg++;
+    const int g = threadIdx.x & ((1 << lg) - 1);
+    for (int32_t i0 = 0; i0 < cnt; i0 += (int)blockDim.x >> lg) {  // block-uniform
+        const int32_t i = i0 + (int)(threadIdx.x >> lg);
+        const bool in = i < cnt;
+        const int32_t u = in ? mu[i] : 0;
+        const double w = in ? mw[i] : 0.0;
+        const long long k = key(w);
+        int32_t before = 0;
+        if (in)
+            for (int32_t j = g; j < cnt; j += 1 << lg) {
+                const int32_t uj = mu[j];
+                const long long kj = key(mw[j]);
+                const bool first = W_FIRST ? kj < k || (kj == k && (uj < u || (uj == u && j < i)))
+                                           : uj < u || (uj == u && (kj < k || (kj == k && j < i)));
+                before += first ? 1 : 0;
+            }
+        __syncwarp();
+        for (int o = 1; o < 1 << lg; o <<= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+        if (in && g == 0) {
+            ou[before] = u;
+            ow[before] = w;
+        }
     }
 }
 
@@ -376,12 +437,23 @@ __device__ int32_t block_gather_merge(const FDev& F, int32_t v, int32_t L, int32
         }
     }
     __syncthreads();
-    for (int32_t i = L + threadIdx.x; i < P; i += blockDim.x) {
-        su[i] = INT32_MAX;
-        sw[i] = __longlong_as_double(0x7ff0000000000000ll);
+    if (L <= min(RANK_SORT_MAX, (int)blockDim.x)) {
+        // counted into (mu, mw), which are free until the merged entries go there
+        block_rank_sort<false>(su, sw, L, mu, mw);
+        __syncthreads();
+        for (int32_t i = threadIdx.x; i < L; i += blockDim.x) {
+            su[i] = mu[i];
+            sw[i] = mw[i];
+        }
+        __syncthreads();
+    } else {
+        for (int32_t i = L + threadIdx.x; i < P; i += blockDim.x) {
+            su[i] = INT32_MAX;
+            sw[i] = __longlong_as_double(0x7ff0000000000000ll);
+        }
+        __syncthreads();
+        block_bitonic_ent(su, sw, P, EntUW());
     }
-    __syncthreads();
-    block_bitonic_ent(su, sw, P, EntUW());
     // heads and run sums
     int32_t cnt = 0;
     for (int32_t base = 0; base < L; base += blockDim.x) {
@@ -404,8 +476,9 @@ __device__ int32_t block_gather_merge(const FDev& F, int32_t v, int32_t L, int32
     return cnt;
 }
 
+// (su, sw): scratch of cnt entries
 __device__ void block_finish_column(const FDev& F, int32_t v, int64_t fidx, int32_t cnt, int32_t* mu, double* mw,
-                                    double* sc, double* s_carry) {
+                                    double* sc, double* s_carry, int32_t* su, double* sw) {
     if (cnt == 0) {
         if (threadIdx.x == 0) {
             F.D[v] = 0.0;
@@ -415,14 +488,21 @@ __device__ void block_finish_column(const FDev& F, int32_t v, int64_t fidx, int3
         __syncthreads();
         return;
     }
-    int P = 2;
-    while (P < cnt) P <<= 1;
-    for (int32_t i = cnt + threadIdx.x; i < P; i += blockDim.x) {
-        mu[i] = INT32_MAX;
-        mw[i] = __longlong_as_double(0x7ff0000000000000ll);
+    if (cnt <= min(RANK_SORT_MAX, (int)blockDim.x)) {
+        block_rank_sort<true>(mu, mw, cnt, su, sw);
+        __syncthreads();
+        mu = su;
+        mw = sw;
+    } else {
+        int P = 2;
+        while (P < cnt) P <<= 1;
+        for (int32_t i = cnt + threadIdx.x; i < P; i += blockDim.x) {
+            mu[i] = INT32_MAX;
+            mw[i] = __longlong_as_double(0x7ff0000000000000ll);
+        }
+        __syncthreads();
+        block_bitonic_ent(mu, mw, P, EntWU());
     }
-    __syncthreads();
-    block_bitonic_ent(mu, mw, P, EntWU());
     block_chunk_scan(mw, sc, cnt, s_carry);
     const double S = sc[cnt - 1];
     for (int32_t i = threadIdx.x; i < cnt; i += blockDim.x) emit_slot(F, v, fidx, i, cnt, mu, mw, sc, S);
@@ -439,9 +519,25 @@ __device__ void block_finish_column(const FDev& F, int32_t v, int64_t fidx, int3
     __syncthreads();
 }
 
+// One block eliminates frontier vertex fi.
+__device__ void elim_block(const FDev& F, int32_t fi, const int32_t* frontier, int32_t* next, int32_t lvl, int32_t L,
+                           int32_t cap, int32_t* su, double* sw, int32_t* mu, double* mw, double* sc, double* s_carry,
+                           int32_t* s_warp, int32_t* s_cnt) {
+    const int32_t v = frontier[fi];
+    const int32_t cnt = block_gather_merge(F, v, L, cap, su, sw, mu, mw, s_warp, s_cnt);
+    block_finish_column(F, v, fi, cnt, mu, mw, sc, s_carry, su, sw);
+    const int64_t s = F.bag_start[v];
+    const int32_t len = F.bag_len[v];
+    for (int32_t q = threadIdx.x; q < len; q += blockDim.x) {
+        const int32_t u = F.pool_u[s + q];
+        if (F.level[u] < 0) release_entry(F, u, next);
+    }
+    if (threadIdx.x == 0) F.level[v] = lvl;
+}
+
 // Block tier (shared memory) and global tier (scratch slices), one block per vertex.
-__global__ void k_elim_block(FDev F, const int32_t* frontier, const int32_t* live_cnt, const int32_t* list,
-                             int64_t nlist_idx, int32_t cap, int32_t* g_u, double* g_w) {
+__global__ void k_elim_block(FDev F, const int32_t* frontier, int32_t* next, int32_t lvl, const int32_t* live_cnt,
+                             const int32_t* list, int64_t nlist_idx, int32_t cap, int32_t* g_u, double* g_w) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int32_t s_warp[33];
     __shared__ int32_t s_cnt;
@@ -449,8 +545,6 @@ __global__ void k_elim_block(FDev F, const int32_t* frontier, const int32_t* liv
     const int64_t nlist = F.ctr[nlist_idx];
     for (int64_t li = blockIdx.x; li < nlist; li += gridDim.x) {
         const int32_t fi = list[li];
-        const int32_t v = frontier[fi];
-        const int32_t L = live_cnt[fi];
         int32_t *su, *mu;
         double *sw, *mw, *sc, *s_carry;
         if (g_u) {  // global scratch: 2 int arrays + 3 double arrays of cap, carry after
@@ -469,54 +563,18 @@ __global__ void k_elim_block(FDev F, const int32_t* frontier, const int32_t* liv
             mu = su + cap;
             s_carry = s_carry_static;
         }
-        int32_t cnt = block_gather_merge(F, v, L, cap, su, sw, mu, mw, s_warp, &s_cnt);
-        block_finish_column(F, v, fi, cnt, mu, mw, sc, s_carry);
+        elim_block(F, fi, frontier, next, lvl, live_cnt[fi], cap, su, sw, mu, mw, sc, s_carry, s_warp, &s_cnt);
     }
 }
 
-// ---------------------------------------------------------------- release / fill bookkeeping
-__global__ void k_release(FDev F, const int32_t* frontier, int32_t* next, int32_t lvl) {
-    const int64_t nf = F.ctr[C_REM];
-    const int lane = threadIdx.x & 31;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t fi = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; fi < nf; fi += nw) {
-        const int32_t v = frontier[fi];
-        const int64_t s = F.bag_start[v];
-        const int32_t len = F.bag_len[v];
-        for (int32_t q = lane; q < len; q += 32) {
-            int32_t u = F.pool_u[s + q];
-            if (F.level[u] >= 0) continue;
-            int32_t old = atomicSub(&F.count[u], 1);
-            if (old == 1) next[atomicAdd((unsigned long long*)&F.ctr[C_NEXT], 1ull)] = u;
-        }
-        __syncwarp();
-        if (lane == 0) F.level[v] = lvl;
-    }
-}
-
-__global__ void k_fill_incoming(FDev F, int32_t* incoming, int32_t* owners) {
-    const int64_t nf = F.ctr[C_REM];
-    const int lane = threadIdx.x & 31;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t fi = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; fi < nf; fi += nw) {
-        const int64_t s = F.fstart[fi];
-        const int32_t c = F.fcnt[fi];
-        for (int32_t q = lane; q < c; q += 32) {
-            int32_t a = F.fill_a[s + q], b = F.fill_b[s + q];
-            if (atomicAdd(&incoming[a], 1) == 0) owners[atomicAdd((unsigned long long*)&F.ctr[C_OWNERS], 1ull)] = a;
-            if (atomicAdd(&incoming[b], 1) == 0) owners[atomicAdd((unsigned long long*)&F.ctr[C_OWNERS], 1ull)] = b;
-        }
-    }
-}
-
+// ---------------------------------------------------------------- fill bookkeeping
 // warp per owner: make room for the incoming fill (relocate, dropping stale entries)
-__global__ void k_reserve(FDev F, int32_t* incoming, const int32_t* owners) {
+__device__ void reserve(const FDev& F, int64_t warp, int64_t nw) {
     const int64_t no = F.ctr[C_OWNERS];
     const int lane = threadIdx.x & 31;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t oi = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; oi < no; oi += nw) {
-        const int32_t a = owners[oi];
-        const int32_t inc = incoming[a];
+    for (int64_t oi = warp; oi < no; oi += nw) {
+        const int32_t a = F.owners[oi];
+        const int32_t inc = F.incoming[a];
         const int32_t len = F.bag_len[a];
         if (len + inc > F.bag_cap[a]) {
             const int64_t s = F.bag_start[a];
@@ -558,15 +616,17 @@ __global__ void k_reserve(FDev F, int32_t* incoming, const int32_t* owners) {
             }
         }
         __syncwarp();
-        if (lane == 0) incoming[a] = 0;
+        if (lane == 0) F.incoming[a] = 0;
     }
 }
+__global__ void k_reserve(FDev F) {
+    reserve(F, SSP_WARP_OF_GRID);
+}
 
-__global__ void k_fill_scatter(FDev F) {
+__device__ void fill_scatter(const FDev& F, int64_t warp, int64_t nw) {
     const int64_t nf = F.ctr[C_REM];
     const int lane = threadIdx.x & 31;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t fi = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; fi < nf; fi += nw) {
+    for (int64_t fi = warp; fi < nf; fi += nw) {
         const int64_t s = F.fstart[fi];
         const int32_t c = F.fcnt[fi];
         for (int32_t q = lane; q < c; q += 32) {
@@ -587,6 +647,178 @@ __global__ void k_fill_scatter(FDev F) {
                 atomicOr((unsigned long long*)&F.ctr[C_ERR], (unsigned long long)FERR_OVERFLOW);
             }
         }
+    }
+}
+__global__ void k_fill_scatter(FDev F) {
+    fill_scatter(F, SSP_WARP_OF_GRID);
+}
+
+// ---------------------------------------------------------------- many levels in one launch
+// The levels of small frontiers, which are most: latency alone counts there (an elimination of 32 entries is a chain of
+// five dependent loads and two sorts; the host loop's launches and its wait for the counters come on top).  One cooperative
+// launch, a block per SM, runs level after level with four barriers over its blocks: on B200 30-37 us a level for
+// frontiers of 30-320 vertices where launches and a read-back took about 95 (the factors of a 30k-vertex geometric
+// graph 32 -> 24.5 ms, of a 40^3 grid 27.5 -> 22).  It starts with a level whose capacities the host has checked, and
+// at every level boundary takes the host loop's own decisions on the same numbers; what it does not handle (a
+// truncation, the dense tail, a pool to compact, buffers to grow, bags above ELIM_LIVE_MAX, wide frontiers) ends it
+// there, and the host loop goes on from the state it leaves.
+// ELIM_FRONT_MAX: 3.5 vertices for each warp of the grid; such a level takes 86-90 us here, as in the host loop, and wider
+// ones are better spread over the launches' larger grids.  ELIM_LIVE_MAX: what fits the static shared memory.
+enum { ST_LIVE = 0, ST_ELIM, ST_LVL, ST_PREV, ST_LUSED, ST_STOP, ST_ERR, ST_N };
+constexpr int ELIM_THREADS = 256, ELIM_LIVE_MAX = 512;
+constexpr int64_t ELIM_FRONT_MAX = 4096;
+
+struct ElimArgs {
+    FDev F;
+    int32_t* front[2];  // frontier of the first level and the other list, in turn
+    int32_t *live_cnt, *list_b, *list_g;
+    int64_t* st;             // ST_*
+    unsigned* bar;           // arrivals, releases
+    int32_t* log;            // frontier size by level
+    int64_t max_degree, dense_threshold, pool_init, pool_cap, Lcap, Fcap;
+    // several graphs: per graph its vertices, truncation, and the accounting of ST_LIVE, ST_ELIM, ST_PREV
+    const int64_t *g_n, *g_max;
+    int64_t *g_live, *g_elim, *g_prev;
+};
+
+// Barrier over the grid; the last block to arrive runs ctl (all its threads) before the others go on.  The wait is
+// bounded: after a few seconds the kernel reports ST_ERR and ends.  Returns false then.
+template <class Ctl>
+__device__ bool grid_barrier(const ElimArgs& A, Ctl ctl) {
+    __shared__ unsigned s_ticket;
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_ticket = atomicAdd(&A.bar[0], 1u);
+        s_ok = 1;
+    }
+    __syncthreads();
+    const unsigned round = s_ticket / gridDim.x;
+    if (s_ticket % gridDim.x == gridDim.x - 1) {
+        if (threadIdx.x == 0) __threadfence();
+        __syncthreads();
+        ctl();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicExch(&A.bar[1], round + 1);
+        }
+    } else if (threadIdx.x == 0) {
+        int spins = 0;
+        while ((int)(*(volatile unsigned*)&A.bar[1] - (round + 1)) < 0) {
+            if (++spins > 1024) __nanosleep(100);
+            if (spins > (1 << 23)) {
+                atomicExch((unsigned long long*)&A.st[ST_ERR], 1ull);
+                s_ok = 0;
+                break;
+            }
+        }
+    }
+    if (threadIdx.x == 0) __threadfence();
+    __syncthreads();
+    return s_ok != 0;
+}
+
+__global__ void __launch_bounds__(ELIM_THREADS) k_elim_levels(ElimArgs A) {
+    constexpr int NWARP = ELIM_THREADS / 32;
+    __shared__ int32_t s_mu[NWARP][32];
+    __shared__ double s_mw[NWARP][32];
+    __shared__ double s_c[NWARP][32];
+    __shared__ int32_t b_su[ELIM_LIVE_MAX], b_mu[ELIM_LIVE_MAX];
+    __shared__ double b_sw[ELIM_LIVE_MAX], b_mw[ELIM_LIVE_MAX], b_sc[ELIM_LIVE_MAX];
+    __shared__ double s_carry[ELIM_LIVE_MAX / 32 + 1];
+    __shared__ int32_t s_warp[33];
+    __shared__ int32_t s_cnt;
+    const FDev& F = A.F;
+    const int wib = threadIdx.x >> 5;
+    const int64_t warp = (int64_t)blockIdx.x * NWARP + wib, nw = (int64_t)gridDim.x * NWARP;
+    int64_t* ctr = F.ctr;
+    auto nothing = [] {};
+    // the level begins: its frontier is the list just counted
+    auto begin = [&] {
+        if (threadIdx.x == 0) {
+            const int64_t nf = ctr[C_NEXT];
+            A.log[A.st[ST_LVL]] = (int32_t)nf;
+            A.st[ST_LUSED] = ctr[C_LCUR];
+            A.st[ST_PREV] = ctr[C_FCUR];
+            A.st[ST_ELIM] += nf;
+            ctr[C_REM] = nf;
+            ctr[C_NEXT] = 0;
+            ctr[C_OWNERS] = 0;
+            ctr[C_NFILL] = 0;
+        }
+        for (int32_t g = threadIdx.x; g < F.nseg; g += ELIM_THREADS) {
+            A.g_prev[g] = F.gctr[3 * g + GC_FCUR];
+            A.g_elim[g] += F.gctr[3 * g + GC_NFRONT];
+            F.gctr[3 * g + GC_NFILL] = 0;
+        }
+    };
+    // the boundary after a level, with the upcoming frontier counted: the host loop's tests in its order
+    auto boundary = [&] {
+        __shared__ int s_stop;
+        if (threadIdx.x == 0) {
+            const int64_t nf = ctr[C_NEXT], n = F.n, elim = A.st[ST_ELIM], maxlive = ctr[C_MAXLIVE];
+            const int64_t live = A.st[ST_LIVE] + 2 * ctr[C_NFILL] - 2 * A.st[ST_PREV];
+            const int64_t reserve = 2 * (A.pool_init + 2 * ctr[C_FCUR]) + 16 * (n - elim) + 1024;
+            s_stop = ctr[C_ERR] != 0 || nf == 0 || nf > ELIM_FRONT_MAX || ctr[C_NG] > 0 || maxlive > ELIM_LIVE_MAX ||
+                     (F.nseg == 0 && A.max_degree > 0 && live > A.max_degree * (n - elim)) || elim + nf > n ||
+                     (A.dense_threshold > 0 && n - elim <= A.dense_threshold && nf <= DENSE_FRONTIER_MAX) ||
+                     ctr[C_POOL] + reserve > A.pool_cap || ctr[C_LCUR] > A.Lcap || ctr[C_FCUR] > A.Fcap;
+        }
+        __syncthreads();
+        for (int32_t g = threadIdx.x; g < F.nseg; g += ELIM_THREADS) {
+            const int64_t live = A.g_live[g] + (A.g_prev[g] >= 0 ? 2 * F.gctr[3 * g + GC_NFILL] - 2 * A.g_prev[g] : 0);
+            if (A.g_max[g] > 0 && F.gctr[3 * g + GC_NFRONT] > 0 && live > A.g_max[g] * (A.g_n[g] - A.g_elim[g])) s_stop = 1;
+        }
+        __syncthreads();
+        if (s_stop) {
+            if (threadIdx.x == 0) A.st[ST_STOP] = 1;
+            return;
+        }
+        for (int32_t g = threadIdx.x; g < F.nseg; g += ELIM_THREADS)
+            if (A.g_prev[g] >= 0) A.g_live[g] += 2 * F.gctr[3 * g + GC_NFILL] - 2 * A.g_prev[g];
+        if (threadIdx.x == 0) A.st[ST_LIVE] += 2 * ctr[C_NFILL] - 2 * A.st[ST_PREV];
+        __syncthreads();
+        begin();
+    };
+    if (!grid_barrier(A, begin)) return;
+    for (int cur = 0;; cur ^= 1) {
+        const int32_t* frontier = A.front[cur];
+        int32_t* next = A.front[cur ^ 1];
+        const int32_t lvl = (int32_t)A.st[ST_LVL];
+        // eliminate: some blocks take the bags above 32 live entries, the others' warps the rest
+        const int64_t nlist = ctr[C_NB], nrest = ctr[C_REM] - nlist;
+        const int nb = (int)min(nlist, (int64_t)gridDim.x - min((nrest + NWARP - 1) / NWARP, (int64_t)gridDim.x / 2));
+        if ((int)blockIdx.x < nb) {
+            for (int64_t li = blockIdx.x; li < nlist; li += nb) {
+                const int32_t fi = A.list_b[li];
+                elim_block(F, fi, frontier, next, lvl, A.live_cnt[fi], ELIM_LIVE_MAX, b_su, b_sw, b_mu, b_mw, b_sc,
+                           s_carry, s_warp, &s_cnt);
+            }
+        } else {
+            elim_warp(F, frontier, next, lvl, A.live_cnt, s_mu, s_mw, s_c, warp - (int64_t)nb * NWARP,
+                      nw - (int64_t)nb * NWARP);
+        }
+        if (!grid_barrier(A, nothing)) return;
+        reserve(F, warp, nw);
+        if (blockIdx.x == 0) {  // (nothing below reads these before the next barrier)
+            if (threadIdx.x == 0) {
+                ctr[C_FCUR] = 0;
+                ctr[C_NB] = 0;
+                ctr[C_NG] = 0;
+                ctr[C_MAXLIVE] = 0;
+                A.st[ST_LVL] = lvl + 1;
+            }
+            for (int32_t g = threadIdx.x; g < F.nseg; g += ELIM_THREADS)
+                F.gctr[3 * g + GC_FCUR] = F.gctr[3 * g + GC_NFRONT] = 0;
+        }
+        if (!grid_barrier(A, nothing)) return;
+        fill_scatter(F, warp, nw);
+        if (!grid_barrier(A, nothing)) return;
+        live_count(F, next, A.live_cnt, A.list_b, A.list_g, warp, nw);
+        if (!grid_barrier(A, boundary)) return;
+        if (A.st[ST_STOP]) return;
     }
 }
 
@@ -712,30 +944,7 @@ __global__ void k_dense_build(FDev F, const int32_t* rem, int32_t T, const int32
     }
 }
 
-// Sorted position of every entry of (mu, mw)[0 .. cnt) by counting the entries before it in (w, u) order: 2^lg threads per
-// entry compare it with all others (u is unique, so the order is total), one barrier instead of the bitonic network's
-// one per stage.  (ou, ow) receive the sorted entries.
-__device__ __forceinline__ void block_rank_sort(const int32_t* mu, const double* mw, int32_t cnt, int32_t* ou, double* ow) {
-    int lg = 0;
-    while (lg < 5 && (cnt << (lg + 1)) <= (int)blockDim.x) lg++;
-    const int g = threadIdx.x & ((1 << lg) - 1);
-    for (int32_t i0 = 0; i0 < cnt; i0 += (int)blockDim.x >> lg) {  // block-uniform
-        const int32_t i = i0 + (int)(threadIdx.x >> lg);
-        const bool in = i < cnt;
-        const int32_t u = in ? mu[i] : 0;
-        const double w = in ? mw[i] : 0.0;
-        int32_t before = 0;
-        if (in)
-            for (int32_t j = g; j < cnt; j += 1 << lg) before += EntWU()(mu[j], mw[j], u, w) ? 1 : 0;
-        __syncwarp();
-        for (int o = 1; o < 1 << lg; o <<= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
-        if (in && g == 0) {
-            ou[before] = u;
-            ow[before] = w;
-        }
-    }
-}
-constexpr int RANK_SORT_MAX = 512;  // entries; counting is quadratic
+  // entries; counting is quadratic
 
 // Single block: eliminate the T remaining vertices in key order.  A chain of T columns, so what counts is the latency
 // of one: the row's nonzeros are collected in any order (their keys are unique), ranked, scanned in 32-wide chunks
@@ -780,7 +989,7 @@ __global__ void __launch_bounds__(1024) k_dense_elim(FDev F, const int32_t* rem,
         int32_t* su = mu;
         double* sw = mw;
         if (cnt <= RANK_SORT_MAX) {
-            block_rank_sort(mu, mw, cnt, s_u, s_w);
+            block_rank_sort<true>(mu, mw, cnt, s_u, s_w);
             su = s_u;
             sw = s_w;
         } else {
@@ -1178,11 +1387,11 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
     int32_t* live_cnt = W.get_t<int32_t>(nm("live_cnt"), n);
     int32_t* list_b = W.get_t<int32_t>(nm("list_b"), n);
     int32_t* list_g = W.get_t<int32_t>(nm("list_g"), n);
-    int32_t* incoming = W.get_t<int32_t>(nm("incoming"), n);
-    int32_t* owners = W.get_t<int32_t>(nm("owners"), n);
+    F.incoming = W.get_t<int32_t>(nm("incoming"), n);
+    F.owners = W.get_t<int32_t>(nm("owners"), n);
     F.fstart = W.get_t<int64_t>(nm("fstart"), n);
     F.fcnt = W.get_t<int32_t>(nm("fcnt"), n);
-    SSP_CUDA(cudaMemsetAsync(incoming, 0, sizeof(int32_t) * n, C.stream));
+    SSP_CUDA(cudaMemsetAsync(F.incoming, 0, sizeof(int32_t) * n, C.stream));
     k_init_count<<<grid_for(n * 32, T256, 148 * 64), T256, 0, C.stream>>>(F, next);
     SSP_CHECK_LAUNCH();
     C.kernels_launched++;
@@ -1370,6 +1579,68 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
             F.fill_b = W.get_t<int32_t>(nm("fill_b"), Fcap);
             F.fill_w = W.get_t<double>(nm("fill_w"), Fcap);
         }
+        if (nf <= ELIM_FRONT_MAX && h[C_NG] == 0 && h[C_MAXLIVE] <= ELIM_LIVE_MAX) {
+            // this level and those after it, up to one that needs the host
+            int64_t st[ST_N] = {live_entries, eliminated, lvl, -1, Lused_prev, 0, 0};
+            int64_t* d_st = W.get_t<int64_t>(nm("el_st"), ST_N + 1);
+            int64_t* d_g = W.get_t<int64_t>(nm("el_g"), 5 * (size_t)nseg + 1);
+            int32_t* d_log = W.get_t<int32_t>(nm("el_log"), n + 1);
+            std::vector<int64_t> hg;
+            for (int32_t g = 0; g < nseg; g++) hg.push_back(opt.seg_row0[g + 1] - opt.seg_row0[g]);
+            // a stopped graph has no vertex in a frontier any more, so its test never holds again
+            for (const auto* v : {&g_maxdeg, &g_live, &g_elim, &g_prev}) hg.insert(hg.end(), v->begin(), v->end());
+            SSP_CUDA(cudaMemcpyAsync(d_st, st, sizeof(st), cudaMemcpyHostToDevice, C.stream));
+            SSP_CUDA(cudaMemsetAsync(d_st + ST_N, 0, sizeof(int64_t), C.stream));
+            if (nseg)
+                SSP_CUDA(cudaMemcpyAsync(d_g, hg.data(), sizeof(int64_t) * hg.size(), cudaMemcpyHostToDevice, C.stream));
+            ElimArgs A;
+            A.F = F;
+            A.front[0] = next;
+            A.front[1] = frontier;
+            A.live_cnt = live_cnt;
+            A.list_b = list_b;
+            A.list_g = list_g;
+            A.st = d_st;
+            A.bar = (unsigned*)(d_st + ST_N);
+            A.log = d_log;
+            A.max_degree = opt.max_degree;
+            A.dense_threshold = opt.dense_threshold;
+            A.pool_init = pool_init;
+            A.pool_cap = pool_cap;
+            A.Lcap = Lcap;
+            A.Fcap = Fcap;
+            A.g_n = d_g;
+            A.g_max = d_g + nseg;
+            A.g_live = d_g + 2 * nseg;
+            A.g_elim = d_g + 3 * nseg;
+            A.g_prev = d_g + 4 * nseg;
+            int sms = 0;
+            SSP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, C.device));
+            void* args[] = {&A};
+            SSP_CUDA(cudaLaunchCooperativeKernel((const void*)k_elim_levels, dim3((unsigned)sms), dim3(ELIM_THREADS), args, 0,
+                                                 C.stream));
+            C.kernels_launched++;
+            read_i64s(C, d_st, st, ST_N);
+            if (st[ST_ERR]) throw Error(SSP_ERR_CUDA, "factor: a level's barrier was not reached in time");
+            const int32_t done = (int32_t)st[ST_LVL] - lvl;
+            std::vector<int32_t> sizes(done);
+            SSP_CUDA(cudaMemcpyAsync(sizes.data(), d_log + lvl, sizeof(int32_t) * done, cudaMemcpyDeviceToHost, C.stream));
+            if (nseg) {
+                read_i64s(C, A.g_live, g_live.data(), nseg);
+                read_i64s(C, A.g_elim, g_elim.data(), nseg);
+                read_i64s(C, A.g_prev, g_prev.data(), nseg);
+            }
+            SSP_CUDA(cudaStreamSynchronize(C.stream));
+            out.frontier_sizes.pop_back();
+            out.frontier_sizes.insert(out.frontier_sizes.end(), sizes.begin(), sizes.end());
+            live_entries = st[ST_LIVE];
+            eliminated = st[ST_ELIM];
+            lvl = (int32_t)st[ST_LVL];
+            prev_fcur = st[ST_PREV];
+            Lused_prev = st[ST_LUSED];
+            if (done & 1) std::swap(frontier, next);
+            continue;
+        }
         Lused_prev = h[C_LCUR];
         prev_fcur = h[C_FCUR];
         for (int32_t g = 0; g < nseg; g++) {
@@ -1378,7 +1649,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
         }
         std::swap(frontier, next);
         k_level_begin<<<1, 1, 0, C.stream>>>(F.ctr, F.gctr, F.nseg);  // REM <- NEXT (frontier size), NEXT <- 0
-        k_elim_warp<<<grid_for(nf * 32, 128, 148 * 64), 128, 0, C.stream>>>(F, frontier, live_cnt);
+        k_elim_warp<<<grid_for(nf * 32, 128, 148 * 64), 128, 0, C.stream>>>(F, frontier, next, lvl, live_cnt);
         SSP_CHECK_LAUNCH();
         C.kernels_launched += 2;
         if (h[C_NB] > 0) {
@@ -1386,7 +1657,8 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
             while (cap < std::min<int64_t>(h[C_MAXLIVE], BLOCK_TIER_MAX)) cap <<= 1;
             size_t smem = (size_t)cap * (3 * sizeof(double) + 2 * sizeof(int32_t));
             int blocks = (int)std::min<int64_t>(h[C_NB], 148 * 4);
-            k_elim_block<<<blocks, 256, smem, C.stream>>>(F, frontier, live_cnt, list_b, C_NB, cap, nullptr, nullptr);
+            k_elim_block<<<blocks, 256, smem, C.stream>>>(F, frontier, next, lvl, live_cnt, list_b, C_NB, cap, nullptr,
+                                                       nullptr);
             SSP_CHECK_LAUNCH();
             C.kernels_launched++;
         }
@@ -1396,17 +1668,15 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
             int blocks = (int)std::min<int64_t>(h[C_NG], 32);
             int32_t* gu = W.get_t<int32_t>(nm("gscr_u"), (size_t)2 * cap * blocks);
             double* gw = W.get_t<double>(nm("gscr_w"), (size_t)4 * cap * blocks);
-            k_elim_block<<<blocks, 1024, 0, C.stream>>>(F, frontier, live_cnt, list_g, C_NG, cap, gu, gw);
+            k_elim_block<<<blocks, 1024, 0, C.stream>>>(F, frontier, next, lvl, live_cnt, list_g, C_NG, cap, gu, gw);
             SSP_CHECK_LAUNCH();
             C.kernels_launched++;
         }
         const int gw32 = grid_for(nf * 32, T256, 148 * 64);
-        k_release<<<gw32, T256, 0, C.stream>>>(F, frontier, next, lvl);
-        k_fill_incoming<<<gw32, T256, 0, C.stream>>>(F, incoming, owners);
-        k_reserve<<<grid_for(n * 32, T256, 148 * 64), T256, 0, C.stream>>>(F, incoming, owners);
+        k_reserve<<<grid_for(n * 32, T256, 148 * 64), T256, 0, C.stream>>>(F);
         k_fill_scatter<<<gw32, T256, 0, C.stream>>>(F);
         SSP_CHECK_LAUNCH();
-        C.kernels_launched += 4;
+        C.kernels_launched += 2;
         eliminated += nf;
         lvl++;
         live_count(next);
