@@ -30,6 +30,7 @@
 namespace ssp {
 
 constexpr int TILE = SSP_TILE;    // columns per tile
+constexpr int RED_BLOCKS = 6;     // ... resident per SM: one wave of them is the grid
 constexpr int RED_THREADS = 256;  // column reductions: (256 / TILE) row lanes x TILE columns
 
 // mixed precision: relative reduction asked of one FP32 inner solve, and the round limit
@@ -134,38 +135,77 @@ __global__ void k_seg_tile_active(int32_t nseg, int32_t ntiles, int64_t ld, cons
 // ---------------------------------------------------------------- column reductions
 enum ColOp { OP_SUM = 0, OP_DOT = 1, OP_SQ = 2, OP_SQDIFF_CENTERED = 3 };
 
-// grid (nparts, ntiles); thread = (row lane = tid / 8, column = tid % 8); part[blk][col]
-template <int OP, class T>
-__global__ void __launch_bounds__(RED_THREADS) k_colred_partial(int64_t n, const T* __restrict__ a,
-                                                                const T* __restrict__ b,
-                                                                const double* __restrict__ mean, int64_t rows_per_blk,
-                                                                int64_t ld, double* __restrict__ part, SegDev G) {
-    __shared__ double s[RED_THREADS];
-    const int64_t t = blockIdx.y;
-    const int c = threadIdx.x % TILE, rl = threadIdx.x / TILE;
-    int64_t r0, r1, sb;
-    red_block(G, n, rows_per_blk, ld, r0, r1, sb);
-    const T* at = a + t * n * TILE;
-    const T* bt = b ? b + t * n * TILE : nullptr;
-    const double mu = (OP == OP_SQDIFF_CENTERED) ? mean[sb + t * TILE + c] : 0.0;
-    double acc = 0.0;
-    for (int64_t r = r0 + rl; r < r1; r += RED_THREADS / TILE) {
-        const double x = (double)at[r * TILE + c];
-        if (OP == OP_SUM) acc += x;
-        else if (OP == OP_DOT) acc += x * (double)bt[r * TILE + c];
-        else if (OP == OP_SQ) acc += x * x;
-        else {
-            const double d = (x - mu) - (double)bt[r * TILE + c];  // (Y - mean) - A x
-            acc += d * d;
-        }
-    }
-    s[threadIdx.x] = acc;
+// 16 bytes of a tile's row: a thread of the vector kernels below has these columns of every RROWS<T>-th row of its block.
+template <class T>
+struct alignas(16) Vec {
+    static constexpr int V = 16 / sizeof(T);
+    T v[V];
+};
+template <class T>
+__device__ __forceinline__ Vec<T> vec_at(const T* p) {
+    return *reinterpret_cast<const Vec<T>*>(p);
+}
+template <class T>
+__device__ __forceinline__ void vec_to(T* p, const Vec<T>& x) {
+    *reinterpret_cast<Vec<T>*>(p) = x;
+}
+template <class T>
+constexpr int RROWS = RED_THREADS * Vec<T>::V / TILE;
+
+// the block's per-column sums of acc (thread: columns c ..), row lanes in order
+template <class T>
+__device__ __forceinline__ void block_part(const double (&acc)[Vec<T>::V], int64_t t, int64_t ld, double* part) {
+    __shared__ double s[RED_THREADS * Vec<T>::V];
+#pragma unroll
+    for (int u = 0; u < Vec<T>::V; u++) s[threadIdx.x * Vec<T>::V + u] = acc[u];
     __syncthreads();
     if (threadIdx.x < TILE) {
         double tt = s[threadIdx.x];
-        for (int i = 1; i < RED_THREADS / TILE; i++) tt += s[i * TILE + threadIdx.x];
+        for (int i = 1; i < RROWS<T>; i++) tt += s[i * TILE + threadIdx.x];
         part[(int64_t)blockIdx.x * ld + t * TILE + threadIdx.x] = tt;
     }
+}
+
+// Grid (nparts, ntiles); part[blk][col].  These stream their operands once, so the bound is DRAM: 16-byte loads, two rows of a
+// thread in flight, and a grid of one wave (148 x RED_BLOCKS; a few blocks more, as before, ran alone afterwards).
+// Measured on B200 with a lane per value -> here, over 1185-1194 columns: r.z at ER n = 250,000 FP64 868 -> 671 us (7.1 TB/s),
+// at n = 229,373 FP32 553 -> 339 (6.4); r -= alpha q 1.29 -> 1.19 ms (6.0) and 653 -> 600 us (5.4).  The rows of a block stay
+// contiguous: taken in turn by all blocks, r -= alpha q took 1.31 ms.
+template <int OP, class T>
+__global__ void __launch_bounds__(RED_THREADS, RED_BLOCKS) k_colred_partial(int64_t n, const T* __restrict__ a,
+                                                                const T* __restrict__ b,
+                                                                const double* __restrict__ mean, int64_t rows_per_blk,
+                                                                int64_t ld, double* __restrict__ part, SegDev G) {
+    constexpr int V = Vec<T>::V;
+    const int64_t t = blockIdx.y;
+    const int c = threadIdx.x * V % TILE, rl = threadIdx.x * V / TILE;
+    int64_t r0, r1, sb;
+    red_block(G, n, rows_per_blk, ld, r0, r1, sb);
+    const T* at = a + t * n * TILE + c;
+    const T* bt = b ? b + t * n * TILE + c : nullptr;
+    double mu[V], acc[V];
+#pragma unroll
+    for (int u = 0; u < V; u++) {
+        mu[u] = (OP == OP_SQDIFF_CENTERED) ? mean[sb + t * TILE + c + u] : 0.0;
+        acc[u] = 0.0;
+    }
+#pragma unroll 2
+    for (int64_t r = r0 + rl; r < r1; r += RROWS<T>) {
+        const Vec<T> x = vec_at(at + r * TILE);
+        Vec<T> y;
+        if (OP == OP_DOT || OP == OP_SQDIFF_CENTERED) y = vec_at(bt + r * TILE);
+#pragma unroll
+        for (int u = 0; u < V; u++) {
+            if (OP == OP_SUM) acc[u] += (double)x.v[u];
+            else if (OP == OP_DOT) acc[u] += (double)x.v[u] * (double)y.v[u];
+            else if (OP == OP_SQ) acc[u] += (double)x.v[u] * (double)x.v[u];
+            else {
+                const double d = ((double)x.v[u] - mu[u]) - (double)y.v[u];  // (Y - mean) - A x
+                acc[u] += d * d;
+            }
+        }
+    }
+    block_part<T>(acc, t, ld, part);
 }
 
 // out[c] = sum over parts of part[i][c]: a block per 32 columns, warp w sums the parts i = w (mod FIN_WARPS) two
@@ -221,7 +261,7 @@ struct Reducer {
         ld = ld_;
         G = segs;
         const int64_t ntiles = ld / TILE;
-        int64_t target = std::max<int64_t>(8, std::min<int64_t>(1184 / std::max<int64_t>(1, ntiles) + 1, 1024));
+        int64_t target = std::max<int64_t>(8, std::min<int64_t>(148 * RED_BLOCKS / std::max<int64_t>(1, ntiles), 1024));
         rows_per_blk = std::max<int64_t>(RED_THREADS / TILE, ceil_div<int64_t>(n, target));
         if (G.nseg <= 1 || !row0) {
             nparts = (int)ceil_div<int64_t>(n, rows_per_blk);
@@ -300,50 +340,84 @@ __global__ void k_center(int64_t n, int32_t k, int64_t ld, const double* __restr
 // the next p update (k_update_xp), which reads p anyway, or to k_axpy_x after the last iteration: x gets
 // the same additions in the same order, one n x k stream fewer per iteration.
 template <class T>
-__global__ void __launch_bounds__(RED_THREADS) k_axpy_r_rr(int64_t n, const double* __restrict__ alpha,
+__global__ void __launch_bounds__(RED_THREADS, RED_BLOCKS) k_axpy_r_rr(int64_t n, const double* __restrict__ alpha,
                                                            const T* __restrict__ q, T* __restrict__ r,
                                                            int64_t rows_per_blk, int64_t ld, double* __restrict__ part,
                                                            SegDev G) {
-    __shared__ double s[RED_THREADS];
+    constexpr int V = Vec<T>::V;
     const int64_t t = blockIdx.y;
-    const int c = threadIdx.x % TILE, rl = threadIdx.x / TILE;
+    const int c = threadIdx.x * V % TILE, rl = threadIdx.x * V / TILE;
     int64_t r0, r1, sb;
     red_block(G, n, rows_per_blk, ld, r0, r1, sb);
-    const double a64 = alpha[sb + t * TILE + c];
-    const T a = (T)a64;
-    const int64_t base = t * n * TILE;
-    double acc = 0.0;
-    for (int64_t row = r0 + rl; row < r1; row += RED_THREADS / TILE) {
-        const int64_t o = base + row * TILE + c;
-        T rv = r[o];
-        if (a64 != 0.0) {
-            rv -= a * q[o];
-            r[o] = rv;
+    double a64[V], acc[V];
+    bool any = false;
+#pragma unroll
+    for (int u = 0; u < V; u++) {
+        a64[u] = alpha[sb + t * TILE + c + u];
+        any |= a64[u] != 0.0;
+        acc[u] = 0.0;
+    }
+    const int64_t base = t * n * TILE + c;
+    auto row_done = [&](Vec<T> rv, const Vec<T>& qv, int64_t o) {
+        if (any) {
+#pragma unroll
+            for (int u = 0; u < V; u++)
+                if (a64[u] != 0.0) rv.v[u] -= (T)a64[u] * qv.v[u];
+            vec_to(r + o, rv);
         }
-        acc += (double)rv * (double)rv;
+#pragma unroll
+        for (int u = 0; u < V; u++) acc[u] += (double)rv.v[u] * (double)rv.v[u];
+    };
+    int64_t row = r0 + rl;
+    for (; row + RROWS<T> < r1; row += 2 * RROWS<T>) {  // both rows' loads before the first store
+        const int64_t o0 = base + row * TILE, o1 = o0 + RROWS<T> * TILE;
+        const Vec<T> ra = vec_at(r + o0), rb = vec_at(r + o1);
+        Vec<T> qa = {}, qb = {};
+        if (any) {
+            qa = vec_at(q + o0);
+            qb = vec_at(q + o1);
+        }
+        row_done(ra, qa, o0);
+        row_done(rb, qb, o1);
     }
-    s[threadIdx.x] = acc;
-    __syncthreads();
-    if (threadIdx.x < TILE) {
-        double tt = s[threadIdx.x];
-        for (int i = 1; i < RED_THREADS / TILE; i++) tt += s[i * TILE + threadIdx.x];
-        part[(int64_t)blockIdx.x * ld + t * TILE + threadIdx.x] = tt;
+    if (row < r1) {
+        const int64_t o = base + row * TILE;
+        const Vec<T> ra = vec_at(r + o);
+        row_done(ra, any ? vec_at(q + o) : Vec<T>{}, o);
     }
+    block_part<T>(acc, t, ld, part);
 }
 
-// x += alpha p (the previous step's alpha and p), then p = z + beta p
+// x += alpha p (the previous step's alpha and p), then p = z + beta p.  Five streams in 16-byte pieces (FP32 5.4 GB:
+// 1.09 -> 0.94 ms; FP64 stays at 6.7 TB/s)
 template <class T>
 __global__ void k_update_xp(int64_t n, int64_t ld, const double* __restrict__ alpha, const double* __restrict__ beta,
                             const T* __restrict__ z, T* __restrict__ p, T* __restrict__ x, SegDev G) {
+    constexpr int V = Vec<T>::V;
     const int64_t t = blockIdx.y;
     const int64_t cnt = n * TILE;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * V; i < cnt;
+         i += (int64_t)gridDim.x * blockDim.x * V) {
         const int64_t o = t * cnt + i;
         const int64_t c = seg_of_row(G, i / TILE) * ld + t * TILE + (i % TILE);
-        const double a64 = alpha[c];
-        const T pv = p[o];
-        if (a64 != 0.0) x[o] += (T)a64 * pv;
-        p[o] = z[o] + (T)beta[c] * pv;
+        double a64[V];
+        bool any = false;
+#pragma unroll
+        for (int u = 0; u < V; u++) {
+            a64[u] = alpha[c + u];
+            any |= a64[u] != 0.0;
+        }
+        Vec<T> pv = vec_at(p + o), zv = vec_at(z + o);
+        if (any) {
+            Vec<T> xv = vec_at(x + o);
+#pragma unroll
+            for (int u = 0; u < V; u++)
+                if (a64[u] != 0.0) xv.v[u] += (T)a64[u] * pv.v[u];
+            vec_to(x + o, xv);
+        }
+#pragma unroll
+        for (int u = 0; u < V; u++) pv.v[u] = zv.v[u] + (T)beta[c + u] * pv.v[u];
+        vec_to(p + o, pv);
     }
 }
 
@@ -397,34 +471,38 @@ __global__ void k_add_into(int64_t count, const T* __restrict__ e, double* __res
 }
 
 // r = (Y - mean) - q with partial ||r||^2 per column: the true FP64 residual after a refinement round
-__global__ void __launch_bounds__(RED_THREADS) k_true_resid(int64_t n, int32_t k, const double* __restrict__ Y,
+__global__ void __launch_bounds__(RED_THREADS, RED_BLOCKS) k_true_resid(int64_t n, int32_t k, const double* __restrict__ Y,
                                                             const double* __restrict__ mean,
                                                             const double* __restrict__ q, double* __restrict__ r,
                                                             int64_t rows_per_blk, int64_t ld, double* __restrict__ part,
                                                             SegDev G) {
-    __shared__ double s[RED_THREADS];
+    constexpr int V = Vec<double>::V;
     const int64_t t = blockIdx.y;
-    const int c = threadIdx.x % TILE, rl = threadIdx.x / TILE;
+    const int c = threadIdx.x * V % TILE, rl = threadIdx.x * V / TILE;
     int64_t r0, r1, sb;
     red_block(G, n, rows_per_blk, ld, r0, r1, sb);
     const int64_t col = t * TILE + c;
     if (G.kseg) k = G.kseg[sb / ld];
-    const double mu = mean[sb + col];
-    const int64_t base = t * n * TILE;
-    double acc = 0.0;
-    for (int64_t row = r0 + rl; row < r1; row += RED_THREADS / TILE) {
-        const int64_t o = base + row * TILE + c;
-        const double rv = col < k ? (Y[o] - mu) - q[o] : 0.0;
-        r[o] = rv;
-        acc += rv * rv;
+    double mu[V], acc[V];
+#pragma unroll
+    for (int u = 0; u < V; u++) {
+        mu[u] = mean[sb + col + u];
+        acc[u] = 0.0;
     }
-    s[threadIdx.x] = acc;
-    __syncthreads();
-    if (threadIdx.x < TILE) {
-        double tt = s[threadIdx.x];
-        for (int i = 1; i < RED_THREADS / TILE; i++) tt += s[i * TILE + threadIdx.x];
-        part[(int64_t)blockIdx.x * ld + t * TILE + threadIdx.x] = tt;
+    const int64_t base = t * n * TILE + c;
+#pragma unroll 2
+    for (int64_t row = r0 + rl; row < r1; row += RROWS<double>) {
+        const int64_t o = base + row * TILE;
+        const Vec<double> yv = vec_at(Y + o), qv = vec_at(q + o);
+        Vec<double> rv;
+#pragma unroll
+        for (int u = 0; u < V; u++) {
+            rv.v[u] = col + u < k ? (yv.v[u] - mu[u]) - qv.v[u] : 0.0;
+            acc[u] += rv.v[u] * rv.v[u];
+        }
+        vec_to(r + o, rv);
     }
+    block_part<double>(acc, t, ld, part);
 }
 
 // ---------------------------------------------------------------- per-column scalars
@@ -1989,6 +2067,9 @@ static int32_t pcg_solve(Context& C, int64_t n, int32_t k, int64_t ld, const Spm
     const dim3 egrid((unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div<int64_t>(n * TILE, 256),
                                                                       2048 / std::max<int64_t>(1, ntiles) + 4)),
                      (unsigned)ntiles);
+    const dim3 vgrid((unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div<int64_t>(n * TILE, 256 * Vec<T>::V),
+                                                                      2048 / std::max<int64_t>(1, ntiles) + 4)),
+                     (unsigned)ntiles);
     const SegDev& G = R.G;
     const int64_t ns = (int64_t)G.nseg * ld;  // per-(graph, column) state entries
     const int cg = grid_for(ns, 256);
@@ -2094,7 +2175,7 @@ static int32_t pcg_solve(Context& C, int64_t n, int32_t k, int64_t ld, const Spm
         apply_precond();
         R.run<OP_DOT, T>(B.r, B.z, S.rz_new);
         k_cols_beta<<<cg, 256, 0, C.stream>>>(ns, S);
-        k_update_xp<T><<<egrid, 256, 0, C.stream>>>(n, ld, S.alpha, S.beta, B.z, B.p, B.e, G);
+        k_update_xp<T><<<vgrid, 256, 0, C.stream>>>(n, ld, S.alpha, S.beta, B.z, B.p, B.e, G);
         SSP_CHECK_LAUNCH();
         C.kernels_launched += 2;
     }
@@ -2139,7 +2220,7 @@ static int32_t pcg_solve(Context& C, int64_t n, int32_t k, int64_t ld, const Spm
             body_kernels += pc(P.has_shapes ? &P.shapes : nullptr, nullptr);
             R.run<OP_DOT, T>(B.r, B.z, S.rz_new);
             k_cols_beta<<<cg, 256, 0, C.stream>>>(ns, S);
-            k_update_xp<T><<<egrid, 256, 0, C.stream>>>(n, ld, S.alpha, S.beta, B.z, B.p, B.e, G);
+            k_update_xp<T><<<vgrid, 256, 0, C.stream>>>(n, ld, S.alpha, S.beta, B.z, B.p, B.e, G);
             launch_spmm<T>(C, n, A, aval, B.p, B.q, ld, G.nseg == 1, k, ra);
             pq_dot();
             k_cols_alpha<<<cg, 256, 0, C.stream>>>(ns, S);
