@@ -675,6 +675,21 @@ __device__ __forceinline__ void chunk_epilogue(T* out, const T* aux, int64_t tof
     }
 }
 
+// two columns
+template <int MODE, class T>
+__device__ __forceinline__ void chunk_epilogue(float* out, const float* aux, int64_t toff, int64_t v, int col, float2 acc,
+                                               const float* dlast) {
+    const int64_t o = toff + v * TILE + col;
+    float2 y = *reinterpret_cast<const float2*>((MODE == M_BWD ? out : aux) + o);
+    if (MODE != M_BWD) y = {y.x - acc.x, y.y - acc.y};
+    if (MODE != M_FWD) {
+        const float d = MODE == M_BWD ? aux[v] : dlast[v];
+        if (d != 0.0f) y = {y.x / d, y.y / d};
+        if (MODE == M_BWD) y = {y.x - acc.x, y.y - acc.y};
+    }
+    *reinterpret_cast<float2*>(out + o) = y;
+}
+
 // Row sums of the triangular solves.  A row's entries are summed in segments of ROW_SEG: entry i of a segment goes to
 // accumulator i mod 4 (in entry order), the four are combined as (a0 + a1) + (a2 + a3), and the segments' sums are
 // added in order.  Every launch width forms a row this way -- one lane per (row, column), or the entry slots of a warp
@@ -703,6 +718,41 @@ __device__ __forceinline__ T row_sum_lane(const int32_t* si, const T* sv, I q0, 
                 if (q + u < e) a[u] += sv[q + u] * x[u];
         }
         tot += (a[0] + a[1]) + (a[2] + a[3]);
+    }
+    return tot;
+}
+
+// The same for two FP32 columns of a lane, half the load instructions for a row.  ER n = 229,373, 1185 columns on B200: the
+// truncated level 1.28 -> 0.92 ms, the backward levels 0.79 -> 0.56 an application.
+__device__ __forceinline__ float2 row_sum_lane2(const int32_t* si, const float* sv, int q0, int q1, const float* xt) {
+    float2 tot = {0, 0};
+    auto at = [&](int q) { return *reinterpret_cast<const float2*>(xt + (int64_t)si[q] * TILE); };
+    for (int s = q0; s < q1; s += ROW_SEG) {
+        const int e = min(s + ROW_SEG, q1);
+        float2 a[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+        auto add = [&](int u, float v, const float2& x) {
+            a[u].x += v * x.x;
+            a[u].y += v * x.y;
+        };
+        int q = s;
+        for (; q + 3 < e; q += 4) {
+            float2 x[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) x[u] = at(q + u);
+#pragma unroll
+            for (int u = 0; u < 4; u++) add(u, sv[q + u], x[u]);
+        }
+        if (q < e) {
+            float2 x[3];
+#pragma unroll
+            for (int u = 0; u < 3; u++)
+                if (q + u < e) x[u] = at(q + u);
+#pragma unroll
+            for (int u = 0; u < 3; u++)
+                if (q + u < e) add(u, sv[q + u], x[u]);
+        }
+        tot.x += (a[0].x + a[1].x) + (a[2].x + a[3].x);
+        tot.y += (a[0].y + a[1].y) + (a[2].y + a[3].y);
     }
     return tot;
 }
@@ -776,6 +826,19 @@ __global__ void __launch_bounds__(CH_THREADS, MINB)
                 if (i < r1 - r0) sr[i] = rowmap[r0 + i];
             }
             __syncwarp();
+            if constexpr (W == TILE && sizeof(T) == 4) {
+                // a lane has two columns of a row, a half-warp the row: loads of 8 bytes, as in FP64
+                for (int32_t pr = lane; pr < (r1 - r0) * (W / 2); pr += 32) {
+                    const int32_t rr = pr / (W / 2), col = pr % (W / 2) * 2;
+                    const int64_t vrow = sr[rr];
+                    if (!row_on(ra, vrow, t)) continue;
+                    const int32_t q0 = sp[rr], q1 = t * TILE + col < kcols ? sp[rr + 1] : q0;
+                    const float2 sum = row_sum_lane2(si, sv, q0, q1, xt + col);
+                    chunk_epilogue<MODE, T>(out, aux, toff, vrow, col, sum, dlast);
+                }
+                __syncwarp();
+                continue;
+            }
             const int32_t pairs = (r1 - r0) * W;
             for (int32_t pr = lane; pr < pairs; pr += 32) {
                 const int32_t rr = pr / W, col = c0 + pr % W;
@@ -818,8 +881,9 @@ __global__ void __launch_bounds__(CH_THREADS, MINB)
 // Bound by random 256-byte row gathers through L2 (51 GB in 5.0 ms at ER n = 250,000).  Measured on B200, one FP64 product,
 // with the long rows walked whole and serial last entries -> here: R-MAT n = 24,281, 883K entries, 2693 columns 4.21 ->
 // 1.60 ms; 3-D grid n = 80,840, 1085 columns 1.05 -> 0.58; ER n = 250,000, degree 20, 1194 columns 6.4 -> 5.0; ER n = 1M, 80
-// columns 2.70 -> 2.10.  FP32 stays at 3.1 ms at ER n = 229,373, 1185 columns.  Slower: 16-column halves of a tile, whose
-// gathered rows then fit L2 (2.89 against 2.75 ms at ER n = 1M); sixteen gathers in flight in FP32 (3.14 against 3.07).
+// columns 2.70 -> 2.10.  FP32 (spmm_row_pair) 3.08 -> 2.37 ms at ER n = 229,373, 1185 columns.  Slower: 16-column halves of a
+// tile, whose gathered rows then fit L2 (2.89 against 2.75 ms at ER n = 1M); FP64 in 16-byte pieces the same way (6.2 ms
+// against 5.06 at ER n = 250,000); FP32 with 3, 5 or 6 pairs in flight (2.67, 2.90, 2.98) and a half-warp per row (3.83).
 // Six resident blocks per SM (five ran slower: FP32 29.7 against 22.6 ms at ER n = 1M, 1327 columns).
 struct SpmmItems {
     const int32_t* chunks = nullptr;  // nchunks + 1 row starts (a row of more than CHUNK_CAP entries is skipped there)
@@ -852,6 +916,42 @@ __device__ __forceinline__ T spmm_row(const int32_t* si, const T* sv, int32_t q,
     return (a[0] + a[1]) + (a[2] + a[3]);
 }
 
+// The same sums of an FP32 row by a whole warp: a lane has two columns, and the half-warps take every second entry, so that
+// a load instruction moves 256 bytes as in FP64.  Both halves return the row's sums.  (q0, q1: the row's entries;
+// xt: at the lane's first column)
+__device__ __forceinline__ float2 spmm_row_pair(const int32_t* si, const float* sv, int32_t q0, int32_t q1,
+                                                const float* xt, int half) {
+    constexpr int U = 4;
+    float2 a = {0, 0};
+    int32_t q = q0 + half;
+    for (; q + 2 * (U - 1) < q1; q += 2 * U) {
+        float2 x[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) x[u] = *reinterpret_cast<const float2*>(xt + (int64_t)si[q + 2 * u] * TILE);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            a.x += sv[q + 2 * u] * x[u].x;
+            a.y += sv[q + 2 * u] * x[u].y;
+        }
+    }
+    if (q < q1) {
+        float2 x[U - 1];
+#pragma unroll
+        for (int u = 0; u < U - 1; u++)
+            if (q + 2 * u < q1) x[u] = *reinterpret_cast<const float2*>(xt + (int64_t)si[q + 2 * u] * TILE);
+#pragma unroll
+        for (int u = 0; u < U - 1; u++)
+            if (q + 2 * u < q1) {
+                a.x += sv[q + 2 * u] * x[u].x;
+                a.y += sv[q + 2 * u] * x[u].y;
+            }
+    }
+    __syncwarp();
+    a.x += __shfl_xor_sync(0xffffffffu, a.x, 16);
+    a.y += __shfl_xor_sync(0xffffffffu, a.y, 16);
+    return a;
+}
+
 // W: columns per warp row (TILE, or 8 when at most 8 are real); ACC adds into q (the second and later column slabs)
 template <class T, int W, bool ACC>
 __global__ void __launch_bounds__(CH_THREADS, 6)
@@ -869,7 +969,8 @@ __global__ void __launch_bounds__(CH_THREADS, 6)
     int32_t* si = s_idx[w];
     T* sv = s_val[w];
     int32_t* sp = s_ptr[w];
-    double dot = 0.0;  // per-lane partial of p.q for column (lane % W)
+    constexpr bool PAIR = W == TILE && sizeof(T) == 4;
+    double dot = 0.0, dot1 = 0.0;  // per-lane partials of p.q for column (lane % W), or for the lane's two columns
     for (int32_t c = blockIdx.x * CH_WARPS + w; c < S.nseg + S.nchunks; c += gridDim.x * CH_WARPS) {
         const bool seg = c < S.nseg;  // segments, the larger items, first
         const int32_t r0 = seg ? S.segrow[c] : S.chunks[c - S.nseg], r1 = seg ? r0 + 1 : S.chunks[c - S.nseg + 1];
@@ -883,6 +984,33 @@ __global__ void __launch_bounds__(CH_THREADS, 6)
         }
         for (int32_t i = lane; i <= r1 - r0; i += 32) sp[i] = seg ? i * ne : (int32_t)(ptr[r0 + i] - e0);
         __syncwarp();
+        if constexpr (PAIR) {
+            const int half = lane >> 4, col = (lane & 15) * 2;
+            for (int32_t rr = 0; rr < r1 - r0; rr++) {
+                const int64_t row = r0 + rr;
+                if (!row_on(ra, row, t)) continue;  // warp-uniform
+                float2 acc = spmm_row_pair(si, sv, sp[rr], t * TILE + col < kcols ? sp[rr + 1] : 0, xt + col, half);
+                if (half) continue;
+                if (seg) {
+                    *reinterpret_cast<float2*>(lpart + (int64_t)c * ld + t * TILE + col) = acc;
+                    continue;
+                }
+                const int64_t o = toff + row * TILE + col;
+                if (ACC) {
+                    const float2 old = __ldcs(reinterpret_cast<const float2*>(q + o));
+                    acc.x += old.x;
+                    acc.y += old.y;
+                }
+                __stcs(reinterpret_cast<float2*>(q + o), acc);
+                if (part) {
+                    const float2 pv = *reinterpret_cast<const float2*>(xt + row * TILE + col);
+                    dot += (double)acc.x * (double)pv.x;
+                    dot1 += (double)acc.y * (double)pv.y;
+                }
+            }
+            __syncwarp();
+            continue;
+        }
         const int32_t pairs = (r1 - r0) * W;
         for (int32_t pr = lane; pr < pairs; pr += 32) {
             const int32_t rr = pr / W, col = pr % W;
@@ -904,7 +1032,12 @@ __global__ void __launch_bounds__(CH_THREADS, 6)
         __syncwarp();
     }
     if (part) {
-        s_red[threadIdx.x] = dot;
+        if (!PAIR) {
+            s_red[threadIdx.x] = dot;
+        } else if (lane < 16) {
+            s_red[w * TILE + 2 * lane] = dot;
+            s_red[w * TILE + 2 * lane + 1] = dot1;
+        }
         __syncthreads();
         if (threadIdx.x < TILE) {
             double tt = 0.0;
@@ -1271,8 +1404,8 @@ static void launch_level_w(int code, dim3 grid, cudaStream_t s, int64_t n, const
                                                                 nsub, dlast, ra);
         break;
     default:
-        k_chunked<MODE, T, TILE, MINB><<<grid, CH_THREADS, 0, s>>>(n, ch, nc, ptr, idx, val, rowmap, y, y, aux, kcols,
-                                                                nsub, dlast, ra);
+        k_chunked<MODE, T, TILE, MINB><<<grid, CH_THREADS, 0, s>>>(
+            n, ch, nc, ptr, idx, val, rowmap, y, y, aux, kcols, nsub, dlast, ra);
         break;
     }
 }
