@@ -1473,12 +1473,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
         SSP_CHECK_LAUNCH();
         const int64_t R = read_i64(C, F.ctr + C_REM);
         if (R == 0) return 0;
-        std::vector<int32_t> lens(v1 - v0);
-        SSP_CUDA(cudaMemcpyAsync(lens.data(), F.bag_len + v0, sizeof(int32_t) * (v1 - v0), cudaMemcpyDeviceToHost,
-                                 C.stream));
-        SSP_CUDA(cudaStreamSynchronize(C.stream));
-        int32_t maxlen = 0;
-        for (auto x : lens) maxlen = std::max(maxlen, x);
+        const int32_t maxlen = device_max_i32(C, F.bag_len + v0, v1 - v0);
         int32_t cap = 64;
         while (cap < maxlen) cap <<= 1;
         trunc_diag(rem, R, at, cap);
@@ -1689,13 +1684,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
         int32_t* rem = W.get_t<int32_t>(nm("rem"), R + 1);
         SSP_CUDA(cudaMemsetAsync(F.ctr + C_REM, 0, sizeof(int64_t), C.stream));
         k_collect_live<<<grid_for(n, T256), T256, 0, C.stream>>>(n, F.level, rem, F.ctr + C_REM);
-        int32_t maxlen = 0;
-        {
-            std::vector<int32_t> lens(n);
-            SSP_CUDA(cudaMemcpyAsync(lens.data(), F.bag_len, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, C.stream));
-            SSP_CUDA(cudaStreamSynchronize(C.stream));
-            for (auto x : lens) maxlen = std::max(maxlen, x);
-        }
+        const int32_t maxlen = device_max_i32(C, F.bag_len, n);
         int32_t cap = 64;
         while (cap < maxlen) cap <<= 1;
         trunc_diag(rem, R, lvl, cap);
@@ -1726,13 +1715,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
         double* Wd = W.get_t<double>(nm("W"), (size_t)T * T);
         SSP_CUDA(cudaMemsetAsync(Wd, 0, sizeof(double) * T * T, C.stream));
         // bag sizes bound the build scratch
-        int32_t maxlen = 0;
-        {
-            std::vector<int32_t> lens(n);
-            SSP_CUDA(cudaMemcpyAsync(lens.data(), F.bag_len, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, C.stream));
-            SSP_CUDA(cudaStreamSynchronize(C.stream));
-            for (auto x : lens) maxlen = std::max(maxlen, x);
-        }
+        const int32_t maxlen = device_max_i32(C, F.bag_len, n);
         int32_t cap = 64;
         while (cap < maxlen) cap <<= 1;
         if (cap <= BLOCK_TIER_MAX) {
@@ -1798,11 +1781,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
     // sort each row by column id (deterministic summation order in the forward solve)
     {
         int64_t* seg_start = out.row_ptr;
-        int32_t maxrow = 0;
-        std::vector<int32_t> rc(n);
-        SSP_CUDA(cudaMemcpyAsync(rc.data(), rowcnt, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, C.stream));
-        SSP_CUDA(cudaStreamSynchronize(C.stream));
-        for (auto x : rc) maxrow = std::max(maxrow, x);
+        const int32_t maxrow = device_max_i32(C, rowcnt, n);
         segsort_pairs_i32_f64(C, out.row_idx, out.row_val, seg_start, rowcnt, n, maxrow);
     }
     out.D = F.D;
@@ -1861,24 +1840,26 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
                                                                                 *pptr, *pidx, *pval, *prow, *pent);
             SSP_CHECK_LAUNCH();
             C.kernels_launched += 2;
-            hp.resize(n + 1);
-            SSP_CUDA(cudaMemcpyAsync(hp.data(), *pptr, sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToHost, C.stream));
+            // a truncation's rows, the last level, are most of a large graph: they are cut into chunks on the device, and the
+            // host, whose plans look at the levels before, does not get their pointers.  A last level of one row
+            // (a complete elimination's) is not worth the launches and the wait, some 50 us.
+            const int64_t last = NL > 0 ? lp[NL - 1] : 0;
+            const bool on_dev = n - last > 4096;
+            hp.resize((on_dev ? last : n) + 1);
+            SSP_CUDA(cudaMemcpyAsync(hp.data(), *pptr, sizeof(int64_t) * hp.size(), cudaMemcpyDeviceToHost, C.stream));
             SSP_CUDA(cudaStreamSynchronize(C.stream));
-            const int64_t last_nnz = NL > 0 ? hp[lp[NL]] - hp[lp[NL - 1]] : 0;
+            const int64_t last_nnz = out.nnz - hp[last];
             if (pptr == &out.prow_ptr) out.last_fwd_nnz = last_nnz;
             else out.last_bwd_nnz = last_nnz;
             std::vector<int32_t> starts;
             chunk_lvl.assign(NL + 1, 0);
             for (int32_t l = 0; l < NL; l++) {
                 chunk_lvl[l] = (int32_t)starts.size();
-                make_chunks(hp, (int32_t)lp[l], (int32_t)lp[l + 1], starts);
+                if (l + 1 < NL || !on_dev) make_chunks(hp, (int32_t)lp[l], (int32_t)lp[l + 1], starts);
             }
-            chunk_lvl[NL] = (int32_t)starts.size();
-            starts.push_back((int32_t)n);
-            *chunks = W.get_t<int32_t>(nm(tagp) + "_chunks", starts.size());
-            SSP_CUDA(cudaMemcpyAsync(*chunks, starts.data(), sizeof(int32_t) * starts.size(), cudaMemcpyHostToDevice,
-                                     C.stream));
-            SSP_CUDA(cudaStreamSynchronize(C.stream));
+            const DevChunks D = device_chunks(C, *pptr, on_dev ? (int32_t)last : (int32_t)n, (int32_t)n, nm(tagp), starts);
+            chunk_lvl[NL] = (int32_t)starts.size() + D.nchunks;
+            *chunks = D.starts;
         };
         build(out.level_rows, out.row_ptr, out.row_idx, out.row_val, "prow", &out.prow_ptr, &out.prow_idx, &out.prow_val,
               &out.fchunk, out.fchunk_lvl, out.hfptr, &out.frow, &out.fent);

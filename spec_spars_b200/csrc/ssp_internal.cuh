@@ -267,6 +267,22 @@ constexpr int CHUNK_CAP = SSP_CHUNK_CAP;
 constexpr int CHUNK_ROWS = 32;
 void make_chunks(const std::vector<int64_t>& ptr, int32_t r0, int32_t r1, std::vector<int32_t>& starts);
 void make_chunks(const int64_t* ptr, int32_t r0, int32_t r1, std::vector<int32_t>& starts);
+// The same for large ranges, on the device (windows of rows, so the cuts differ from make_chunks' at a window's end).  starts
+// holds before's entries, then the nchunks starts of [r0, r1), then r1.  Each row longer than a chunk is also cut into
+// segments of CHUNK_CAP entries.
+struct DevChunks {
+    int32_t* starts = nullptr;
+    int32_t nchunks = 0;
+    int32_t nlong = 0, nseg = 0;
+    int32_t* lrow = nullptr;    // [nlong] the long rows
+    int32_t* lseg = nullptr;    // [nlong + 1] first segment of each
+    int32_t* segrow = nullptr;  // [nseg] row of each segment
+    int64_t* seg = nullptr;     // [nseg] its first entry
+};
+DevChunks device_chunks(Context& C, const int64_t* ptr, int32_t r0, int32_t r1, const std::string& tag,
+                        const std::vector<int32_t>& before = {});
+// the largest of n values on the device (0 at least)
+int32_t device_max_i32(Context& C, const int32_t* v, int64_t n);
 // Copies between pageable host memory and the device on C.stream, returning once the host side is done
 // (host to device: the source may be reused; device to host: the data is in dst).  Large copies go through
 // a pinned staging ring with the host-side memcpy split over a few threads and overlapped with the DMA;
@@ -395,7 +411,7 @@ struct DevFactor {
     // forward solve of that level finish its rows (z = y / D) and the backward solve skip it.
     int64_t last_fwd_nnz = -1;
     int64_t last_bwd_nnz = -1;
-    std::vector<int64_t> hfptr, hbptr;  // prow_ptr and pcol_ptr on the host
+    std::vector<int64_t> hfptr, hbptr;  // prow_ptr and pcol_ptr on the host, up to the last level's first row
     // The dense tail (dense_levels > 0): the last tail_rows storage rows, one per level from level tail_l0 on.  linv is
     // the inverse of their unit lower triangular block of L (row-major, tail_rows x tail_rows); tin_* are the
     // entries of their rows in earlier levels, with their own row pointers and chunks (ssp_tail.cu).

@@ -1925,7 +1925,6 @@ static SpmmPlan make_spmm_plan(Context& C, int64_t n, const int64_t* lap_ptr, co
     A.nnz = read_i64(C, lap_ptr + n);
     A.nslabs = spmm_slab_count(C, n, lap_ptr, lap_idx, A.nnz);
     const int32_t m = A.nslabs;
-    std::vector<int64_t> hp((size_t)m * n + 1);
     if (m == 1) {
         A.ptr = lap_ptr;
         A.idx = lap_idx;
@@ -1947,62 +1946,21 @@ static SpmmPlan make_spmm_plan(Context& C, int64_t n, const int64_t* lap_ptr, co
         A.idx = sidx;
         A.val = sval;
     }
-    SSP_CUDA(cudaMemcpyAsync(hp.data(), A.ptr, sizeof(int64_t) * hp.size(), cudaMemcpyDeviceToHost, C.stream));
-    SSP_CUDA(cudaStreamSynchronize(C.stream));
     // per slab: the chunks, and the segments of the rows longer than one
-    std::vector<int32_t> i32;
-    std::vector<int64_t> i64;
-    struct Off {
-        size_t chunks, segrow, lrow, lseg, seg;
-    };
-    std::vector<Off> off(m);
     int32_t most = 0, most_seg = 0;
     for (int32_t b = 0; b < m; b++) {
-        const int64_t* bp = hp.data() + (size_t)b * n;
+        const DevChunks D = device_chunks(C, A.ptr + (int64_t)b * n, 0, (int32_t)n, "pcg_a" + std::to_string(b));
         SpmmItems& I = A.items[b];
-        std::vector<int32_t> ch, segrow, lrow, lseg;
-        make_chunks(bp, 0, (int32_t)n, ch);
-        I.nchunks = (int32_t)ch.size();
-        ch.push_back((int32_t)n);
-        off[b].seg = i64.size();
-        for (int32_t c = 0; c < I.nchunks; c++) {
-            const int64_t e0 = bp[ch[c]], e1 = bp[ch[c + 1]];
-            if (e1 - e0 <= CHUNK_CAP) continue;
-            lrow.push_back(ch[c]);
-            lseg.push_back((int32_t)segrow.size());
-            for (int64_t e = e0; e < e1; e += CHUNK_CAP) {
-                segrow.push_back(ch[c]);
-                i64.push_back(e);
-            }
-        }
-        lseg.push_back((int32_t)segrow.size());
-        I.nseg = (int32_t)segrow.size();
-        I.nlong = (int32_t)lrow.size();
-        auto add = [&](const std::vector<int32_t>& v) {
-            const size_t at = i32.size();
-            i32.insert(i32.end(), v.begin(), v.end());
-            return at;
-        };
-        off[b].chunks = add(ch);
-        off[b].segrow = add(segrow);
-        off[b].lrow = add(lrow);
-        off[b].lseg = add(lseg);
+        I.chunks = D.starts;
+        I.nchunks = D.nchunks;
+        I.nseg = D.nseg;
+        I.seg = D.seg;
+        I.segrow = D.segrow;
+        I.nlong = D.nlong;
+        I.lrow = D.lrow;
+        I.lseg = D.lseg;
         most = std::max(most, I.nchunks + I.nseg);
         most_seg = std::max(most_seg, I.nseg);
-    }
-    int32_t* d = W.get_t<int32_t>("pcg_achunks", i32.size());
-    int64_t* d64 = W.get_t<int64_t>("pcg_aseg", i64.size() + 1);
-    SSP_CUDA(cudaMemcpyAsync(d, i32.data(), sizeof(int32_t) * i32.size(), cudaMemcpyHostToDevice, C.stream));
-    if (!i64.empty())
-        SSP_CUDA(cudaMemcpyAsync(d64, i64.data(), sizeof(int64_t) * i64.size(), cudaMemcpyHostToDevice, C.stream));
-    SSP_CUDA(cudaStreamSynchronize(C.stream));
-    for (int32_t b = 0; b < m; b++) {
-        SpmmItems& I = A.items[b];
-        I.chunks = d + off[b].chunks;
-        I.segrow = d + off[b].segrow;
-        I.lrow = d + off[b].lrow;
-        I.lseg = d + off[b].lseg;
-        I.seg = d64 + off[b].seg;
     }
     const int bx = chunk_blocks(most);
     A.grid = dim3((unsigned)bx, (unsigned)(ld / TILE));
