@@ -582,6 +582,28 @@ __global__ void k_cols_check(int64_t cnt, int32_t it, ColState S) {
     }
 }
 
+// One iteration's entry of the residual history: per segment (block) the largest ||r|| / ||b|| of its columns, then the
+// columns still active.  Kept on the device so that a probe's iterations are launched without waiting: reading them back
+// after each took 60-80 us an iteration.
+__global__ void __launch_bounds__(32) k_hist(int64_t ld, ColState S, double* __restrict__ hist) {
+    const int64_t sg = blockIdx.x;
+    double m = 0.0;
+    for (int64_t j = threadIdx.x; j < ld; j += 32) {
+        const double b = S.bnorm2[sg * ld + j];
+        if (b > 0) {
+            const double q = sqrt(S.rr[sg * ld + j] / b);
+            if (m < q) m = q;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const double q = __shfl_xor_sync(0xffffffffu, m, o);
+        if (m < q) m = q;
+    }
+    if (threadIdx.x) return;
+    hist[sg] = m;
+    if (sg == 0) hist[gridDim.x] = (double)*S.nactive;
+}
+
 __global__ void k_cols_beta(int64_t cnt, ColState S) {
     for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < cnt; c += (int64_t)gridDim.x * blockDim.x) {
         double b = 0.0;
@@ -2216,6 +2238,8 @@ static int32_t pcg_solve(Context& C, int64_t n, int32_t k, int64_t ld, const Spm
     apply_precond();
     R.run<OP_DOT, T>(B.r, B.z, S.rz);
     SSP_CUDA(cudaMemcpyAsync(B.p, B.z, sizeof(T) * total, cudaMemcpyDeviceToDevice, C.stream));
+    const bool history = opt.history || seg_history;
+    double* d_hist = history ? C.ws.get_t<double>("pcg_hist", (size_t)max_iters * (G.nseg + 1)) : nullptr;
     tm.loop.begin(C.stream);
     while (it < max_iters) {
         tm.spmm.begin(C.stream);
@@ -2234,29 +2258,16 @@ static int32_t pcg_solve(Context& C, int64_t n, int32_t k, int64_t ld, const Spm
         SSP_CHECK_LAUNCH();
         C.kernels_launched++;
         update_act();
-        active = read_i64(C, S.nactive);
-        finish_measure();
-        if (opt.history || seg_history) {
-            std::vector<double> hrr(ns), hbb(ns);
-            SSP_CUDA(cudaMemcpyAsync(hrr.data(), S.rr, sizeof(double) * ns, cudaMemcpyDeviceToHost, C.stream));
-            SSP_CUDA(cudaMemcpyAsync(hbb.data(), S.bnorm2, sizeof(double) * ns, cudaMemcpyDeviceToHost, C.stream));
-            SSP_CUDA(cudaStreamSynchronize(C.stream));
-            double mx = 0.0;
-            for (int64_t j = 0; j < ns; j++)
-                if (hbb[j] > 0) mx = std::max(mx, std::sqrt(hrr[j] / hbb[j]));
-            if (opt.history) opt.history->push_back(mx);
-            if (seg_history) {
-                auto& H = opt.segs->history;
-                H.resize(G.nseg);
-                for (int32_t sg = 0; sg < G.nseg; sg++) {
-                    double m2 = 0.0;
-                    for (int64_t j = 0; j < ld; j++) {
-                        const int64_t o = (int64_t)sg * ld + j;
-                        if (hbb[o] > 0) m2 = std::max(m2, std::sqrt(hrr[o] / hbb[o]));
-                    }
-                    H[sg].push_back(m2);
-                }
-            }
+        if (history) {
+            k_hist<<<(unsigned)G.nseg, 32, 0, C.stream>>>(ld, S, d_hist + (int64_t)(it - 1) * (G.nseg + 1));
+            SSP_CHECK_LAUNCH();
+            C.kernels_launched++;
+        }
+        // A history's solve waits only at the end (or while it measures, or reports): iterations after the last column has
+        // stopped change nothing (alpha is 0) and are dropped from the history below.
+        if (!history || P.measure || opt.verbose) {
+            active = read_i64(C, S.nactive);
+            finish_measure();
         }
         if (opt.verbose && (it % 10 == 0 || active == 0))
             fprintf(stderr, "[ssp] pcg%s iter %d: %lld columns active\n", sizeof(T) == 4 ? " (fp32 inner)" : "", it,
@@ -2269,6 +2280,21 @@ static int32_t pcg_solve(Context& C, int64_t n, int32_t k, int64_t ld, const Spm
         k_update_xp<T><<<vgrid, 256, 0, C.stream>>>(n, ld, S.alpha, S.beta, B.z, B.p, B.e, G);
         SSP_CHECK_LAUNCH();
         C.kernels_launched += 2;
+    }
+    if (history && it > 0) {
+        std::vector<double> hh((size_t)it * (G.nseg + 1));
+        SSP_CUDA(cudaMemcpyAsync(hh.data(), d_hist, sizeof(double) * hh.size(), cudaMemcpyDeviceToHost, C.stream));
+        SSP_CUDA(cudaStreamSynchronize(C.stream));
+        if (seg_history) opt.segs->history.resize(G.nseg);
+        const int32_t ran = it;
+        for (it = 0; it < ran;) {
+            const double* e = hh.data() + (size_t)it * (G.nseg + 1);
+            if (opt.history) opt.history->push_back(*std::max_element(e, e + G.nseg));
+            for (int32_t sg = 0; seg_history && sg < G.nseg; sg++) opt.segs->history[sg].push_back(e[sg]);
+            it++;
+            active = (int64_t)e[G.nseg];
+            if (active == 0) break;
+        }
     }
     if (device_loop && active > 0 && it < max_iters) {
         // one iteration = preconditioner, r.z, beta, p update, SpMM, alpha, x/r update, check, control
