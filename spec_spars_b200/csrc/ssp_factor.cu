@@ -682,7 +682,8 @@ struct ElimArgs {
 };
 
 // Barrier over the grid; the last block to arrive runs ctl (all its threads) before the others go on.  The wait is
-// bounded: after a few seconds the kernel reports ST_ERR and ends.  Returns false then.
+// bounded (some ten seconds: blocks may have to wait for other streams' kernels before they all run); past that the
+// kernel reports ST_ERR and ends.  Returns false then.
 template <class Ctl>
 __device__ bool grid_barrier(const ElimArgs& A, Ctl ctl) {
     __shared__ unsigned s_ticket;
@@ -708,7 +709,7 @@ __device__ bool grid_barrier(const ElimArgs& A, Ctl ctl) {
         int spins = 0;
         while ((int)(*(volatile unsigned*)&A.bar[1] - (round + 1)) < 0) {
             if (++spins > 1024) __nanosleep(100);
-            if (spins > (1 << 23)) {
+            if (spins > (1 << 26)) {
                 atomicExch((unsigned long long*)&A.st[ST_ERR], 1ull);
                 s_ok = 0;
                 break;
