@@ -677,7 +677,7 @@ struct LoopGraph {
 enum { M_FWD = 1, M_BWD = 2, M_FWD_LAST = 4 };
 constexpr int CH_THREADS = 256;
 constexpr int CH_WARPS = CH_THREADS / 32;
-constexpr int MINB_FWD = 6, MINB_BWD = 5;
+constexpr int MINB_FWD = 6, MINB_BWD = 5, MINB_WIDE64 = 4;
 
 template <int MODE, class T>
 __device__ __forceinline__ void chunk_epilogue(T* out, const T* aux, int64_t toff, int64_t v, int col, T acc,
@@ -698,18 +698,30 @@ __device__ __forceinline__ void chunk_epilogue(T* out, const T* aux, int64_t tof
 }
 
 // two columns
-template <int MODE, class T>
-__device__ __forceinline__ void chunk_epilogue(float* out, const float* aux, int64_t toff, int64_t v, int col, float2 acc,
-                                               const float* dlast) {
+template <class T>
+struct ColPair;
+template <>
+struct ColPair<double> {
+    using V = double2;
+};
+template <>
+struct ColPair<float> {
+    using V = float2;
+};
+
+// the epilogue of two columns
+template <int MODE, class T, class V>
+__device__ __forceinline__ void chunk_epilogue2(T* out, const T* aux, int64_t toff, int64_t v, int col, V acc,
+                                                const T* dlast) {
     const int64_t o = toff + v * TILE + col;
-    float2 y = *reinterpret_cast<const float2*>((MODE == M_BWD ? out : aux) + o);
+    V y = *reinterpret_cast<const V*>((MODE == M_BWD ? out : aux) + o);
     if (MODE != M_BWD) y = {y.x - acc.x, y.y - acc.y};
     if (MODE != M_FWD) {
-        const float d = MODE == M_BWD ? aux[v] : dlast[v];
-        if (d != 0.0f) y = {y.x / d, y.y / d};
+        const T d = MODE == M_BWD ? aux[v] : dlast[v];
+        if (d != (T)0) y = {y.x / d, y.y / d};
         if (MODE == M_BWD) y = {y.x - acc.x, y.y - acc.y};
     }
-    *reinterpret_cast<float2*>(out + o) = y;
+    *reinterpret_cast<V*>(out + o) = y;
 }
 
 // Row sums of the triangular solves.  A row's entries are summed in segments of ROW_SEG: entry i of a segment goes to
@@ -744,28 +756,32 @@ __device__ __forceinline__ T row_sum_lane(const int32_t* si, const T* sv, I q0, 
     return tot;
 }
 
-// The same for two FP32 columns of a lane, half the load instructions for a row.  ER n = 229,373, 1185 columns on B200: the
-// truncated level 1.28 -> 0.92 ms, the backward levels 0.79 -> 0.56 an application.
-__device__ __forceinline__ float2 row_sum_lane2(const int32_t* si, const float* sv, int q0, int q1, const float* xt) {
-    float2 tot = {0, 0};
-    auto at = [&](int q) { return *reinterpret_cast<const float2*>(xt + (int64_t)si[q] * TILE); };
+// The same for two columns of a lane, half the load instructions for a row.  On B200 an FP32 application at ER n =
+// 229,373, 1185 columns: the truncated level 1.28 -> 0.92 ms, the backward levels 0.79 -> 0.56.  FP64 (four blocks per SM: at
+// five and six the 16-byte gathers spill), ER n = 250,000, 1194 columns: 3.10 -> 2.95 ms in all.
+template <class T>
+__device__ __forceinline__ typename ColPair<T>::V row_sum_lane2(const int32_t* si, const T* sv, int q0, int q1,
+                                                                  const T* xt) {
+    using V = typename ColPair<T>::V;
+    V tot = {0, 0};
+    auto at = [&](int q) { return *reinterpret_cast<const V*>(xt + (int64_t)si[q] * TILE); };
     for (int s = q0; s < q1; s += ROW_SEG) {
         const int e = min(s + ROW_SEG, q1);
-        float2 a[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
-        auto add = [&](int u, float v, const float2& x) {
+        V a[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+        auto add = [&](int u, T v, const V& x) {
             a[u].x += v * x.x;
             a[u].y += v * x.y;
         };
         int q = s;
         for (; q + 3 < e; q += 4) {
-            float2 x[4];
+            V x[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) x[u] = at(q + u);
 #pragma unroll
             for (int u = 0; u < 4; u++) add(u, sv[q + u], x[u]);
         }
         if (q < e) {
-            float2 x[3];
+            V x[3];
 #pragma unroll
             for (int u = 0; u < 3; u++)
                 if (q + u < e) x[u] = at(q + u);
@@ -813,7 +829,7 @@ __device__ __forceinline__ T seg_sum_slots(const int32_t* si, const T* sv, int s
 // Grid: x over chunks, y over (tile, sub-tile): a tile's TILE columns are covered by nsub = TILE / W warps'
 // column ranges (nsub = 1 for the full-width layout, or for the narrow one when only W columns are real).
 // MINB: resident blocks per SM asked of the compiler, what each direction's own register choice gives (forward 6,
-// backward 5; forcing six on the backward solve cost the preconditioner 7 %).
+// backward 5; forcing six on the backward solve cost the preconditioner 7 %), or 4 at full width in FP64 (row_sum_lane2).
 template <int MODE, class T, int W, int MINB>
 __global__ void __launch_bounds__(CH_THREADS, MINB)
     k_chunked(int64_t n, const int32_t* __restrict__ cstart, int32_t nchunks, const int64_t* __restrict__ ptr,
@@ -848,15 +864,15 @@ __global__ void __launch_bounds__(CH_THREADS, MINB)
                 if (i < r1 - r0) sr[i] = rowmap[r0 + i];
             }
             __syncwarp();
-            if constexpr (W == TILE && sizeof(T) == 4) {
-                // a lane has two columns of a row, a half-warp the row: loads of 8 bytes, as in FP64
+            if constexpr (W == TILE) {
+                // a lane has two columns of a row, a half-warp the row
                 for (int32_t pr = lane; pr < (r1 - r0) * (W / 2); pr += 32) {
                     const int32_t rr = pr / (W / 2), col = pr % (W / 2) * 2;
                     const int64_t vrow = sr[rr];
                     if (!row_on(ra, vrow, t)) continue;
                     const int32_t q0 = sp[rr], q1 = t * TILE + col < kcols ? sp[rr + 1] : q0;
-                    const float2 sum = row_sum_lane2(si, sv, q0, q1, xt + col);
-                    chunk_epilogue<MODE, T>(out, aux, toff, vrow, col, sum, dlast);
+                    const auto sum = row_sum_lane2<T>(si, sv, q0, q1, xt + col);
+                    chunk_epilogue2<MODE, T>(out, aux, toff, vrow, col, sum, dlast);
                 }
                 __syncwarp();
                 continue;
@@ -1211,17 +1227,6 @@ static int chunk_blocks(int32_t nchunks) {
 // 200, 951 columns 2.0 -> 0.68 ms; geometric graph n = 30,011, 60 columns 9.7 -> 1.8 ms.
 // Slower: a row per lane without ordering rows by length (1.3x to 1.6x); rows and entries staged through shared memory
 // by cp.async, by warp or by block (1.3x to 2.2x: more instructions per round than the latency they hide).
-template <class T>
-struct WalkPair;
-template <>
-struct WalkPair<double> {
-    using V = double2;
-};
-template <>
-struct WalkPair<float> {
-    using V = float2;
-};
-
 // Rows row .. row + nr of the storage order, 2^lg slots per row; last: the level's last round
 struct WalkRound {
     int32_t row;
@@ -1235,7 +1240,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
     k_trsv_walk(int64_t n, const WalkRound* __restrict__ rounds, int32_t nrounds, const FactorRow* __restrict__ rows,
                 const FactorEnt<T>* __restrict__ ent, const T* __restrict__ aux, T* y, int32_t kcols, int nsub, int cl,
                 RowAct ra) {
-    using V = typename WalkPair<T>::V;
+    using V = typename ColPair<T>::V;
     constexpr int LPS = W / 2, B = 4;
     extern __shared__ WalkRound s_rounds[];
     for (int i = threadIdx.x; i < nrounds; i += NT) s_rounds[i] = rounds[i];
@@ -1426,7 +1431,7 @@ static void launch_level_w(int code, dim3 grid, cudaStream_t s, int64_t n, const
                                                                 nsub, dlast, ra);
         break;
     default:
-        k_chunked<MODE, T, TILE, MINB><<<grid, CH_THREADS, 0, s>>>(
+        k_chunked<MODE, T, TILE, (sizeof(T) == 8 ? MINB_WIDE64 : MINB)><<<grid, CH_THREADS, 0, s>>>(
             n, ch, nc, ptr, idx, val, rowmap, y, y, aux, kcols, nsub, dlast, ra);
         break;
     }
