@@ -1809,11 +1809,12 @@ static void tune_trsv_shapes(Context& C, const DevFactor& F, const TrsvPlan& P, 
 }
 
 // The preconditioner application as a CUDA graph, with its level shapes.  measure: the shapes are still to be
-// measured by the solve's next applications (pcg_solve), which then rebuild the graph.
+// measured by the solve's next applications (pcg_solve), after which the graph is captured anew.
 struct Precond {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     TrsvShapes shapes;
+    bool planned = false;
     bool has_shapes = false;
     bool measure = false;
     uint64_t key = 0;
@@ -2043,10 +2044,9 @@ static void capture_precond(Context& C, Precond& P, int64_t& launches, const PcA
 }
 
 // The solve's preconditioner: its level shapes (forced, cached, the rule, or the rule until the solve's first
-// applications have measured them) and its graph.  elem: bytes per value of the triangular solves.
-static void build_precond_graph(Context& C, const DevFactor& F, int64_t n, int64_t ld, int32_t kcols, size_t elem,
-                                Precond& P, int64_t& launches, PcgReport& rep, const RowAct& ra,
-                                const PcApply& pc) {
+// applications have measured them).  Its graph is captured by the first application that launches one (pcg_solve).  elem: bytes per value of the triangular solves.
+static void plan_precond(Context& C, const DevFactor& F, int64_t n, int64_t ld, int32_t kcols, size_t elem, Precond& P,
+                         PcgReport& rep, const RowAct& ra) {
     TrsvShapes store;
     uint64_t key = 0;
     const bool narrow = TILE > NARROW_W && kcols <= NARROW_W;
@@ -2065,7 +2065,8 @@ static void build_precond_graph(Context& C, const DevFactor& F, int64_t n, int64
             P.mstep = 0;
         }
     }
-    capture_precond(C, P, launches, pc);
+    P.planned = true;
+    P.drop_graph();
 }
 
 static FactorVals<double> fp64_vals(Context& C, const DevFactor& F, int64_t ld) {
@@ -2216,14 +2217,18 @@ static int32_t pcg_solve(Context& C, int64_t n, int32_t k, int64_t ld, const Spm
             const TrsvShapes f = forced_shapes(F, P.mstep);
             C.kernels_launched += pc(&f, &P.mev[P.mstep]);
             if (++P.mstep == TRSV_NWIDTH) SSP_CUDA(cudaEventRecord(P.m1, C.stream));
+        } else if (device_loop) {
+            // launched once before the loop's own graph takes over: capturing it costs more than its launches
+            C.kernels_launched += pc(P.has_shapes ? &P.shapes : nullptr, nullptr);
         } else {
+            if (!P.exec) capture_precond(C, P, pc_launches, pc);
             SSP_CUDA(cudaGraphLaunch(P.exec, C.stream));
             C.kernels_launched += pc_launches;
         }
         tm.pc.end(C.stream);
     };
     // after a synchronization that follows the last measured application: keep the fastest width per level,
-    // cache it, and rebuild the graph with it
+    // cache it, and drop the graph that lacks it
     auto finish_measure = [&]() {
         if (!P.measure || P.mstep < TRSV_NWIDTH) return;
         shapes_from_events(F, (int)ntiles, P.mev, TRSV_NWIDTH, P.shapes);
@@ -2234,7 +2239,7 @@ static int32_t pcg_solve(Context& C, int64_t n, int32_t k, int64_t ld, const Spm
         P.measure = false;
         cache_shapes(C, P.key, P.shapes);
         report_shapes(rep, SSP_TRSV_TUNED, F, P.shapes, P.plan);
-        capture_precond(C, P, pc_launches, pc);
+        P.drop_graph();
     };
     int64_t active = read_i64(C, S.nactive);
     int32_t it = 0;
@@ -2491,7 +2496,7 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
                     return launch_precond<double>(C, F, P.plan, V64, n, r, z, ld, k, ra, sh, lev);
                 };
             }
-            build_precond_graph(C, F, n, ld, k, elem, P, pc_launches, rep, ra, pc);
+            plan_precond(C, F, n, ld, k, elem, P, rep, ra);
             it = pcg_solve<double>(C, n, k, ld, A, A.val, F, pc, P, pc_launches,
                                    PcgBufs<double>{x, r, z, p, q}, S, R, opt.max_iters, opt, tm, rep, ra);
         }
@@ -2534,7 +2539,7 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
                                                                                    LevelEvents* lev) {
                     return launch_precond<float>(C, F, P32.plan, V32, n, r32, z32, ld, k, ra, sh, lev);
                 };
-                if (!P32.exec) build_precond_graph(C, F, n, ld, k, sizeof(float), P32, pc32, rep, ra, pc32f);
+                if (!P32.planned) plan_precond(C, F, n, ld, k, sizeof(float), P32, rep, ra);
                 int32_t cap = opt.max_iters - it;
                 if (first_its >= 0)
                     cap = std::min(cap, std::max(MIXED_MIN_ROUND_ITERS, MIXED_ROUND_ITER_FACTOR * first_its));
@@ -2559,7 +2564,7 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
                 const PcApply pc64f = [&C, &F, &P64, V64, n, r, z, ld, k, ra](const TrsvShapes* sh, LevelEvents* lev) {
                     return launch_precond<double>(C, F, P64.plan, V64, n, r, z, ld, k, ra, sh, lev);
                 };
-                if (!P64.exec) build_precond_graph(C, F, n, ld, k, sizeof(double), P64, pc64, rep, ra, pc64f);
+                if (!P64.planned) plan_precond(C, F, n, ld, k, sizeof(double), P64, rep, ra);
                 its = pcg_solve<double>(C, n, k, ld, A, A.val, F, pc64f, P64, pc64,
                                         PcgBufs<double>{e64, r, z, p, q}, Si, R, opt.max_iters - it, opt, tm, rep,
                                         ra);
