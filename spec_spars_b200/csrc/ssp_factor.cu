@@ -1429,7 +1429,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
     bool truncated = false;
     int64_t Lused_prev = 0;
     const size_t blk_smem = (size_t)BLOCK_TIER_MAX * (3 * sizeof(double) + 2 * sizeof(int32_t));
-    SSP_CUDA(cudaFuncSetAttribute(k_elim_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)blk_smem));
+    allow_dynamic_smem(C, k_elim_block, blk_smem);
     // several graphs: each graph's own truncation test, with its own live-entry count (the same accounting
     // as the single-graph test below, restricted to its vertices)
     std::vector<int64_t> g_live(nseg, 0), g_elim(nseg, 0), g_prev(nseg, -1), g_cnt(3 * (size_t)nseg + 1, 0);
@@ -1454,7 +1454,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
         if (cap <= 32) return;
         if (cap <= BLOCK_TIER_MAX) {
             size_t smem = (size_t)cap * (2 * sizeof(double) + 2 * sizeof(int32_t));
-            SSP_CUDA(cudaFuncSetAttribute(k_trunc_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            allow_dynamic_smem(C, k_trunc_diag, smem);
             k_trunc_diag<<<(int)std::min<int64_t>(R, 148 * 8), 256, smem, C.stream>>>(F, big, at, cap, nullptr, nullptr, 0);
         } else {
             int blocks = 32;
@@ -1709,8 +1709,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
         SSP_CHECK_LAUNCH();
         int32_t P = 2;
         while (P < T) P <<= 1;
-        SSP_CUDA(cudaFuncSetAttribute(k_sort_rem, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(P * sizeof(int32_t))));
+        allow_dynamic_smem(C, k_sort_rem, (P * sizeof(int32_t)));
         k_sort_rem<<<1, 1024, P * sizeof(int32_t), C.stream>>>(rem, (int32_t)T, P, F.prio, idx);
         SSP_CHECK_LAUNCH();
         double* Wd = W.get_t<double>(nm("W"), (size_t)T * T);
@@ -1721,7 +1720,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
         while (cap < maxlen) cap <<= 1;
         if (cap <= BLOCK_TIER_MAX) {
             size_t smem = (size_t)cap * (2 * sizeof(double) + 2 * sizeof(int32_t));
-            SSP_CUDA(cudaFuncSetAttribute(k_dense_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            allow_dynamic_smem(C, k_dense_build, smem);
             k_dense_build<<<(int)std::min<int64_t>(T, 148 * 4), 256, smem, C.stream>>>(F, rem, (int32_t)T, idx, Wd,
                                                                                         cap, nullptr, nullptr, 0);
         } else {
@@ -1741,7 +1740,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
         }
         // the bitonic sort needs P = pow2 >= T slots per array
         size_t smem = (size_t)P * (2 * sizeof(double) + sizeof(int32_t));
-        SSP_CUDA(cudaFuncSetAttribute(k_dense_elim, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allow_dynamic_smem(C, k_dense_elim, smem);
         k_dense_elim<<<1, 1024, smem, C.stream>>>(F, rem, (int32_t)T, P, idx, Wd, Lused, sparse_levels);
         SSP_CHECK_LAUNCH();
         C.kernels_launched += 5;

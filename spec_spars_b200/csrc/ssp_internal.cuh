@@ -281,6 +281,18 @@ struct DevChunks {
 };
 DevChunks device_chunks(Context& C, const int64_t* ptr, int32_t r0, int32_t r1, const std::string& tag,
                         const std::vector<int32_t>& before = {});
+// Lets kern use smem bytes of dynamic shared memory.  The limit belongs to the function, not to the launch: contexts of
+// several threads share it, so it is always set to the device's most, never to one launch's size, which another thread's
+// launch might exceed in between.  (More than that is refused here.)
+template <class Kernel>
+inline void allow_dynamic_smem(Context& C, Kernel* kern, size_t smem) {
+    cudaFuncAttributes a;
+    int most = 0;
+    SSP_CUDA(cudaFuncGetAttributes(&a, (const void*)kern));
+    SSP_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, C.device));
+    const size_t limit = std::max((size_t)most - a.sharedSizeBytes, smem);
+    SSP_CUDA(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+}
 // the largest of n values on the device (0 at least)
 int32_t device_max_i32(Context& C, const int32_t* v, int64_t n);
 // Copies between pageable host memory and the device on C.stream, returning once the host side is done

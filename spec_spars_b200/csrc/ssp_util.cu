@@ -387,8 +387,7 @@ static void segsort_impl(Context& C, int32_t* keys, double* vals, const int64_t*
         int32_t cap = 64;
         while (cap < std::min(max_len, lim_smem)) cap <<= 1;
         size_t smem = (size_t)cap * (sizeof(int32_t) + (PAIRS ? sizeof(double) : 0));
-        SSP_CUDA(cudaFuncSetAttribute(k_segsort_block<PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+        allow_dynamic_smem(C, k_segsort_block<PAIRS>, smem);
         int blocks = (int)std::min<int64_t>(hc[0], 148 * 4);
         k_segsort_block<PAIRS><<<blocks, 512, smem, C.stream>>>(keys, vals, seg_start, seg_len, list_mid, hc[0],
                                                                 cap, nullptr, nullptr);
