@@ -7,8 +7,8 @@
 // probabilities in [0, 1]: it is formed once per factor (T x T doubles) and the tail of every application is two
 // dense triangular products, y = Linv r and z = Linv^T (D^+ y), with no chain at all.
 //
-// Measured on B200, both directions of one FP64 application (the whole triangular solve, tail included): see
-// launch_precond in ssp_pcg.cu.
+// The figures of the whole application (tail and walked levels) stand at k_trsv_walk in ssp_pcg.cu; what the exact sums of
+// tile_product add to it on B200: 3-D grid n = 80,840 (tail of 1007), 1085 columns, 4.65 -> 4.67 ms.
 #include <algorithm>
 
 #include "ssp_internal.cuh"
@@ -79,15 +79,21 @@ __global__ void __launch_bounds__(32) k_tail_diag(int32_t T, double* __restrict_
         if (i < nb && j < nb && j <= i) M[(o + i) * T + o + j] = x[i];
 }
 
-// One 32 x 32 output tile over k in [k0, k1): out += A(i, k) B(k, j), both fetched through the callers' accessors
+// One 32 x 32 output tile over k in [k0, k1): out = A(i, k) B(k, j), both fetched through the callers' accessors
 // into shared memory (zero outside their ranges).  Thread (ti, tj) holds rows 2 ti, 2 ti + 1 and columns 4 tj ..+3.
+//
+// A sum has up to T terms where a triangular solve's rows have a few, so it is not one chain of additions: chains of
+// SUM_CHAIN terms are added up exactly (Knuth's two-sum, its errors kept in lo) and rounded once.  The error against 64-bit
+// arithmetic then does not grow with T and is that of a solve row by row; one chain was 3 to 15 times further off
+// (tails of 246 and 1110 vertices, FP64 and FP32).
+constexpr int SUM_CHAIN = 8;
 template <class T, class FA, class FB>
-__device__ __forceinline__ void tile_product(int64_t k0, int64_t k1, FA fa, FB fb, T (&acc)[2][4]) {
+__device__ __forceinline__ void tile_product(int64_t k0, int64_t k1, FA fa, FB fb, T (&out)[2][4]) {
     __shared__ T sa[TB][TB + 2];
     __shared__ __align__(16) T sb[TB][TB];
     const int ti = threadIdx.x / 8, tj = threadIdx.x % 8;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    T ra[8], rb[8];
+    T ra[8], rb[8], hi[2][4] = {}, lo[2][4] = {};
     auto fetch = [&](int64_t k) {
 #pragma unroll
         for (int u = 0; u < 8; u++) {
@@ -105,17 +111,33 @@ __device__ __forceinline__ void tile_product(int64_t k0, int64_t k1, FA fa, FB f
         }
         __syncthreads();
         if (k + TB < k1) fetch(k + TB);
-#pragma unroll 8
-        for (int q = 0; q < TB; q++) {
-            const T a0 = sa[2 * ti][q], a1 = sa[2 * ti + 1][q];
+#pragma unroll 1
+        for (int q0 = 0; q0 < TB; q0 += SUM_CHAIN) {
+            T c[2][4] = {};
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const T b = sb[q][4 * tj + j];
-                acc[0][j] += a0 * b;
-                acc[1][j] += a1 * b;
+            for (int q = q0; q < q0 + SUM_CHAIN; q++) {
+                const T a0 = sa[2 * ti][q], a1 = sa[2 * ti + 1][q];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const T b = sb[q][4 * tj + j];
+                    c[0][j] += a0 * b;
+                    c[1][j] += a1 * b;
+                }
             }
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const T h = hi[i][j], s = h + c[i][j], d = s - h;
+                    lo[i][j] += (h - (s - d)) + (c[i][j] - d);
+                    hi[i][j] = s;
+                }
         }
     }
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) out[i][j] = hi[i][j] + lo[i][j];
 }
 
 // A accessors: element (u, lane) of the 32 x 32 fetch is row u, column lane of A (row-major) or, transposed, row
