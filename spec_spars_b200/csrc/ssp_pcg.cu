@@ -916,9 +916,9 @@ __global__ void __launch_bounds__(CH_THREADS, MINB)
 // lpart[segment][column], and k_spmm_long adds a row's segments up: a hub's row, walked by one warp, kept a whole launch
 // waiting.  The lanes of a row have eight gathers in flight, its last entries (under predicates) among them, in four
 // accumulators: a grid's row of seven entries costs one gather latency, where a loop over the last three added three.
-// Bound by random 256-byte row gathers through L2 (51 GB in 5.0 ms at ER n = 250,000).  Measured on B200, one FP64 product,
+// Bound by random 256-byte row gathers through L2 (51 GB in 5.25 ms at ER n = 250,000).  Measured on B200, one FP64 product,
 // with the long rows walked whole and serial last entries -> here: R-MAT n = 24,281, 883K entries, 2693 columns 4.21 ->
-// 1.60 ms; 3-D grid n = 80,840, 1085 columns 1.05 -> 0.58; ER n = 250,000, degree 20, 1194 columns 6.4 -> 5.0; ER n = 1M, 80
+// 1.78 ms; 3-D grid n = 80,840, 1085 columns 1.05 -> 0.57; ER n = 250,000, degree 20, 1194 columns 6.4 -> 5.25; ER n = 1M, 80
 // columns 2.70 -> 2.10.  FP32 (spmm_row_pair) 3.08 -> 2.37 ms at ER n = 229,373, 1185 columns.  Slower: 16-column halves of a
 // tile, whose gathered rows then fit L2 (2.89 against 2.75 ms at ER n = 1M); FP64 in 16-byte pieces the same way (6.2 ms
 // against 5.06 at ER n = 250,000); FP32 with 3, 5 or 6 pairs in flight (2.67, 2.90, 2.98) and a half-warp per row (3.83).
@@ -933,8 +933,14 @@ struct SpmmItems {
     const int32_t* lrow = nullptr;    // rows of more than CHUNK_CAP entries
     const int32_t* lseg = nullptr;    // nlong + 1 first segments
 };
+// Up to SPMM_SEG entries of a row are summed in four chains, a longer row segment by segment.  Rows of 100 to 256 entries in
+// four chains throughout (FP32: two) were rounded 1.2 to 1.3 (1.6 to 1.8) times worse than in the eight of a lane per value;
+// here it is 0.86 to 0.97 (1.02 to 1.04) times.  The products take 1.65 -> 1.78 ms (R-MAT as above), 5.09 -> 5.25 (ER
+// n = 250,000), 0.58 -> 0.57 (3-D grid); eight chains, whose registers cost gathers in flight, made the whole ER call 230 ms
+// instead of 189.
+constexpr int SPMM_SEG = 32;
 template <class T>
-__device__ __forceinline__ T spmm_row(const int32_t* si, const T* sv, int32_t q, int32_t q1, const T* xt) {
+__device__ __forceinline__ T spmm_seg(const int32_t* si, const T* sv, int32_t q, int32_t q1, const T* xt) {
     T a[4] = {0, 0, 0, 0};
     for (; q + 7 < q1; q += 8) {
         T x[8];
@@ -953,10 +959,17 @@ __device__ __forceinline__ T spmm_row(const int32_t* si, const T* sv, int32_t q,
     }
     return (a[0] + a[1]) + (a[2] + a[3]);
 }
+template <class T>
+__device__ __forceinline__ T spmm_row(const int32_t* si, const T* sv, int32_t q, int32_t q1, const T* xt) {
+    if (q1 - q <= SPMM_SEG) return spmm_seg<T>(si, sv, q, q1, xt);
+    T tot = 0;
+    for (; q < q1; q += SPMM_SEG) tot += spmm_seg<T>(si, sv, q, min(q + SPMM_SEG, q1), xt);
+    return tot;
+}
 
 // The same sums of an FP32 row by a whole warp: a lane has two columns, and the half-warps take every second entry, so that
-// a load instruction moves 256 bytes as in FP64.  Both halves return the row's sums.  (q0, q1: the row's entries;
-// xt: at the lane's first column)
+// a load instruction moves 256 bytes as in FP64.  Both halves return the row's sums; a half adds up
+// four entries before they join its chain.  (q0, q1: the row's entries; xt: at the lane's first column)
 __device__ __forceinline__ float2 spmm_row_pair(const int32_t* si, const float* sv, int32_t q0, int32_t q1,
                                                 const float* xt, int half) {
     constexpr int U = 4;
@@ -966,23 +979,23 @@ __device__ __forceinline__ float2 spmm_row_pair(const int32_t* si, const float* 
         float2 x[U];
 #pragma unroll
         for (int u = 0; u < U; u++) x[u] = *reinterpret_cast<const float2*>(xt + (int64_t)si[q + 2 * u] * TILE);
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            a.x += sv[q + 2 * u] * x[u].x;
-            a.y += sv[q + 2 * u] * x[u].y;
-        }
+        const float v0 = sv[q], v1 = sv[q + 2], v2 = sv[q + 4], v3 = sv[q + 6];
+        a.x += (v0 * x[0].x + v1 * x[1].x) + (v2 * x[2].x + v3 * x[3].x);
+        a.y += (v0 * x[0].y + v1 * x[1].y) + (v2 * x[2].y + v3 * x[3].y);
     }
     if (q < q1) {
-        float2 x[U - 1];
+        float2 x[U - 1], t = {0, 0};
 #pragma unroll
         for (int u = 0; u < U - 1; u++)
             if (q + 2 * u < q1) x[u] = *reinterpret_cast<const float2*>(xt + (int64_t)si[q + 2 * u] * TILE);
 #pragma unroll
         for (int u = 0; u < U - 1; u++)
             if (q + 2 * u < q1) {
-                a.x += sv[q + 2 * u] * x[u].x;
-                a.y += sv[q + 2 * u] * x[u].y;
+                t.x += sv[q + 2 * u] * x[u].x;
+                t.y += sv[q + 2 * u] * x[u].y;
             }
+        a.x += t.x;
+        a.y += t.y;
     }
     __syncwarp();
     a.x += __shfl_xor_sync(0xffffffffu, a.x, 16);
