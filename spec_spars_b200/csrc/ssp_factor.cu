@@ -661,19 +661,31 @@ __global__ void k_fill_scatter(FDev F) {
 // graph 32 -> 24.5 ms, of a 40^3 grid 27.5 -> 22).  It starts with a level whose capacities the host has checked, and
 // at every level boundary takes the host loop's own decisions on the same numbers; what it does not handle (a
 // truncation, the dense tail, a pool to compact, buffers to grow, bags above ELIM_LIVE_MAX, wide frontiers) ends it
-// there, and the host loop goes on from the state it leaves.
+// there, and the host loop goes on from the state it leaves.  So does a stream that cannot hold all of its blocks at once: the
+// launch is refused, or its blocks give up before the first level (ST_GO).
 // ELIM_FRONT_MAX: 3.5 vertices for each warp of the grid; such a level takes 86-90 us here, as in the host loop, and wider
 // ones are better spread over the launches' larger grids.  ELIM_LIVE_MAX: what fits the static shared memory.
-enum { ST_LIVE = 0, ST_ELIM, ST_LVL, ST_PREV, ST_LUSED, ST_STOP, ST_ERR, ST_N };
+enum { ST_LIVE = 0, ST_ELIM, ST_LVL, ST_PREV, ST_LUSED, ST_STOP, ST_ERR, ST_GO, ST_N };
+enum { GO_ALL = 1, GO_NONE = 2 };  // ST_GO: every block has arrived, or a block has given up waiting for the others
 constexpr int ELIM_THREADS = 256, ELIM_LIVE_MAX = 512;
 constexpr int64_t ELIM_FRONT_MAX = 4096;
+
+// The launch's blocks (one per SM) and the limit of the wait for them to run; the environment variables make either too
+// much for the device, which takes the ways back to the host loop.
+static int env_int(const char* name, int value) {
+    const char* e = getenv(name);
+    return e && e[0] ? atoi(e) : value;
+}
+static int level_blocks(int sms) { return env_int("SSP_FACTOR_LEVEL_BLOCKS", sms); }
+static int level_start_spins() { return env_int("SSP_FACTOR_LEVEL_SPINS", 1 << 20); }
 
 struct ElimArgs {
     FDev F;
     int32_t* front[2];  // frontier of the first level and the other list, in turn
     int32_t *live_cnt, *list_b, *list_g;
     int64_t* st;             // ST_*
-    unsigned* bar;           // arrivals, releases
+    int start_spins;         // limit on the wait for all blocks to run
+    unsigned* bar;           // arrivals, releases, blocks that run
     int32_t* log;            // frontier size by level
     int64_t max_degree, dense_threshold, pool_init, pool_cap, Lcap, Fcap;
     // several graphs: per graph its vertices, truncation, and the accounting of ST_LIVE, ST_ELIM, ST_PREV
@@ -681,8 +693,26 @@ struct ElimArgs {
     int64_t *g_live, *g_elim, *g_prev;
 };
 
-// Barrier over the grid; the last block to arrive runs ctl (all its threads) before the others go on.  The wait is
-// bounded (some ten seconds: blocks may have to wait for other streams' kernels before they all run); past that the
+// Waits until every block of the grid runs, or gives up after some tenths of a second (other work may hold a part of the
+// device).  One compare-and-swap decides between the last block to arrive and the first to give up, so all blocks, also
+// those that come later, return the same; nothing has been changed when they return false.
+__device__ bool all_blocks_run(const ElimArgs& A) {
+    __shared__ int s_go;
+    if (threadIdx.x == 0) {
+        unsigned long long* go = (unsigned long long*)&A.st[ST_GO];
+        if (atomicAdd(&A.bar[2], 1u) == gridDim.x - 1) atomicCAS(go, 0ull, (unsigned long long)GO_ALL);
+        for (int spins = 0; *(volatile unsigned long long*)go == 0; spins++) {
+            if (spins >= A.start_spins) atomicCAS(go, 0ull, (unsigned long long)GO_NONE);
+            else if (spins > 1024) __nanosleep(100);
+        }
+        s_go = *(volatile unsigned long long*)go == GO_ALL;
+    }
+    __syncthreads();
+    return s_go != 0;
+}
+
+// Barrier over the grid; the last block to arrive runs ctl (all its threads) before the others go on.  All blocks run
+// (all_blocks_run), so the wait is one for a part of a level; it is bounded all the same (some ten seconds), and past that the
 // kernel reports ST_ERR and ends.  Returns false then.
 template <class Ctl>
 __device__ bool grid_barrier(const ElimArgs& A, Ctl ctl) {
@@ -783,6 +813,7 @@ __global__ void __launch_bounds__(ELIM_THREADS) k_elim_levels(ElimArgs A) {
         __syncthreads();
         begin();
     };
+    if (!all_blocks_run(A)) return;
     if (!grid_barrier(A, begin)) return;
     for (int cur = 0;; cur ^= 1) {
         const int32_t* frontier = A.front[cur];
@@ -1427,6 +1458,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
     }
     int64_t prev_fcur = -1;
     bool truncated = false;
+    bool many_levels = true;  // small frontiers' levels in one launch, until a stream turns out not to hold it
     int64_t Lused_prev = 0;
     const size_t blk_smem = (size_t)BLOCK_TIER_MAX * (3 * sizeof(double) + 2 * sizeof(int32_t));
     allow_dynamic_smem(C, k_elim_block, blk_smem);
@@ -1575,10 +1607,10 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
             F.fill_b = W.get_t<int32_t>(nm("fill_b"), Fcap);
             F.fill_w = W.get_t<double>(nm("fill_w"), Fcap);
         }
-        if (nf <= ELIM_FRONT_MAX && h[C_NG] == 0 && h[C_MAXLIVE] <= ELIM_LIVE_MAX) {
+        if (many_levels && nf <= ELIM_FRONT_MAX && h[C_NG] == 0 && h[C_MAXLIVE] <= ELIM_LIVE_MAX) {
             // this level and those after it, up to one that needs the host
-            int64_t st[ST_N] = {live_entries, eliminated, lvl, -1, Lused_prev, 0, 0};
-            int64_t* d_st = W.get_t<int64_t>(nm("el_st"), ST_N + 1);
+            int64_t st[ST_N] = {live_entries, eliminated, lvl, -1, Lused_prev, 0, 0, 0};
+            int64_t* d_st = W.get_t<int64_t>(nm("el_st"), ST_N + 2);
             int64_t* d_g = W.get_t<int64_t>(nm("el_g"), 5 * (size_t)nseg + 1);
             int32_t* d_log = W.get_t<int32_t>(nm("el_log"), n + 1);
             std::vector<int64_t> hg;
@@ -1586,7 +1618,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
             // a stopped graph has no vertex in a frontier any more, so its test never holds again
             for (const auto* v : {&g_maxdeg, &g_live, &g_elim, &g_prev}) hg.insert(hg.end(), v->begin(), v->end());
             SSP_CUDA(cudaMemcpyAsync(d_st, st, sizeof(st), cudaMemcpyHostToDevice, C.stream));
-            SSP_CUDA(cudaMemsetAsync(d_st + ST_N, 0, sizeof(int64_t), C.stream));
+            SSP_CUDA(cudaMemsetAsync(d_st + ST_N, 0, 2 * sizeof(int64_t), C.stream));
             if (nseg)
                 SSP_CUDA(cudaMemcpyAsync(d_g, hg.data(), sizeof(int64_t) * hg.size(), cudaMemcpyHostToDevice, C.stream));
             ElimArgs A;
@@ -1597,6 +1629,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
             A.list_b = list_b;
             A.list_g = list_g;
             A.st = d_st;
+            A.start_spins = level_start_spins();
             A.bar = (unsigned*)(d_st + ST_N);
             A.log = d_log;
             A.max_degree = opt.max_degree;
@@ -1613,29 +1646,39 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
             int sms = 0;
             SSP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, C.device));
             void* args[] = {&A};
-            SSP_CUDA(cudaLaunchCooperativeKernel((const void*)k_elim_levels, dim3((unsigned)sms), dim3(ELIM_THREADS), args, 0,
-                                                 C.stream));
-            C.kernels_launched++;
-            read_i64s(C, d_st, st, ST_N);
-            if (st[ST_ERR]) throw Error(SSP_ERR_CUDA, "factor: a level's barrier was not reached in time");
-            const int32_t done = (int32_t)st[ST_LVL] - lvl;
-            std::vector<int32_t> sizes(done);
-            SSP_CUDA(cudaMemcpyAsync(sizes.data(), d_log + lvl, sizeof(int32_t) * done, cudaMemcpyDeviceToHost, C.stream));
-            if (nseg) {
-                read_i64s(C, A.g_live, g_live.data(), nseg);
-                read_i64s(C, A.g_elim, g_elim.data(), nseg);
-                read_i64s(C, A.g_prev, g_prev.data(), nseg);
+            const cudaError_t le = cudaLaunchCooperativeKernel((const void*)k_elim_levels, dim3((unsigned)level_blocks(sms)),
+                                                               dim3(ELIM_THREADS), args, 0, C.stream);
+            if (le == cudaErrorCooperativeLaunchTooLarge || le == cudaErrorLaunchOutOfResources ||
+                le == cudaErrorNotSupported) {
+                cudaGetLastError();
+                many_levels = false;
+            } else {
+                SSP_CUDA(le);
+                C.kernels_launched++;
+                read_i64s(C, d_st, st, ST_N);
+                if (st[ST_ERR]) throw Error(SSP_ERR_CUDA, "factor: a level's barrier was not reached in time");
+                many_levels = st[ST_GO] == GO_ALL;
             }
-            SSP_CUDA(cudaStreamSynchronize(C.stream));
-            out.frontier_sizes.pop_back();
-            out.frontier_sizes.insert(out.frontier_sizes.end(), sizes.begin(), sizes.end());
-            live_entries = st[ST_LIVE];
-            eliminated = st[ST_ELIM];
-            lvl = (int32_t)st[ST_LVL];
-            prev_fcur = st[ST_PREV];
-            Lused_prev = st[ST_LUSED];
-            if (done & 1) std::swap(frontier, next);
-            continue;
+            if (many_levels) {
+                const int32_t done = (int32_t)st[ST_LVL] - lvl;
+                std::vector<int32_t> sizes(done);
+                SSP_CUDA(cudaMemcpyAsync(sizes.data(), d_log + lvl, sizeof(int32_t) * done, cudaMemcpyDeviceToHost, C.stream));
+                if (nseg) {
+                    read_i64s(C, A.g_live, g_live.data(), nseg);
+                    read_i64s(C, A.g_elim, g_elim.data(), nseg);
+                    read_i64s(C, A.g_prev, g_prev.data(), nseg);
+                }
+                SSP_CUDA(cudaStreamSynchronize(C.stream));
+                out.frontier_sizes.pop_back();
+                out.frontier_sizes.insert(out.frontier_sizes.end(), sizes.begin(), sizes.end());
+                live_entries = st[ST_LIVE];
+                eliminated = st[ST_ELIM];
+                lvl = (int32_t)st[ST_LVL];
+                prev_fcur = st[ST_PREV];
+                Lused_prev = st[ST_LUSED];
+                if (done & 1) std::swap(frontier, next);
+                continue;
+            }
         }
         Lused_prev = h[C_LCUR];
         prev_fcur = h[C_FCUR];
