@@ -14,6 +14,7 @@
 // latency-bound levels (R-MAT scale 18, measured on B200: 7,107 levels, 1.46 s per preconditioner application
 // and 84 s per sparsification, against 4.9 ms and 4.0 s for the light factor at 56 instead of 54 iterations).
 // Otherwise the elimination runs to completion.  Both factorizations, and so the choice, are deterministic.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -41,8 +42,10 @@ double autotune_predicted_iters(const std::vector<double>& hist, double tol) {
     const double tol_rel = tol > 0 ? tol : 1e-6;
     double iters = 1e9;
     const size_t h = hist.size();
-    if (h >= 2 && hist.back() <= tol_rel) {
-        iters = (double)h;  // converged within the probe
+    // Converged within the probe, at its end or before: iterations past convergence run on rounding errors and may end
+    // anywhere (dense graphs converge in six of the probe's twenty), which says nothing about the factor.
+    if (h >= 2 && std::any_of(hist.begin() + 1, hist.end(), [&](double r) { return r <= tol_rel; })) {
+        iters = (double)h;
     } else if (h >= 4) {
         const size_t a = h / 2;
         const double r0 = hist[a - 1], r1 = hist[h - 1];
