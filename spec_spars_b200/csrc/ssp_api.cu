@@ -217,13 +217,14 @@ struct HostOutBuffers {
 constexpr int64_t HOST_OUT_PREFAULT_MIN = 1 << 20;  // entries; smaller outputs allocate at the end
 
 // Columns solved per pass.  The PCG holds six n x ld FP64 blocks (sketch, x, r, z, p, q; the mixed mode adds
-// five FP32 blocks and an FP64 increment), which for the R-MAT configuration (scale 22, eps 0.3: k = 3917)
+// five FP32 blocks and an FP64 increment; rows of more than CHUNK_CAP entries add up to half a block of partial sums), which for the R-MAT configuration (scale 22, eps 0.3: k = 3917)
 // need 450 GB.  The columns are independent once the factor exists, so they are solved in batches of whole
 // 32-column tiles.  Whether to batch is decided before the factorization with room set aside for it (70 % of
 // the free memory, less 40 B per Laplacian entry and 48 B per edge); the batch size after it, from the memory
 // then free (80 %, less the per-edge arrays).  SSP_COLUMN_BATCH=<columns> sets the batch.
-static double column_bytes(int64_t n, int32_t precision) {
-    return (double)n * (8.0 * 6 + (precision == SSP_PRECISION_MIXED ? 4.0 * 5 + 8.0 : 0.0));
+static double column_bytes(const DevGraph& G, int32_t precision) {
+    return (double)G.n * (8.0 * 6 + (precision == SSP_PRECISION_MIXED ? 4.0 * 5 + 8.0 : 0.0) +
+                          (G.max_deg >= CHUNK_CAP ? 4.0 : 0.0));
 }
 static int32_t forced_batch(int32_t k) {
     if (const char* e = getenv("SSP_COLUMN_BATCH")) {
@@ -250,12 +251,12 @@ static double free_for_solve(Context& C) {
     return (double)fr + (double)(C.ws.bytes_with_prefix("sp_Y") + C.ws.bytes_with_prefix("pcg"));
 }
 static bool columns_fit(Context& C, const DevGraph& G, int32_t k, int32_t precision) {
-    const double need = column_bytes(G.n, precision) * (double)tile_ld(k);
+    const double need = column_bytes(G, precision) * (double)tile_ld(k);
     return need <= 0.7 * free_for_solve(C) - 40.0 * (double)G.lap_nnz - 48.0 * (double)G.m;
 }
 static int32_t batch_after_factor(Context& C, const DevGraph& G, int32_t k, int32_t precision) {
     const double avail = 0.8 * free_for_solve(C) - 48.0 * (double)G.m - (1.0 * (1 << 30));
-    const int64_t cols = (int64_t)(avail / column_bytes(G.n, precision)) / SSP_TILE * SSP_TILE;
+    const int64_t cols = (int64_t)(avail / column_bytes(G, precision)) / SSP_TILE * SSP_TILE;
     return (int32_t)std::max<int64_t>(SSP_TILE, std::min<int64_t>(cols, k));
 }
 

@@ -914,7 +914,8 @@ __global__ void __launch_bounds__(CH_THREADS, MINB)
 // ---------------------------------------------------------------- q = A p
 // A warp's item is a chunk (as above) or a segment of CHUNK_CAP entries of a longer row.  A segment's sums go to
 // lpart[segment][column], and k_spmm_long adds a row's segments up: a hub's row, walked by one warp, kept a whole launch
-// waiting.  The lanes of a row have eight gathers in flight, its last entries (under predicates) among them, in four
+// waiting.  Where most rows are that long, lpart holds some tiles' columns only and a product is launched in groups of
+// tiles (SpmmPlan::group).  The lanes of a row have eight gathers in flight, its last entries (under predicates) among them, in four
 // accumulators: a grid's row of seven entries costs one gather latency, where a loop over the last three added three.
 // Bound by random 256-byte row gathers through L2 (51 GB in 5.25 ms at ER n = 250,000).  Measured on B200, one FP64 product,
 // with the long rows walked whole and serial last entries -> here: R-MAT n = 24,281, 883K entries, 2693 columns 4.21 ->
@@ -1008,7 +1009,7 @@ template <class T, int W, bool ACC>
 __global__ void __launch_bounds__(CH_THREADS, 6)
     k_spmm(int64_t n, SpmmItems S, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
            const T* __restrict__ val, const T* __restrict__ p, T* __restrict__ q, int64_t ld, T* __restrict__ lpart,
-           double* __restrict__ part, int32_t kcols, RowAct ra) {
+           int64_t lld, double* __restrict__ part, int32_t kcols, RowAct ra) {
     __shared__ int32_t s_idx[CH_WARPS][CHUNK_CAP];
     __shared__ T s_val[CH_WARPS][CHUNK_CAP];
     __shared__ int32_t s_ptr[CH_WARPS][CHUNK_ROWS + 1];
@@ -1043,7 +1044,7 @@ __global__ void __launch_bounds__(CH_THREADS, 6)
                 float2 acc = spmm_row_pair(si, sv, sp[rr], t * TILE + col < kcols ? sp[rr + 1] : 0, xt + col, half);
                 if (half) continue;
                 if (seg) {
-                    *reinterpret_cast<float2*>(lpart + (int64_t)c * ld + t * TILE + col) = acc;
+                    *reinterpret_cast<float2*>(lpart + (int64_t)c * lld + t * TILE + col) = acc;
                     continue;
                 }
                 const int64_t o = toff + row * TILE + col;
@@ -1071,7 +1072,7 @@ __global__ void __launch_bounds__(CH_THREADS, 6)
             T acc = spmm_row<T>(si, sv, q0, q1, xt + col);
             if (!on) continue;
             if (seg) {
-                lpart[(int64_t)c * ld + t * TILE + col] = acc;
+                lpart[(int64_t)c * lld + t * TILE + col] = acc;
             } else {
                 // q streams out (evict-first), so it does not push the gathered slab out of L2
                 const int64_t o = toff + row * TILE + col;
@@ -1099,9 +1100,9 @@ __global__ void __launch_bounds__(CH_THREADS, 6)
     }
 }
 
-// the long rows: their segments' sums in order into q, and their share of p.q (grid: x over rows, y over tiles)
+// the long rows: their segments' sums in order into q, and their share of p.q (grid: x over rows, y over the group's tiles)
 template <class T, bool ACC>
-__global__ void __launch_bounds__(CH_THREADS) k_spmm_long(int64_t n, SpmmItems S, const T* __restrict__ lpart,
+__global__ void __launch_bounds__(CH_THREADS) k_spmm_long(int64_t n, SpmmItems S, const T* __restrict__ lpart, int64_t lld,
                                                           const T* __restrict__ p, T* __restrict__ q, int64_t ld,
                                                           double* __restrict__ part, int32_t kcols, RowAct ra) {
     __shared__ double s_red[CH_THREADS];
@@ -1114,7 +1115,7 @@ __global__ void __launch_bounds__(CH_THREADS) k_spmm_long(int64_t n, SpmmItems S
         if (!row_on(ra, row, t)) continue;
         T acc = 0;
 #pragma unroll 4
-        for (int32_t g = S.lseg[i]; g < S.lseg[i + 1] && live; g++) acc += lpart[(int64_t)g * ld + t * TILE + lane];
+        for (int32_t g = S.lseg[i]; g < S.lseg[i + 1] && live; g++) acc += lpart[(int64_t)g * lld + t * TILE + lane];
         const int64_t o = toff + row * TILE + lane;
         if (ACC) acc += q[o];
         q[o] = acc;
@@ -1156,7 +1157,7 @@ __global__ void __launch_bounds__(CH_THREADS) k_spmm_diff(int64_t n, SpmmItems S
                                                           const double* __restrict__ val,
                                                           const int32_t* __restrict__ eid, const double* xt,
                                                           double* qt, int32_t kcols, double* __restrict__ d2,
-                                                          int first, double* __restrict__ lpart, int64_t ld) {
+                                                          int first, double* __restrict__ lpart, int64_t lld) {
     __shared__ int32_t s_idx[CH_WARPS][CHUNK_CAP];
     __shared__ double s_val[CH_WARPS][CHUNK_CAP];
     __shared__ int32_t s_eid[CH_WARPS][CHUNK_CAP];
@@ -1213,7 +1214,7 @@ __global__ void __launch_bounds__(CH_THREADS) k_spmm_diff(int64_t n, SpmmItems S
                 }
             }
             const double sum = (a[0] + a[1]) + (a[2] + a[3]);
-            if (seg) lpart[(int64_t)c * ld + lane] = sum;
+            if (seg) lpart[(int64_t)c * lld + lane] = sum;
             else __stcs(qt + row * TILE + lane, sum);
         }
         __syncwarp();
@@ -1877,7 +1878,10 @@ struct SpmmPlan {
     unsigned long_blocks = 0;     // x blocks of k_spmm_long for the last slab (p.q partials follow the grid's)
     int nparts = 0;               // partials of p.q per column
     int launches = 0;             // of one product
-    double* lpart = nullptr;      // sums of the long rows' segments (both precisions)
+    // Sums of the long rows' segments (both precisions), for `group` tiles at a time: as many as fit half an n x ld block,
+    // one at least.  At 1000 entries a row the segments of all columns would be five blocks beside the solve's six.
+    double* lpart = nullptr;
+    int group = 1;
     double* part = nullptr;
 };
 
@@ -2008,9 +2012,13 @@ static SpmmPlan make_spmm_plan(Context& C, int64_t n, const int64_t* lap_ptr, co
     const int32_t nl = A.items[m - 1].nlong;
     A.long_blocks = nl ? (unsigned)std::min(ceil_div(nl, CH_WARPS), 64) : 0;
     A.nparts = bx + (int)A.long_blocks;
-    A.launches = m;
-    for (int32_t b = 0; b < m; b++) A.launches += A.items[b].nlong > 0;
-    A.lpart = most_seg ? W.get_t<double>("pcg_lpart", (size_t)most_seg * ld) : nullptr;
+    const int ntiles = (int)(ld / TILE);
+    A.group = ntiles;
+    if (most_seg) {
+        A.group = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, n * ld / 2 / ((int64_t)most_seg * TILE)));
+        A.lpart = W.get_t<double>("pcg_lpart", (size_t)most_seg * A.group * TILE);
+    }
+    for (int32_t b = 0; b < m; b++) A.launches += A.items[b].nlong > 0 ? 2 * ceil_div(ntiles, A.group) : 1;
     A.part = W.get_t<double>("pcg_spmm_part", (size_t)A.nparts * ld);
     return A;
 }
@@ -2027,12 +2035,23 @@ static void launch_spmm(Context& C, int64_t n, const SpmmPlan& A, const T* aval,
         double* part = dot && b == A.nslabs - 1 ? A.part : nullptr;
         auto kern = narrow ? (b == 0 ? k_spmm<T, NARROW_W, false> : k_spmm<T, NARROW_W, true>)
                            : (b == 0 ? k_spmm<T, TILE, false> : k_spmm<T, TILE, true>);
-        kern<<<A.grid, CH_THREADS, 0, C.stream>>>(n, I, ptr, A.idx, aval, p, q, ld, lpart, part, kcols, ra);
-        if (I.nlong == 0) continue;
-        const dim3 grid(part ? A.long_blocks : (unsigned)std::min(ceil_div(I.nlong, CH_WARPS), 64), A.grid.y);
+        const int ntiles = (int)A.grid.y, group = I.nlong ? A.group : ntiles;
+        const int64_t lld = (int64_t)A.group * TILE;
+        const unsigned lx = part ? A.long_blocks : (unsigned)std::min(ceil_div(I.nlong, CH_WARPS), 64);
         auto fin = b == 0 ? k_spmm_long<T, false> : k_spmm_long<T, true>;
-        fin<<<grid, CH_THREADS, 0, C.stream>>>(n, I, lpart, p, q, ld, part ? part + (int64_t)A.grid.x * ld : nullptr, kcols,
-                                               ra);
+        for (int t0 = 0; t0 < ntiles; t0 += group) {
+            // the kernels count tiles and columns from the group's first
+            const unsigned nt = (unsigned)std::min(group, ntiles - t0);
+            const int64_t o = (int64_t)t0 * n * TILE;
+            const int32_t kc = kcols - t0 * TILE;
+            RowAct rg = ra;
+            if (rg.act) rg.act += t0;
+            double* pt = part ? part + t0 * TILE : nullptr;
+            kern<<<dim3(A.grid.x, nt), CH_THREADS, 0, C.stream>>>(n, I, ptr, A.idx, aval, p + o, q + o, ld, lpart, lld, pt, kc, rg);
+            if (I.nlong == 0) continue;
+            fin<<<dim3(lx, nt), CH_THREADS, 0, C.stream>>>(n, I, lpart, lld, p + o, q + o, ld,
+                                                           pt ? pt + (int64_t)A.grid.x * ld : nullptr, kc, rg);
+        }
     }
 }
 
@@ -2614,18 +2633,21 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
     }
     // true relative residual ||(Y - mean) - A x|| / ||Y - mean|| (with the edges' squared diff norms when asked)
     if (lap_eid && d2 && A.nslabs == 1) {
-        for (int64_t t = 0; t < ntiles; t++)
+        const SpmmItems& I = A.items[0];
+        const int64_t lld = (int64_t)A.group * TILE;
+        for (int64_t t = 0; t < ntiles; t++) {
             k_spmm_diff<<<dim3(A.grid.x, 1), CH_THREADS, 0, C.stream>>>(
-                n, A.items[0], A.ptr, A.idx, A.val, lap_eid, x + t * n * TILE, q + t * n * TILE,
-                (int32_t)(k - t * TILE), d2, (t == 0 && !d2_accumulate) ? 1 : 0, A.lpart ? A.lpart + t * TILE : nullptr, ld);
-        SSP_CHECK_LAUNCH();
-        C.kernels_launched += ntiles;
-        if (A.items[0].nlong) {
-            k_spmm_long<double, false><<<dim3(A.long_blocks, (unsigned)ntiles), CH_THREADS, 0, C.stream>>>(
-                n, A.items[0], A.lpart, x, q, ld, nullptr, k, RowAct());
-            SSP_CHECK_LAUNCH();
+                n, I, A.ptr, A.idx, A.val, lap_eid, x + t * n * TILE, q + t * n * TILE, (int32_t)(k - t * TILE), d2,
+                (t == 0 && !d2_accumulate) ? 1 : 0, A.lpart ? A.lpart + t % A.group * TILE : nullptr, lld);
+            C.kernels_launched++;
+            // the group's long rows, once its last tile's segments are summed
+            if (I.nlong == 0 || (t + 1 < ntiles && (t + 1) % A.group)) continue;
+            const int64_t t0 = t / A.group * A.group;
+            k_spmm_long<double, false><<<dim3(A.long_blocks, (unsigned)(t + 1 - t0)), CH_THREADS, 0, C.stream>>>(
+                n, I, A.lpart, lld, x + t0 * n * TILE, q + t0 * n * TILE, ld, nullptr, (int32_t)(k - t0 * TILE), RowAct());
             C.kernels_launched++;
         }
+        SSP_CHECK_LAUNCH();
         rep.diff_fused = true;
     } else {
         launch_spmm<double>(C, n, A, A.val, x, q, ld, false, k);
