@@ -248,7 +248,7 @@ static double free_for_solve(Context& C) {
         fr += (size_t)(reserved - used);
     cudaGetLastError();
     // the solve's own buffers from an earlier call are reused
-    return (double)fr + (double)(C.ws.bytes_with_prefix("sp_Y") + C.ws.bytes_with_prefix("pcg"));
+    return std::min((double)fr, C.ws.room()) + (double)(C.ws.bytes_with_prefix("sp_Y") + C.ws.bytes_with_prefix("pcg"));
 }
 static bool columns_fit(Context& C, const DevGraph& G, int32_t k, int32_t precision) {
     const double need = column_bytes(G, precision) * (double)tile_ld(k);

@@ -1326,13 +1326,13 @@ __global__ void k_perm_copy(int64_t n, const int32_t* perm, const int64_t* ptr, 
     for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nw) {
         const int32_t v = perm[i];
         const int64_t s = ptr[v], d = pptr[i], c = ptr[v + 1] - s;
-        if (lane == 0) prow[i] = FactorRow{v, (int32_t)c, d};
+        if (lane == 0 && prow) prow[i] = FactorRow{v, (int32_t)c, d};
         for (int64_t q = lane; q < c; q += 32) {
             const int32_t u = idx[s + q];
             const double x = val[s + q];
             pidx[d + q] = u;
             pval[d + q] = x;
-            pent[d + q] = FactorEnt<double>{x, u};
+            if (pent) pent[d + q] = FactorEnt<double>{x, u};
         }
     }
 }
@@ -1478,7 +1478,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
     // D of the R vertices rem (their live bags hold at most cap entries): warps, then blocks for the larger bags, whose
     // list's length stays on the device
     auto trunc_diag = [&](const int32_t* rem, int64_t R, int32_t at, int32_t cap) {
-        int32_t* big = W.get_t<int32_t>(nm("trunc_big"), n);
+        int32_t* big = list_b;  // (a level's lists are made after its truncations)
         SSP_CUDA(cudaMemsetAsync(F.ctr + C_NB, 0, sizeof(int64_t), C.stream));
         k_trunc_diag_warp<<<grid_for(R * 32, T256, 148 * 64), T256, 0, C.stream>>>(F, rem, (int32_t)R, big);
         SSP_CHECK_LAUNCH();
@@ -1612,7 +1612,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
             int64_t st[ST_N] = {live_entries, eliminated, lvl, -1, Lused_prev, 0, 0, 0};
             int64_t* d_st = W.get_t<int64_t>(nm("el_st"), ST_N + 2);
             int64_t* d_g = W.get_t<int64_t>(nm("el_g"), 5 * (size_t)nseg + 1);
-            int32_t* d_log = W.get_t<int32_t>(nm("el_log"), n + 1);
+            int32_t* d_log = deg;  // (no longer needed)
             std::vector<int64_t> hg;
             for (int32_t g = 0; g < nseg; g++) hg.push_back(opt.seg_row0[g + 1] - opt.seg_row0[g]);
             // a stopped graph has no vertex in a frontier any more, so its test never holds again
@@ -1842,9 +1842,10 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
     // work, and everything laid out from here on (and the order in which the solves add a row up) is the same in every run
     out.level_cols = W.get_t<int32_t>(nm("level_cols"), n);
     {
-        uint64_t* key = W.get_t<uint64_t>(nm("lvkey"), n);
-        uint64_t* tkey = W.get_t<uint64_t>(nm("lvkey2"), n);
-        int32_t* tval = W.get_t<int32_t>(nm("lvval2"), n);
+        // the elimination's lists are free now
+        uint64_t* key = (uint64_t*)F.fstart;
+        uint64_t* tkey = (uint64_t*)F.bag_start;
+        int32_t* tval = list_b;
         int bits = 9;
         while (bits < 40 && (int64_t(256) << (bits - 8)) < (int64_t)NL * 256) bits++;
         for (int f = 0; f < 2; f++) {
@@ -1866,6 +1867,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
     for (int32_t l = 0; l <= NL; l++) out.level_ptr[l] = (int32_t)lp[l];
     for (int32_t l = 0; l < NL; l++) out.max_level_rows = std::max(out.max_level_rows, (int32_t)(lp[l + 1] - lp[l]));
     // storage-order row and column forms + per-level chunk lists
+    const int64_t drops = C.ws.drops();
     {
         int32_t* cnt = W.get_t<int32_t>(nm("permcnt"), n + 1);
         auto build = [&](const int32_t* order, const int64_t* ptr, const int32_t* idx, const double* val, const char* tagp,
@@ -1877,8 +1879,8 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
             exclusive_scan_i32_to_i64(C, cnt, *pptr, n + 1, nullptr);
             *pidx = W.get_t<int32_t>(nm(tagp) + "_idx", out.nnz + 1);
             *pval = W.get_t<double>(nm(tagp) + "_val", out.nnz + 1);
-            *prow = W.get_t<FactorRow>(nm(tagp) + "_row", n);
-            *pent = W.get_t<FactorEnt<double>>(nm(tagp) + "_ent", out.nnz + 1);
+            *prow = W.get_optional_t<FactorRow>(nm(tagp) + "_row", n);
+            *pent = W.get_optional_t<FactorEnt<double>>(nm(tagp) + "_ent", out.nnz + 1);
             k_perm_copy<<<grid_for(n * 32, T256, 148 * 64), T256, 0, C.stream>>>(n, order, ptr, idx, val,
                                                                                 *pptr, *pidx, *pval, *prow, *pent);
             SSP_CHECK_LAUNCH();
@@ -1909,6 +1911,8 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
         build(out.level_cols, out.col_ptr, out.col_idx, out.col_val, "pcol", &out.pcol_ptr, &out.pcol_idx, &out.pcol_val,
               &out.bchunk, out.bchunk_lvl, out.hbptr, &out.brow, &out.bent);
     }
+    // (a buffer above may have cost the first form's copies)
+    out.ws_drops = drops;
     build_tail(C, out, T, T > 0 ? W.get_t<double>(nm("W"), (size_t)T * T) : nullptr, tag);
 }
 

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <stdlib.h>
 #include <string>
 #include <vector>
 #include <map>
@@ -87,6 +88,10 @@ __host__ __device__ __forceinline__ double edge_coin(uint64_t seed, int64_t e) {
 // from the device's default memory pool): a buffer that grows, or a workspace that is released, never waits
 // for the whole device the way cudaFree does, so contexts working side by side (the server's slots) do not
 // stall each other.  The context's stream is the only stream that touches these buffers.
+//
+// Optional buffers hold what a call can do without (copies laid out for a faster kernel): when the memory does not allow
+// one, the caller takes the way without it, and when it does not allow another buffer, the optional ones are given back
+// first.  SSP_WORKSPACE_LIMIT_MB=<megabytes> makes every context behave as on a device with that much room for it.
 class Workspace {
 public:
     ~Workspace() { release(); }
@@ -100,32 +105,49 @@ public:
             cudaFreeAsync(it->second.ptr, stream_);
             bufs_.erase(it);
         }
-        void* p = nullptr;
-        cudaError_t e = cudaMallocAsync(&p, bytes, stream_);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            throw Error(SSP_ERR_NOMEM, "device allocation of " + std::to_string(bytes) + " bytes for '" + name +
-                                           "' failed: " + cudaGetErrorString(e));
-        }
-        bufs_[name] = {p, bytes};
+        void* p = must_alloc(name, bytes, stream_);
+        bufs_[name] = {p, bytes, false};
         return p;
     }
     template <class T>
     T* get_t(const std::string& name, size_t count) { return (T*)get(name, count * sizeof(T)); }
+    // null when the memory does not allow it.  The pointer is good while drops() stays the same (KeepOptional).
+    template <class T>
+    T* get_optional_t(const std::string& name, size_t count) {
+        const size_t bytes = count * sizeof(T) ? count * sizeof(T) : 16;
+        auto it = bufs_.find(name);
+        if (it != bufs_.end() && it->second.bytes >= bytes) return (T*)it->second.ptr;
+        if (it != bufs_.end()) {
+            cudaFreeAsync(it->second.ptr, stream_);
+            bufs_.erase(it);
+        }
+        void* p = nullptr;
+        if (alloc(&p, bytes, stream_) != cudaSuccess) return nullptr;
+        bufs_[name] = {p, bytes, true};
+        return (T*)p;
+    }
+    // how often optional buffers have been given back
+    int64_t drops() const { return drops_; }
+    // while one exists, optional buffers stay: their pointers are in use
+    struct KeepOptional {
+        Workspace* w;
+        explicit KeepOptional(Workspace& ws) : w(&ws) { w->keep_++; }
+        KeepOptional(const KeepOptional&) = delete;
+        ~KeepOptional() { w->keep_--; }
+    };
+    // bytes left under SSP_WORKSPACE_LIMIT_MB
+    double room() const {
+        const char* e = getenv("SSP_WORKSPACE_LIMIT_MB");
+        return e && e[0] ? atof(e) * 1048576.0 - (double)total_bytes() : 1e300;
+    }
     // enlarge `name` to `bytes`, preserving its first `keep` bytes
     void* grow(const std::string& name, size_t keep, size_t bytes, cudaStream_t stream) {
         auto it = bufs_.find(name);
         if (it != bufs_.end() && it->second.bytes >= bytes) return it->second.ptr;
-        void* p = nullptr;
-        cudaError_t e = cudaMallocAsync(&p, bytes, stream);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            throw Error(SSP_ERR_NOMEM, "device allocation of " + std::to_string(bytes) + " bytes for '" + name +
-                                           "' failed: " + cudaGetErrorString(e));
-        }
+        void* p = must_alloc(name, bytes, stream);
         if (it != bufs_.end()) {
             if (keep) {
-                e = cudaMemcpyAsync(p, it->second.ptr, keep, cudaMemcpyDeviceToDevice, stream);
+                cudaError_t e = cudaMemcpyAsync(p, it->second.ptr, keep, cudaMemcpyDeviceToDevice, stream);
                 if (e != cudaSuccess) {
                     cudaFreeAsync(p, stream);
                     throw Error(SSP_ERR_CUDA, std::string("workspace grow copy: ") + cudaGetErrorString(e));
@@ -135,7 +157,7 @@ public:
             cudaFreeAsync(it->second.ptr, stream);
             bufs_.erase(it);
         }
-        bufs_[name] = {p, bytes};
+        bufs_[name] = {p, bytes, false};
         return p;
     }
     void release() {
@@ -154,9 +176,40 @@ public:
         return s;
     }
 private:
-    struct Buf { void* ptr; size_t bytes; };
+    struct Buf { void* ptr; size_t bytes; bool optional; };
     std::map<std::string, Buf> bufs_;
     cudaStream_t stream_ = nullptr;
+    int64_t drops_ = 0;
+    int keep_ = 0;
+    cudaError_t alloc(void** p, size_t bytes, cudaStream_t stream) {
+        if ((double)bytes > room()) return cudaErrorMemoryAllocation;
+        const cudaError_t e = cudaMallocAsync(p, bytes, stream);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e;
+    }
+    bool drop_optional() {
+        bool any = false;
+        for (auto it = bufs_.begin(); !keep_ && it != bufs_.end();) {
+            if (!it->second.optional) {
+                ++it;
+                continue;
+            }
+            cudaFreeAsync(it->second.ptr, stream_);
+            it = bufs_.erase(it);
+            any = true;
+        }
+        if (any) drops_++;
+        return any;
+    }
+    void* must_alloc(const std::string& name, size_t bytes, cudaStream_t stream) {
+        void* p = nullptr;
+        cudaError_t e = alloc(&p, bytes, stream);
+        if (e != cudaSuccess && drop_optional()) e = alloc(&p, bytes, stream);
+        if (e != cudaSuccess)
+            throw Error(SSP_ERR_NOMEM, "device allocation of " + std::to_string(bytes) + " bytes for '" + name +
+                                           "' failed: " + cudaGetErrorString(e));
+        return p;
+    }
 };
 
 // Launch shapes of the preconditioner's level launches (ssp_pcg.cu): per level and direction, the column width
@@ -403,7 +456,9 @@ struct DevFactor {
     int64_t* pcol_ptr = nullptr;
     int32_t* pcol_idx = nullptr;
     double* pcol_val = nullptr;
-    FactorRow* frow = nullptr;           // the same rows, entries and values for the walked levels of the solves
+    // the same rows, entries and values for the walked levels of the solves, and linv and tin_* below: optional
+    // (Workspace), good while extras() says so
+    FactorRow* frow = nullptr;
     FactorRow* brow = nullptr;
     FactorEnt<double>* fent = nullptr;
     FactorEnt<double>* bent = nullptr;
@@ -435,6 +490,8 @@ struct DevFactor {
     int64_t tin_nnz = 0;
     int32_t* tchunk = nullptr;
     int32_t ntchunk = 0;
+    int64_t ws_drops = -1;
+    bool extras(const Context& C) const { return ws_drops == C.ws.drops(); }
 };
 // the tail's inverse and split rows from the storage-order row form; X: scratch of T x T doubles
 void build_tail(Context& C, DevFactor& F, int64_t T, double* X, const std::string& tag);

@@ -24,6 +24,7 @@
 #include <cstdlib>
 
 #include <functional>
+#include <optional>
 
 #include "ssp_internal.cuh"
 
@@ -1377,11 +1378,12 @@ struct FactorVals {
     const T* prow_val;
     const T* pcol_val;
     const T* D;
-    const T* tin_val;  // the dense tail's entries in earlier levels, and its inverse
-    const T* linv;
-    T* tail_tmp;       // tail rows x ld scratch
-    const FactorEnt<T>* fent;  // the entries of both forms with their values beside them (walked levels)
-    const FactorEnt<T>* bent;
+    // null where the memory does not allow them:
+    const T* tin_val = nullptr;  // the dense tail's entries in earlier levels, and its inverse
+    const T* linv = nullptr;
+    T* tail_tmp = nullptr;       // tail rows x ld scratch
+    const FactorEnt<T>* fent = nullptr;  // the entries of both forms with their values beside them (walked levels)
+    const FactorEnt<T>* bent = nullptr;
 };
 
 // Column layouts of the triangular-solve launches.  A level launch gives each warp row a width of W columns
@@ -1474,10 +1476,12 @@ struct TrsvSeg {
     int32_t l0, l1;
     const WalkRound* rounds = nullptr;  // device; null: a launch of its own
     int32_t nrounds = 0;
+    size_t at = 0;                      // the first of them in the plan's list
 };
 struct TrsvPlan {
     std::vector<TrsvSeg> fw, bw;
     bool fuse_last = false;
+    bool tail = false;  // the dense tail as a product with its inverse; else its levels like the others
     WalkShape walk;
 };
 
@@ -1513,15 +1517,20 @@ static void launch_walk(Context& C, bool fwd, const TrsvPlan& P, const TrsvSeg& 
     launch(C, fwd, P, S, F, V, n, r, y, kcols, ra);
 }
 
-// The plan for a solve's columns; the rounds go to workspace buffers named after tag.
-static TrsvPlan make_trsv_plan(Context& C, const DevFactor& F, int ntiles, bool narrow, size_t elem,
+// The plan for a solve's columns; the rounds go to workspace buffers named after tag.  Without the copies of the factor's
+// entries no level is walked.
+template <class T>
+static TrsvPlan make_trsv_plan(Context& C, const DevFactor& F, const FactorVals<T>& V, int ntiles, bool narrow,
                                const std::string& tag) {
     TrsvPlan P;
-    const int32_t NL = F.tail_rows ? F.tail_l0 : F.num_levels;
+    constexpr size_t elem = sizeof(T);
+    P.tail = F.tail_rows && V.linv && V.tail_tmp;
+    const bool walks = V.fent && V.bent;
+    const int32_t NL = P.tail ? F.tail_l0 : F.num_levels;
     // the last level finished by its forward launch (M_FWD_LAST); SSP_PRECOND_FUSE_LAST=0 keeps the level's two
     // launches (the same values, bit for bit; for comparisons)
     const char* fuse_env = getenv("SSP_PRECOND_FUSE_LAST");
-    P.fuse_last = !(fuse_env && fuse_env[0] == '0') && F.tail_rows == 0 && F.num_levels > 0 && F.last_bwd_nnz == 0;
+    P.fuse_last = !(fuse_env && fuse_env[0] == '0') && !P.tail && F.num_levels > 0 && F.last_bwd_nnz == 0;
     const double cols = narrow ? NARROW_W : (double)ntiles * TILE;
     // The costs (us, bytes per us) that decide between a launch and a walk, fitted on B200 to the graphs above.  A
     // level's launch takes 13-18 us where it is small (five dependent loads per chunk, most blocks with one chunk) and
@@ -1556,7 +1565,7 @@ static TrsvPlan make_trsv_plan(Context& C, const DevFactor& F, int ntiles, bool 
         return c_launch + (E + 2 * R) * cols * elem / bw_launch;
     };
     // the factor's last level is a launch of its own (M_FWD_LAST when it can be)
-    const int32_t alone = F.tail_rows ? NL : NL - 1;
+    const int32_t alone = !walks ? 0 : P.tail ? NL : NL - 1;
     std::vector<WalkRound> tmp;
     double best = 0;
     for (int cl = 1; cl <= 8; cl *= 2) {
@@ -1594,7 +1603,7 @@ static TrsvPlan make_trsv_plan(Context& C, const DevFactor& F, int ntiles, bool 
             if (r - l >= 2 && g > 0) {
                 const size_t at = all.size();
                 for (int32_t i = 0; i < r - l; i++) level_rounds(ptr, P.walk, fwd ? l + i : r - 1 - i, all);
-                seg.push_back(TrsvSeg{l, r, (const WalkRound*)nullptr + at, (int32_t)(all.size() - at)});
+                seg.push_back(TrsvSeg{l, r, nullptr, (int32_t)(all.size() - at), at});
                 l = r;
             } else {
                 for (r = std::max(r, l + 1); l < r; l++) seg.push_back(TrsvSeg{l, l + 1});
@@ -1604,13 +1613,17 @@ static TrsvPlan make_trsv_plan(Context& C, const DevFactor& F, int ntiles, bool 
     };
     P.fw = plan(true);
     P.bw = plan(false);
-    WalkRound* d = C.ws.get_t<WalkRound>(tag + "_rounds", all.size() + 1);
-    if (!all.empty()) {
-        SSP_CUDA(cudaMemcpyAsync(d, all.data(), sizeof(WalkRound) * all.size(), cudaMemcpyHostToDevice, C.stream));
-        SSP_CUDA(cudaStreamSynchronize(C.stream));
+    if (all.empty()) return P;
+    WalkRound* d = C.ws.get_optional_t<WalkRound>(tag + "_rounds", all.size());
+    if (!d) {
+        FactorVals<T> launched = V;
+        launched.fent = nullptr;
+        return make_trsv_plan<T>(C, F, launched, ntiles, narrow, tag);
     }
+    SSP_CUDA(cudaMemcpyAsync(d, all.data(), sizeof(WalkRound) * all.size(), cudaMemcpyHostToDevice, C.stream));
+    SSP_CUDA(cudaStreamSynchronize(C.stream));
     for (auto* v : {&P.fw, &P.bw})
-        for (TrsvSeg& g : *v) g.rounds = g.nrounds ? d + (g.rounds - (const WalkRound*)nullptr) : nullptr;
+        for (TrsvSeg& g : *v) g.rounds = g.nrounds ? d + g.at : nullptr;
     return P;
 }
 
@@ -1662,7 +1675,7 @@ static int64_t launch_precond(Context& C, const DevFactor& F, const TrsvPlan& P,
         launch_walk<T>(C, true, P, s, F, V, n, r, y, kcols, ra);
         launches++;
     }
-    if (F.tail_rows) {
+    if (P.tail) {
         // the tail's rows less their entries in earlier levels (one launch, as a level), then its block
         const int code = width_code(true, F.tail_l0);
         const int ns = narrow ? 1 : TILE / trsv_width(code);
@@ -2076,14 +2089,15 @@ static void capture_precond(Context& C, Precond& P, int64_t& launches, const PcA
 }
 
 // The solve's preconditioner: its level shapes (forced, cached, the rule, or the rule until the solve's first
-// applications have measured them).  Its graph is captured by the first application that launches one (pcg_solve).  elem: bytes per value of the triangular solves.
-static void plan_precond(Context& C, const DevFactor& F, int64_t n, int64_t ld, int32_t kcols, size_t elem, Precond& P,
-                         PcgReport& rep, const RowAct& ra) {
+// applications have measured them).  Its graph is captured by the first application that launches one (pcg_solve).
+template <class T>
+static void plan_precond(Context& C, const DevFactor& F, const FactorVals<T>& V, int64_t n, int64_t ld, int32_t kcols,
+                         Precond& P, PcgReport& rep, const RowAct& ra) {
     TrsvShapes store;
     uint64_t key = 0;
     const bool narrow = TILE > NARROW_W && kcols <= NARROW_W;
-    const ShapeSource src = trsv_shape_source(C, F, n, ld, kcols, elem, ra.act != nullptr, store, key);
-    P.plan = make_trsv_plan(C, F, (int)(ld / TILE), narrow, elem, elem == sizeof(float) ? "pcg32" : "pcg");
+    const ShapeSource src = trsv_shape_source(C, F, n, ld, kcols, sizeof(T), ra.act != nullptr, store, key);
+    P.plan = make_trsv_plan<T>(C, F, V, (int)(ld / TILE), narrow, sizeof(T) == sizeof(float) ? "pcg32" : "pcg");
     P.measure = false;
     P.has_shapes = src == ShapeSource::Forced || src == ShapeSource::Cached;
     if (P.has_shapes) {
@@ -2102,34 +2116,61 @@ static void plan_precond(Context& C, const DevFactor& F, int64_t n, int64_t ld, 
 }
 
 static FactorVals<double> fp64_vals(Context& C, const DevFactor& F, int64_t ld) {
-    double* tmp = F.tail_rows ? C.ws.get_t<double>("pcg_tail", (size_t)F.tail_rows * ld) : nullptr;
-    return FactorVals<double>{F.prow_val, F.pcol_val, F.D, F.tin_val, F.linv, tmp, F.fent, F.bent};
+    FactorVals<double> V{F.prow_val, F.pcol_val, F.D};
+    if (F.extras(C) && F.tail_rows) {
+        V.tin_val = F.tin_val;
+        V.linv = F.linv;
+        V.tail_tmp = C.ws.get_optional_t<double>("pcg_tail", (size_t)F.tail_rows * ld);
+    }
+    if (F.extras(C) && F.frow && F.brow) {
+        V.fent = F.fent;
+        V.bent = F.bent;
+    }
+    return V;
 }
-// the factor's values rounded to FP32, in workspace buffers named after tag
-static FactorVals<float> fp32_vals(Context& C, const DevFactor& F, int64_t n, int64_t ld, const std::string& tag) {
-    const int64_t T = F.tail_rows;
-    const int64_t cnt[5] = {F.nnz, F.nnz, n, T ? F.tin_nnz : 0, T * T};
-    const double* src[5] = {F.prow_val, F.pcol_val, F.D, F.tin_val, F.linv};
-    float* f = C.ws.get_t<float>(tag + "_fval", 2 * F.nnz + n + cnt[3] + cnt[4] + 1);
-    int64_t at[5], o = 0;
-    for (int i = 0; i < 5; i++) {
-        at[i] = o;
-        o += cnt[i];
-        if (cnt[i] <= 0) continue;
-        k_d2f<<<grid_for(cnt[i], 256, 148 * 16), 256, 0, C.stream>>>(cnt[i], src[i], f + at[i]);
+// The factor's values rounded to FP32, in workspace buffers named after tag: the caller gets the first 2 nnz + n (f32_base)
+// before it needs the memory for anything optional.
+static float* f32_base(Context& C, const DevFactor& F, int64_t n, const std::string& tag) {
+    return C.ws.get_t<float>(tag + "_fval", 2 * F.nnz + n + 1);
+}
+static FactorVals<float> fp32_vals(Context& C, const DevFactor& F, int64_t n, int64_t ld, float* base,
+                                   const std::string& tag) {
+    auto put = [&](int64_t cnt, const double* src, float* dst) {
+        if (cnt <= 0) return;
+        k_d2f<<<grid_for(cnt, 256, 148 * 16), 256, 0, C.stream>>>(cnt, src, dst);
         SSP_CHECK_LAUNCH();
         C.kernels_launched++;
+    };
+    FactorVals<float> V{base, base + F.nnz, base + 2 * F.nnz};
+    put(F.nnz, F.prow_val, base);
+    put(F.nnz, F.pcol_val, base + F.nnz);
+    put(n, F.D, base + 2 * F.nnz);
+    if (F.extras(C) && F.tail_rows) {
+        const int64_t T = F.tail_rows;
+        float* f = C.ws.get_optional_t<float>(tag + "_ftail", F.tin_nnz + T * T + 1);
+        float* tmp = f ? C.ws.get_optional_t<float>(tag + "_tail", (size_t)T * ld) : nullptr;
+        if (tmp) {
+            put(F.tin_nnz, F.tin_val, f);
+            put(T * T, F.linv, f + F.tin_nnz);
+            V.tin_val = f;
+            V.linv = f + F.tin_nnz;
+            V.tail_tmp = tmp;
+        }
     }
-    float* tmp = T ? C.ws.get_t<float>(tag + "_tail", (size_t)T * ld) : nullptr;
-    FactorEnt<float>* e = C.ws.get_t<FactorEnt<float>>(tag + "_ent", 2 * F.nnz + 1);
-    if (F.nnz > 0) {
-        const int g = grid_for(F.nnz, 256, 148 * 16);
-        k_ent_f32<<<g, 256, 0, C.stream>>>(F.nnz, F.fent, e);
-        k_ent_f32<<<g, 256, 0, C.stream>>>(F.nnz, F.bent, e + F.nnz);
-        SSP_CHECK_LAUNCH();
-        C.kernels_launched += 2;
+    const bool ents = F.extras(C) && F.frow && F.brow && F.fent && F.bent;
+    FactorEnt<float>* e = ents ? C.ws.get_optional_t<FactorEnt<float>>(tag + "_ent", 2 * F.nnz + 1) : nullptr;
+    if (e) {
+        if (F.nnz > 0) {
+            const int g = grid_for(F.nnz, 256, 148 * 16);
+            k_ent_f32<<<g, 256, 0, C.stream>>>(F.nnz, F.fent, e);
+            k_ent_f32<<<g, 256, 0, C.stream>>>(F.nnz, F.bent, e + F.nnz);
+            SSP_CHECK_LAUNCH();
+            C.kernels_launched += 2;
+        }
+        V.fent = e;
+        V.bent = e + F.nnz;
     }
-    return FactorVals<float>{f + at[0], f + at[1], f + at[2], f + at[3], f + at[4], tmp, e, e + F.nnz};
+    return V;
 }
 
 // apply M^{-1} to R into Z once (tile-major n x ld blocks; stage entry point).  When the shapes are to be
@@ -2138,8 +2179,9 @@ void precond_apply_device(Context& C, const DevFactor& F, const double* R, doubl
     TrsvShapes store;
     uint64_t key = 0;
     const ShapeSource src = trsv_shape_source(C, F, F.n, ld, (int32_t)ld, sizeof(double), false, store, key);
-    const TrsvPlan P = make_trsv_plan(C, F, (int)(ld / TILE), TILE > NARROW_W && ld <= NARROW_W, sizeof(double), "pcg");
     const FactorVals<double> V = fp64_vals(C, F, ld);
+    const Workspace::KeepOptional keep(C.ws);
+    const TrsvPlan P = make_trsv_plan<double>(C, F, V, (int)(ld / TILE), TILE > NARROW_W && ld <= NARROW_W, "pcg");
     const TrsvShapes* sh = nullptr;
     if (src == ShapeSource::Forced || src == ShapeSource::Cached) {
         sh = &store;
@@ -2504,10 +2546,12 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
         int64_t pc_launches = 0;
         if (read_i64(C, S.nactive) > 0) {
             PcApply pc;
-            size_t elem = sizeof(double);
+            std::optional<Workspace::KeepOptional> keep;
             if (opt.precision == SSP_PRECISION_PC32 && !(TILE > NARROW_W && k <= NARROW_W)) {
                 // FP64 PCG with the triangular solves in FP32: r rounded on the way in, z widened on the way out
-                const FactorVals<float> V32 = fp32_vals(C, F, n, ld, "pcgp");
+                float* base = f32_base(C, F, n, "pcgp");
+                const FactorVals<float> V32 = fp32_vals(C, F, n, ld, base, "pcgp");
+                keep.emplace(W);
                 // r32 and z32 live in q's memory: q (= A p) is dead from the r update to the next Laplacian
                 // product, and the preconditioner runs in between, so this mode needs no more memory than FP64
                 float* r32 = reinterpret_cast<float*>(q);
@@ -2520,15 +2564,16 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
                     SSP_CHECK_LAUNCH();
                     return l + 2;
                 };
-                elem = sizeof(float);
+                plan_precond<float>(C, F, V32, n, ld, k, P, rep, ra);
             } else {
                 // (its scratch is allocated here: the applications are captured into graphs)
                 const FactorVals<double> V64 = fp64_vals(C, F, ld);
+                keep.emplace(W);
                 pc = [&C, &F, &P, V64, n, r, z, ld, k, ra](const TrsvShapes* sh, LevelEvents* lev) {
                     return launch_precond<double>(C, F, P.plan, V64, n, r, z, ld, k, ra, sh, lev);
                 };
+                plan_precond<double>(C, F, V64, n, ld, k, P, rep, ra);
             }
-            plan_precond(C, F, n, ld, k, elem, P, rep, ra);
             it = pcg_solve<double>(C, n, k, ld, A, A.val, F, pc, P, pc_launches,
                                    PcgBufs<double>{x, r, z, p, q}, S, R, opt.max_iters, opt, tm, rep, ra);
         }
@@ -2542,7 +2587,7 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
             C.kernels_launched++;
         };
         to_f32(lap_nnz, A.val, aval32);
-        const FactorVals<float> V32 = fp32_vals(C, F, n, ld, "pcgm");
+        float* base32 = f32_base(C, F, n, "pcgm");
         float* e32 = W.get_t<float>("pcgm_e", total);
         float* r32 = W.get_t<float>("pcgm_r", total);
         float* z32 = W.get_t<float>("pcgm_z", total);
@@ -2550,6 +2595,9 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
         float* q32 = W.get_t<float>("pcgm_q", total);
         ColState Si = make_colstate(C, ns, "pcgm_in");
         double* worst = W.get_t<double>("pcgm_worst", 1);
+        const FactorVals<float> V32 = fp32_vals(C, F, n, ld, base32, "pcgm");
+        FactorVals<double> V64{};  // once a round falls back
+        std::optional<Workspace::KeepOptional> keep(std::in_place, W);
         double* e64 = nullptr;  // FP64 inner increment, only if a round falls back
         Precond P32, P64;
         int64_t pc32 = 0, pc64 = 0;
@@ -2571,7 +2619,7 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
                                                                                    LevelEvents* lev) {
                     return launch_precond<float>(C, F, P32.plan, V32, n, r32, z32, ld, k, ra, sh, lev);
                 };
-                if (!P32.planned) plan_precond(C, F, n, ld, k, sizeof(float), P32, rep, ra);
+                if (!P32.planned) plan_precond<float>(C, F, V32, n, ld, k, P32, rep, ra);
                 int32_t cap = opt.max_iters - it;
                 if (first_its >= 0)
                     cap = std::min(cap, std::max(MIXED_MIN_ROUND_ITERS, MIXED_ROUND_ITER_FACTOR * first_its));
@@ -2583,7 +2631,12 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
                 hit_cap = its >= cap;
                 k_add_into<float><<<grid_for(total, 256, 148 * 16), 256, 0, C.stream>>>(total, e32, x);
             } else {
-                if (!e64) e64 = W.get_t<double>("pcgm_e64", total);
+                if (!e64) {
+                    keep.reset();  // no FP32 round follows, so what they used may go
+                    e64 = W.get_t<double>("pcgm_e64", total);
+                    V64 = fp64_vals(C, F, ld);
+                    keep.emplace(W);
+                }
                 // the FP64 inner solve runs in place on the residual of the active columns and goes straight
                 // to (half) the outer threshold
                 k_rhs_masked<double><<<egrid, 256, 0, C.stream>>>(n, ld, r, S.active, r, R.G);
@@ -2592,11 +2645,10 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
                 k_cols_init_inner<<<cg, 256, 0, C.stream>>>(ld, k, 0.0, S.thr, Si, R.G);
                 SSP_CHECK_LAUNCH();
                 C.kernels_launched += 2;
-                const FactorVals<double> V64 = fp64_vals(C, F, ld);
                 const PcApply pc64f = [&C, &F, &P64, V64, n, r, z, ld, k, ra](const TrsvShapes* sh, LevelEvents* lev) {
                     return launch_precond<double>(C, F, P64.plan, V64, n, r, z, ld, k, ra, sh, lev);
                 };
-                if (!P64.planned) plan_precond(C, F, n, ld, k, sizeof(double), P64, rep, ra);
+                if (!P64.planned) plan_precond<double>(C, F, V64, n, ld, k, P64, rep, ra);
                 its = pcg_solve<double>(C, n, k, ld, A, A.val, F, pc64f, P64, pc64,
                                         PcgBufs<double>{e64, r, z, p, q}, Si, R, opt.max_iters - it, opt, tm, rep,
                                         ra);

@@ -205,9 +205,12 @@ void build_tail(Context& C, DevFactor& F, int64_t T, double* X, const std::strin
     Workspace& W = C.ws;
     const int64_t r0 = F.n - T;
     F.tail_l0 = F.num_levels - (int32_t)T;
-    double* M = W.get_t<double>(tag + "_linv", (size_t)T * T);
-    int32_t* cnt = W.get_t<int32_t>(tag + "_tincnt", T + 1);
-    F.tin_ptr = W.get_t<int64_t>(tag + "_tinptr", T + 1);
+    // Without the memory for it there is no dense tail: its levels are solved like the others.
+    const Workspace::KeepOptional keep(W);
+    double* M = W.get_optional_t<double>(tag + "_linv", (size_t)T * T);
+    int32_t* cnt = W.get_optional_t<int32_t>(tag + "_tincnt", T + 1);
+    F.tin_ptr = W.get_optional_t<int64_t>(tag + "_tinptr", T + 1);
+    if (!M || !cnt || !F.tin_ptr) return;
     SSP_CUDA(cudaMemsetAsync(M, 0, sizeof(double) * T * T, C.stream));
     SSP_CUDA(cudaMemsetAsync(cnt + T, 0, sizeof(int32_t), C.stream));
     const unsigned wb = (unsigned)ceil_div<int64_t>(T * 32, 256);
@@ -218,8 +221,9 @@ void build_tail(Context& C, DevFactor& F, int64_t T, double* X, const std::strin
     SSP_CUDA(cudaMemcpyAsync(hp.data(), F.tin_ptr, sizeof(int64_t) * (T + 1), cudaMemcpyDeviceToHost, C.stream));
     SSP_CUDA(cudaStreamSynchronize(C.stream));
     F.tin_nnz = hp[T];
-    F.tin_idx = W.get_t<int32_t>(tag + "_tinidx", F.tin_nnz + 1);
-    F.tin_val = W.get_t<double>(tag + "_tinval", F.tin_nnz + 1);
+    F.tin_idx = W.get_optional_t<int32_t>(tag + "_tinidx", F.tin_nnz + 1);
+    F.tin_val = W.get_optional_t<double>(tag + "_tinval", F.tin_nnz + 1);
+    if (!F.tin_idx || !F.tin_val) return;
     k_tail_split<<<wb, 256, 0, C.stream>>>((int32_t)T, F.prow_ptr + r0, F.prow_idx, F.prow_val, F.level, F.tail_l0,
                                            F.tin_ptr, F.tin_idx, F.tin_val, M);
     k_tail_diag<<<(unsigned)ceil_div<int64_t>(T, TB), 32, 0, C.stream>>>((int32_t)T, M);
@@ -237,7 +241,8 @@ void build_tail(Context& C, DevFactor& F, int64_t T, double* X, const std::strin
     make_chunks(hp.data(), 0, (int32_t)T, ch);
     F.ntchunk = (int32_t)ch.size();
     ch.push_back((int32_t)T);
-    F.tchunk = W.get_t<int32_t>(tag + "_tinchunk", ch.size());
+    F.tchunk = W.get_optional_t<int32_t>(tag + "_tinchunk", ch.size());
+    if (!F.tchunk) return;
     SSP_CUDA(cudaMemcpyAsync(F.tchunk, ch.data(), sizeof(int32_t) * ch.size(), cudaMemcpyHostToDevice, C.stream));
     SSP_CUDA(cudaStreamSynchronize(C.stream));
     F.linv = M;
