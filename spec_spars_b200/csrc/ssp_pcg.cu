@@ -1525,7 +1525,13 @@ static TrsvPlan make_trsv_plan(Context& C, const DevFactor& F, const FactorVals<
     TrsvPlan P;
     constexpr size_t elem = sizeof(T);
     P.tail = F.tail_rows && V.linv && V.tail_tmp;
-    const bool walks = V.fent && V.bent;
+    // SSP_TRSV_WALK=0 launches every level, =1 walks every one that can be; SSP_TRSV_CLUSTER=1|2|4|8 sets the blocks of a
+    // cluster (as far as they are resident at once).  For comparisons.
+    const char* walk_env = getenv("SSP_TRSV_WALK");
+    const char* cl_env = getenv("SSP_TRSV_CLUSTER");
+    const bool walk_all = walk_env && walk_env[0] == '1';
+    const int set_cl = cl_env ? atoi(cl_env) : 0;
+    const bool walks = V.fent && V.bent && !(walk_env && walk_env[0] == '0');
     const int32_t NL = P.tail ? F.tail_l0 : F.num_levels;
     // the last level finished by its forward launch (M_FWD_LAST); SSP_PRECOND_FUSE_LAST=0 keeps the level's two
     // launches (the same values, bit for bit; for comparisons)
@@ -1570,7 +1576,7 @@ static TrsvPlan make_trsv_plan(Context& C, const DevFactor& F, const FactorVals<
     double best = 0;
     for (int cl = 1; cl <= 8; cl *= 2) {
         const WalkShape w = walk_shape(ntiles, narrow, cl);
-        if (cl > 1 && w.blocks > 128) break;
+        if (cl > 1 && (w.blocks > 128 || (set_cl && cl > set_cl))) break;
         double us = 0;
         for (int32_t l = 0; l < alone; l++)
             for (const auto* ptr : {&F.hfptr, &F.hbptr}) {
@@ -1578,7 +1584,7 @@ static TrsvPlan make_trsv_plan(Context& C, const DevFactor& F, const FactorVals<
                 level_rounds(*ptr, w, l, tmp);
                 us += std::min(launch_us(*ptr, l), walk_us(*ptr, w, l, tmp.size()));
             }
-        if (cl == 1 || us < best) {
+        if (cl == 1 || us < best || set_cl) {
             best = us;
             P.walk = w;
         }
@@ -1593,7 +1599,7 @@ static TrsvPlan make_trsv_plan(Context& C, const DevFactor& F, const FactorVals<
             tmp.clear();
             level_rounds(ptr, P.walk, l, tmp);
             cnt[l] = tmp.size();
-            gain[l] = launch_us(ptr, l) - walk_us(ptr, P.walk, l, tmp.size());
+            gain[l] = walk_all ? c_launch : launch_us(ptr, l) - walk_us(ptr, P.walk, l, tmp.size());
         }
         for (int32_t l = 0; l < NL;) {
             int32_t r = l;
@@ -2092,7 +2098,7 @@ static void capture_precond(Context& C, Precond& P, int64_t& launches, const PcA
 // applications have measured them).  Its graph is captured by the first application that launches one (pcg_solve).
 template <class T>
 static void plan_precond(Context& C, const DevFactor& F, const FactorVals<T>& V, int64_t n, int64_t ld, int32_t kcols,
-                         Precond& P, PcgReport& rep, const RowAct& ra) {
+                         Precond& P, PcgReport& rep, const RowAct& ra, int verbose) {
     TrsvShapes store;
     uint64_t key = 0;
     const bool narrow = TILE > NARROW_W && kcols <= NARROW_W;
@@ -2110,6 +2116,15 @@ static void plan_precond(Context& C, const DevFactor& F, const FactorVals<T>& V,
             P.key = key;
             P.mstep = 0;
         }
+    }
+    if (verbose) {
+        int32_t walked = 0, launched = 0;
+        for (const auto* v : {&P.plan.fw, &P.plan.bw})
+            for (const TrsvSeg& g : *v) (g.rounds ? walked : launched) += g.l1 - g.l0;
+        const WalkShape& w = P.plan.walk;
+        fprintf(stderr, "[ssp] triangular solves%s: %d levels walked (%d columns, %d threads, clusters of %d), %d launched, "
+                "dense tail of %d\n", sizeof(T) == 4 ? " (fp32)" : "", walked, w.W, w.NT, w.cl, launched,
+                P.plan.tail ? F.tail_rows : 0);
     }
     P.planned = true;
     P.drop_graph();
@@ -2564,7 +2579,7 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
                     SSP_CHECK_LAUNCH();
                     return l + 2;
                 };
-                plan_precond<float>(C, F, V32, n, ld, k, P, rep, ra);
+                plan_precond<float>(C, F, V32, n, ld, k, P, rep, ra, opt.verbose);
             } else {
                 // (its scratch is allocated here: the applications are captured into graphs)
                 const FactorVals<double> V64 = fp64_vals(C, F, ld);
@@ -2572,7 +2587,7 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
                 pc = [&C, &F, &P, V64, n, r, z, ld, k, ra](const TrsvShapes* sh, LevelEvents* lev) {
                     return launch_precond<double>(C, F, P.plan, V64, n, r, z, ld, k, ra, sh, lev);
                 };
-                plan_precond<double>(C, F, V64, n, ld, k, P, rep, ra);
+                plan_precond<double>(C, F, V64, n, ld, k, P, rep, ra, opt.verbose);
             }
             it = pcg_solve<double>(C, n, k, ld, A, A.val, F, pc, P, pc_launches,
                                    PcgBufs<double>{x, r, z, p, q}, S, R, opt.max_iters, opt, tm, rep, ra);
@@ -2619,7 +2634,7 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
                                                                                    LevelEvents* lev) {
                     return launch_precond<float>(C, F, P32.plan, V32, n, r32, z32, ld, k, ra, sh, lev);
                 };
-                if (!P32.planned) plan_precond<float>(C, F, V32, n, ld, k, P32, rep, ra);
+                if (!P32.planned) plan_precond<float>(C, F, V32, n, ld, k, P32, rep, ra, opt.verbose);
                 int32_t cap = opt.max_iters - it;
                 if (first_its >= 0)
                     cap = std::min(cap, std::max(MIXED_MIN_ROUND_ITERS, MIXED_ROUND_ITER_FACTOR * first_its));
@@ -2648,7 +2663,7 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
                 const PcApply pc64f = [&C, &F, &P64, V64, n, r, z, ld, k, ra](const TrsvShapes* sh, LevelEvents* lev) {
                     return launch_precond<double>(C, F, P64.plan, V64, n, r, z, ld, k, ra, sh, lev);
                 };
-                if (!P64.planned) plan_precond<double>(C, F, V64, n, ld, k, P64, rep, ra);
+                if (!P64.planned) plan_precond<double>(C, F, V64, n, ld, k, P64, rep, ra, opt.verbose);
                 its = pcg_solve<double>(C, n, k, ld, A, A.val, F, pc64f, P64, pc64,
                                         PcgBufs<double>{e64, r, z, p, q}, Si, R, opt.max_iters - it, opt, tm, rep,
                                         ra);
