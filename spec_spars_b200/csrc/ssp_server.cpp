@@ -111,18 +111,64 @@ bool same_batch(const ssp_params& a, const ssp_params& b) {
            a.reweight == b.reweight && batchable(a) && batchable(b);
 }
 
+// Device memory of a run over n vertices, nnz stored entries and ld columns, segs of its Laplacian's rows' segments
+// (a row of more than 256 entries is summed in segments of 256).  A request is refused by what it needs at least, and
+// admitted beside others by all that a context holds after one.
+struct Footprint {
+    int64_t needed;
+    int64_t besides;
+    int64_t total() const { return needed + besides; }
+};
+Footprint footprint(int64_t n, int64_t nnz, int64_t ld, int64_t segs, const ssp_params& p) {
+    // n x ld blocks: sketch + x, r, z, p, q in FP64 (+ five FP32 blocks and an FP64 increment when mixed), and the segments'
+    // sums, half a block at most; graph, Laplacian, factor pools and sampling arrays per stored entry; a fixed allowance
+    const bool mixed = p.precision == SSP_PRECISION_MIXED;
+    const double blocks = mixed ? 6.0 + 2.5 + 1.0 : 6.0;
+    const int64_t sums = std::max(std::min(8 * segs * ld, 4 * n * ld), 8 * segs * 32);
+    Footprint f;
+    f.needed = (int64_t)(blocks * 8.0 * (double)n * (double)ld) + 200 * nnz + 96 * n + sums + (16ll << 20);
+    // Contexts held 250 to 310 bytes an entry after light factors of ER, R-MAT and dense graphs, and 370 with the copies of
+    // the factor's entries where it has nearly as many as the graph; FP32 copies when the solves are; the inverse of the dense
+    // tail of a complete factor, and its columns.
+    const bool f32 = p.precision != SSP_PRECISION_FP64;
+    const int64_t T = p.factor_max_degree <= 0 ? std::min<int64_t>(n, std::max<int64_t>(0, p.dense_threshold)) : 0;
+    f.besides = 180 * nnz + 32 * n + 8 * T * T + 8 * T * ld + (f32 ? 25 * nnz + 4 * T * T : 0);
+    return f;
+}
+int64_t row_segments(const int64_t* colptr, int64_t n) {
+    int64_t s = 0;
+    for (int64_t v = 0; v < n; v++) {
+        const int64_t len = colptr[v + 1] - colptr[v] + 1;  // with the diagonal
+        if (len > 256) s += (len + 255) / 256;
+    }
+    return s;
+}
+Footprint request_footprint(const ssp_csc& g, const ssp_params& p) {
+    const int64_t n = g.n, nnz = g.nnz;
+    const int64_t k = ssp_params_jl_dim(&p, n);
+    const int64_t segs = g.mem == SSP_MEM_HOST && g.colptr ? row_segments(g.colptr, n) : nnz / 256 + std::min(n, nnz / 256);
+    Footprint f = footprint(n, nnz, (k + 31) / 32 * 32, segs, p);
+    // the SpMM's column-slab copy of the Laplacian when slabs are on and the graph has more rows than one slab holds
+    // (256-byte rows, at most 16 slabs)
+    const int64_t slab_rows = std::max<int64_t>(1, (int64_t)(ssp::spmm_slab_mb() * 1048576.0 / 256));
+    const int64_t slabs = ssp::spmm_slab_mb() > 0 && n > slab_rows
+                              ? std::min<int64_t>(16, (n + slab_rows - 1) / slab_rows) : 0;
+    f.needed += slabs ? 12 * (nnz + n) + 12 * slabs * n : 0;
+    return f;
+}
+
 // device footprint of a batch: its union's n x ld blocks use the largest k of the batch for every row
 int64_t batch_footprint(const std::vector<Job*>& js) {
     if (js.size() == 1) return js[0]->est_bytes;
-    int64_t ld = 0, n = 0, nnz = 0;
+    int64_t ld = 0, n = 0, nnz = 0, segs = 0;
     for (const Job* j : js) {
         const int64_t k = ssp_params_jl_dim(&j->params, j->n);
         ld = std::max<int64_t>(ld, (k + 31) / 32 * 32);
         n += j->n;
         nnz += (int64_t)j->values.size();
+        segs += row_segments(j->colptr.data(), j->n);
     }
-    const double blocks = js[0]->params.precision == SSP_PRECISION_MIXED ? 6.0 + 2.5 + 1.0 : 6.0;
-    return (int64_t)(blocks * 8.0 * (double)n * (double)ld) + 200 * nnz + 96 * n + (16ll << 20);
+    return footprint(n, nnz, ld, segs, js[0]->params).total();
 }
 
 }  // namespace
@@ -317,19 +363,7 @@ void ssp_server_opts_default(ssp_server_opts* o) {
 
 int64_t ssp_request_footprint(const ssp_csc* graph, const ssp_params* params) {
     if (!graph || !params || graph->n <= 0) return -1;
-    const int64_t n = graph->n, nnz = graph->nnz;
-    const int64_t k = ssp_params_jl_dim(params, n);
-    const int64_t ld = (k + 31) / 32 * 32;  // whole 32-column tiles
-    // n x ld blocks: sketch + x, r, z, p, q in FP64 (+ five FP32 blocks and an FP64 increment when mixed);
-    // graph, Laplacian, factor pools and sampling arrays per stored entry; the SpMM's column-slab copy of
-    // the Laplacian when slabs are on and the graph has more rows than one slab holds (256-byte rows, at
-    // most 16 slabs); a fixed allowance
-    const double blocks = params->precision == SSP_PRECISION_MIXED ? 6.0 + 2.5 + 1.0 : 6.0;
-    const int64_t slab_rows = std::max<int64_t>(1, (int64_t)(ssp::spmm_slab_mb() * 1048576.0 / 256));
-    const int64_t slabs = ssp::spmm_slab_mb() > 0 && n > slab_rows
-                              ? std::min<int64_t>(16, (n + slab_rows - 1) / slab_rows) : 0;
-    const int64_t slab_bytes = slabs ? 12 * (nnz + n) + 12 * slabs * n : 0;
-    return (int64_t)(blocks * 8.0 * (double)n * (double)ld) + 200 * nnz + 96 * n + slab_bytes + (16ll << 20);
+    return request_footprint(*graph, *params).total();
 }
 
 int ssp_server_create(const ssp_server_opts* opts, ssp_server** out) {
@@ -377,7 +411,7 @@ int ssp_submit(ssp_server* s, const ssp_request* req, uint64_t* ticket) {
     if (g.mem != SSP_MEM_HOST || g.n <= 0 || g.nnz < 0 || !g.colptr || (g.nnz > 0 && (!g.rowidx || !g.values)) ||
         g.colptr[0] != 0 || g.colptr[g.n] != g.nnz)
         return fail(SSP_ERR_INVALID, "ssp_submit: the graph must be a valid host CSC");
-    const int64_t est = ssp_request_footprint(&g, &req->params);
+    const Footprint fp = request_footprint(g, req->params);
     std::unique_ptr<Job> j(new Job());
     j->n = g.n;
     j->colptr.assign(g.colptr, g.colptr + g.n + 1);
@@ -386,12 +420,12 @@ int ssp_submit(ssp_server* s, const ssp_request* req, uint64_t* ticket) {
     j->params = req->params;
     j->check_probes = req->check_probes;
     j->output_file = req->params.output_file ? req->params.output_file : "";
-    j->est_bytes = est;
+    j->est_bytes = fp.total();
     std::lock_guard<std::mutex> lk(s->mu);
     if (s->stopping) return fail(SSP_ERR_INVALID, "ssp_submit: server is shutting down");
-    if (est > s->opts.hbm_budget_bytes) {
+    if (fp.needed > s->opts.hbm_budget_bytes) {
         s->rejected++;
-        return fail(SSP_ERR_CAPACITY, "ssp_submit: estimated footprint " + std::to_string(est) +
+        return fail(SSP_ERR_CAPACITY, "ssp_submit: estimated footprint " + std::to_string(fp.needed) +
                                           " bytes exceeds the HBM budget " + std::to_string(s->opts.hbm_budget_bytes));
     }
     if (s->opts.max_pending > 0 && (int64_t)s->pending.size() >= s->opts.max_pending) {
