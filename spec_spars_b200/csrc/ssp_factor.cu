@@ -976,12 +976,10 @@ __global__ void k_dense_build(FDev F, const int32_t* rem, int32_t T, const int32
     }
 }
 
-  // entries; counting is quadratic
-
 // Single block: eliminate the T remaining vertices in key order.  A chain of T columns, so what counts is the latency
 // of one: the row's nonzeros are collected in any order (their keys are unique), ranked, scanned in 32-wide chunks
 // whose carries every thread adds up for itself, and each fill goes out as two fire-and-forget additions (a pair of
-// rows gets at most one fill per column, so the sums are the same in every run) -- five barriers a column.  On B200 the
+// rows gets at most one fill per column, so the sums are the same in every run) -- six barriers a column.  On B200 the
 // tails of 1852 vertices (geometric graph, n = 30,011), 1112 (3-D grid, n = 64,000) and 1007 (n = 80,840) take 7.6, 3.5 and
 // 1.9 ms; with an ordered compaction, a bitonic sort and read-modify-write fills they took 23.3, 11.0 and 5.8.  Columns
 // longer than RANK_SORT_MAX are still sorted by the network.
@@ -1475,15 +1473,17 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
         for (int32_t g = 0; g < nseg; g++)
             for (int64_t v = opt.seg_row0[g]; v < opt.seg_row0[g + 1]; v++) g_live[g] += hdeg[v];
     }
-    // D of the R vertices rem (their live bags hold at most cap entries): warps, then blocks for the larger bags, whose
+    // D of the R vertices rem (their bags hold at most maxlen entries): warps, then blocks for the larger bags, whose
     // list's length stays on the device
-    auto trunc_diag = [&](const int32_t* rem, int64_t R, int32_t at, int32_t cap) {
+    auto trunc_diag = [&](const int32_t* rem, int64_t R, int32_t at, int32_t maxlen) {
         int32_t* big = list_b;  // (a level's lists are made after its truncations)
         SSP_CUDA(cudaMemsetAsync(F.ctr + C_NB, 0, sizeof(int64_t), C.stream));
         k_trunc_diag_warp<<<grid_for(R * 32, T256, 148 * 64), T256, 0, C.stream>>>(F, rem, (int32_t)R, big);
         SSP_CHECK_LAUNCH();
         C.kernels_launched++;
-        if (cap <= 32) return;
+        if (maxlen <= 32) return;
+        int32_t cap = 64;
+        while (cap < maxlen) cap <<= 1;
         if (cap <= BLOCK_TIER_MAX) {
             size_t smem = (size_t)cap * (2 * sizeof(double) + 2 * sizeof(int32_t));
             allow_dynamic_smem(C, k_trunc_diag, smem);
@@ -1506,13 +1506,10 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
         SSP_CHECK_LAUNCH();
         const int64_t R = read_i64(C, F.ctr + C_REM);
         if (R == 0) return 0;
-        const int32_t maxlen = device_max_i32(C, F.bag_len + v0, v1 - v0);
-        int32_t cap = 64;
-        while (cap < maxlen) cap <<= 1;
-        trunc_diag(rem, R, at, cap);
+        trunc_diag(rem, R, at, device_max_i32(C, F.bag_len + v0, v1 - v0));
         k_set_level<<<grid_for(R, T256), T256, 0, C.stream>>>(rem, (int32_t)R, at, F.level);
         SSP_CHECK_LAUNCH();
-        C.kernels_launched += 3;
+        C.kernels_launched += 2;
         int64_t hh[C_NCTR];
         read_i64s(C, F.ctr, hh, C_NCTR);
         if (hh[C_ERR]) throw Error(SSP_ERR_CAPACITY, "factor: truncation overflow");
@@ -1728,13 +1725,10 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
         int32_t* rem = W.get_t<int32_t>(nm("rem"), R + 1);
         SSP_CUDA(cudaMemsetAsync(F.ctr + C_REM, 0, sizeof(int64_t), C.stream));
         k_collect_live<<<grid_for(n, T256), T256, 0, C.stream>>>(n, F.level, rem, F.ctr + C_REM);
-        const int32_t maxlen = device_max_i32(C, F.bag_len, n);
-        int32_t cap = 64;
-        while (cap < maxlen) cap <<= 1;
-        trunc_diag(rem, R, lvl, cap);
+        trunc_diag(rem, R, lvl, device_max_i32(C, F.bag_len, n));
         k_set_level<<<grid_for(R, T256), T256, 0, C.stream>>>(rem, (int32_t)R, lvl, F.level);
         SSP_CHECK_LAUNCH();
-        C.kernels_launched += 3;
+        C.kernels_launched += 2;
         int64_t hh[C_NCTR];
         read_i64s(C, F.ctr, hh, C_NCTR);
         if (hh[C_ERR]) throw Error(SSP_ERR_CAPACITY, "factor: truncation overflow");
@@ -1786,7 +1780,7 @@ void factor_device(Context& C, int64_t n, const int64_t* colptr, const int32_t* 
         allow_dynamic_smem(C, k_dense_elim, smem);
         k_dense_elim<<<1, 1024, smem, C.stream>>>(F, rem, (int32_t)T, P, idx, Wd, Lused, sparse_levels);
         SSP_CHECK_LAUNCH();
-        C.kernels_launched += 5;
+        C.kernels_launched += 4;
         Lused += T * (T - 1) / 2;
         int64_t hh[C_NCTR];
         read_i64s(C, F.ctr, hh, C_NCTR);
