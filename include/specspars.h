@@ -154,7 +154,7 @@ typedef struct {
     int32_t trsv_shapes;            /* SSP_TRSV_*: how the preconditioner's level-launch shapes were chosen */
     int32_t trsv_levels_w8;         /* level launches (forward + backward) at 8 columns per warp row, */
     int32_t trsv_levels_w16;        /* ... at 16, */
-    int32_t trsv_levels_w32;        /* ... at 32 (runs of thin levels are not counted: always 8) */
+    int32_t trsv_levels_w32;        /* ... at 32 (levels walked inside one launch are not counted) */
     double ms_trsv_tune;            /* device time of the applications that measured them (real
                                        applications of the solve; 0 when taken from the cache) */
 } ssp_stats;

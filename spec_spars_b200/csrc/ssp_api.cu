@@ -217,7 +217,8 @@ struct HostOutBuffers {
 constexpr int64_t HOST_OUT_PREFAULT_MIN = 1 << 20;  // entries; smaller outputs allocate at the end
 
 // Columns solved per pass.  The PCG holds six n x ld FP64 blocks (sketch, x, r, z, p, q; the mixed mode adds
-// five FP32 blocks and an FP64 increment; rows of more than CHUNK_CAP entries add up to half a block of partial sums), which for the R-MAT configuration (scale 22, eps 0.3: k = 3917)
+// five FP32 blocks and an FP64 increment; rows of more than CHUNK_CAP entries add up to half a block of partial
+// sums), which for the R-MAT configuration (scale 22, eps 0.3: k = 3917)
 // need 450 GB.  The columns are independent once the factor exists, so they are solved in batches of whole
 // 32-column tiles.  Whether to batch is decided before the factorization with room set aside for it (70 % of
 // the free memory, less 40 B per Laplacian entry and 48 B per edge); the batch size after it, from the memory

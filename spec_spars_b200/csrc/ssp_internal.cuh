@@ -214,7 +214,8 @@ private:
 
 // Launch shapes of the preconditioner's level launches (ssp_pcg.cu): per level and direction, the column width
 // of a warp's row -- code 0, 1, 2 for 8, 16, 32 columns, TILE / width blocks per column tile.  Every width gives
-// the same values bit for bit, so a shape changes only the time.  Chosen by measurement per factor and kept in
+// the same values bit for bit, so a shape changes only the time.  (Which levels are launched at all, and not walked, follows
+// from the solve's columns; walked levels add a row up in another order.)  Chosen by measurement per factor and kept in
 // the context under a signature of the factor's level structure and the solve's shape.
 struct TrsvShapes {
     std::vector<uint8_t> fw, bw;  // per level

@@ -673,8 +673,9 @@ struct LoopGraph {
 // one longer row).  Each warp owns whole chunks: it stages the chunk's (index, value) pairs in its own
 // shared-memory slice with coalesced streaming loads (the matrix is read once per tile and should not
 // evict the gathered slab from L2), then every (row, column) lane pair sums its row with independent
-// gathers from the tile slab.  Warps never wait for each other.  Modes: SpMM (+ p.q partials), SpMM
-// adding into its output (the second and later column slabs of the matrix), forward solve, backward solve.
+// gathers from the tile slab.  Warps never wait for each other.  The Laplacian product (k_spmm) works on such
+// chunks too; the modes here are the forward solve, the backward solve, and the forward solve of the last level with that
+// level's backward step.
 enum { M_FWD = 1, M_BWD = 2, M_FWD_LAST = 4 };
 constexpr int CH_THREADS = 256;
 constexpr int CH_WARPS = CH_THREADS / 32;
@@ -916,8 +917,8 @@ __global__ void __launch_bounds__(CH_THREADS, MINB)
 // A warp's item is a chunk (as above) or a segment of CHUNK_CAP entries of a longer row.  A segment's sums go to
 // lpart[segment][column], and k_spmm_long adds a row's segments up: a hub's row, walked by one warp, kept a whole launch
 // waiting.  Where most rows are that long, lpart holds some tiles' columns only and a product is launched in groups of
-// tiles (SpmmPlan::group).  The lanes of a row have eight gathers in flight, its last entries (under predicates) among them, in four
-// accumulators: a grid's row of seven entries costs one gather latency, where a loop over the last three added three.
+// tiles (SpmmPlan::group).  The lanes of a row have eight gathers in flight, its last entries (under predicates) among them,
+// in four accumulators: a grid's row of seven entries costs one gather latency, where a loop over the last three added three.
 // Bound by random 256-byte row gathers through L2 (51 GB in 5.25 ms at ER n = 250,000).  Measured on B200, one FP64 product,
 // with the long rows walked whole and serial last entries -> here: R-MAT n = 24,281, 883K entries, 2693 columns 4.21 ->
 // 1.78 ms; 3-D grid n = 80,840, 1085 columns 1.05 -> 0.57; ER n = 250,000, degree 20, 1194 columns 6.4 -> 5.25; ER n = 1M, 80
