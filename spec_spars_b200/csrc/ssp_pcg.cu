@@ -25,6 +25,7 @@
 
 #include <functional>
 #include <optional>
+#include <type_traits>
 
 #include "ssp_internal.cuh"
 
@@ -919,9 +920,9 @@ __global__ void __launch_bounds__(CH_THREADS, MINB)
 // waiting.  Where most rows are that long, lpart holds some tiles' columns only and a product is launched in groups of
 // tiles (SpmmPlan::group).  The lanes of a row have eight gathers in flight, its last entries (under predicates) among them,
 // in four accumulators: a grid's row of seven entries costs one gather latency, where a loop over the last three added three.
-// Bound by random 256-byte row gathers through L2 (51 GB in 5.25 ms at ER n = 250,000).  Measured on B200, one FP64 product,
+// Bound by random 256-byte row gathers through L2 (51 GB in 5.1 ms at ER n = 250,000).  Measured on B200, one FP64 product,
 // with the long rows walked whole and serial last entries -> here: R-MAT n = 24,281, 883K entries, 2693 columns 4.21 ->
-// 1.78 ms; 3-D grid n = 80,840, 1085 columns 1.05 -> 0.57; ER n = 250,000, degree 20, 1194 columns 6.4 -> 5.25; ER n = 1M, 80
+// 1.78 ms; 3-D grid n = 80,840, 1085 columns 1.05 -> 0.58; ER n = 250,000, degree 20, 1194 columns 6.4 -> 5.1; ER n = 1M, 80
 // columns 2.70 -> 2.10.  FP32 (spmm_row_pair) 3.08 -> 2.37 ms at ER n = 229,373, 1185 columns.  Slower: 16-column halves of a
 // tile, whose gathered rows then fit L2 (2.89 against 2.75 ms at ER n = 1M); FP64 in 16-byte pieces the same way (6.2 ms
 // against 5.06 at ER n = 250,000); FP32 with 3, 5 or 6 pairs in flight (2.67, 2.90, 2.98) and a half-warp per row (3.83).
@@ -936,11 +937,12 @@ struct SpmmItems {
     const int32_t* lrow = nullptr;    // rows of more than CHUNK_CAP entries
     const int32_t* lseg = nullptr;    // nlong + 1 first segments
 };
-// Up to SPMM_SEG entries of a row are summed in four chains, a longer row segment by segment.  Rows of 100 to 256 entries in
-// four chains throughout (FP32: two) were rounded 1.2 to 1.3 (1.6 to 1.8) times worse than in the eight of a lane per value;
-// here it is 0.86 to 0.97 (1.02 to 1.04) times.  The products take 1.65 -> 1.78 ms (R-MAT as above), 5.09 -> 5.25 (ER
-// n = 250,000), 0.58 -> 0.57 (3-D grid); eight chains, whose registers cost gathers in flight, made the whole ER call 230 ms
-// instead of 189.
+// Up to SPMM_SEG entries of a row are summed in four chains; where rows are longer on average (SpmmPlan::segs), segment by
+// segment.  Rows of 100 to 256 entries in four chains throughout (FP32: two) were rounded 1.2 to 1.3 (1.6 to 1.8) times worse
+// than in the eight of a lane per value; in segments it is 0.86 to 0.97 (1.02 to 1.04) times, and shorter rows are the same.
+// The products take 1.65 -> 1.78 ms (R-MAT as above) and 2.05 -> 2.13 (ER n = 20,000, degree 200); with segments on ER n = 1M,
+// degree 20, 1327 columns, one took 32.5 ms instead of 30.7.  Eight chains, whose registers cost gathers in flight, made a
+// whole call on ER n = 250,000 230 ms instead of 189.
 constexpr int SPMM_SEG = 32;
 template <class T>
 __device__ __forceinline__ T spmm_seg(const int32_t* si, const T* sv, int32_t q, int32_t q1, const T* xt) {
@@ -962,9 +964,9 @@ __device__ __forceinline__ T spmm_seg(const int32_t* si, const T* sv, int32_t q,
     }
     return (a[0] + a[1]) + (a[2] + a[3]);
 }
-template <class T>
+template <class T, bool SEGS>
 __device__ __forceinline__ T spmm_row(const int32_t* si, const T* sv, int32_t q, int32_t q1, const T* xt) {
-    if (q1 - q <= SPMM_SEG) return spmm_seg<T>(si, sv, q, q1, xt);
+    if (!SEGS || q1 - q <= SPMM_SEG) return spmm_seg<T>(si, sv, q, q1, xt);
     T tot = 0;
     for (; q < q1; q += SPMM_SEG) tot += spmm_seg<T>(si, sv, q, min(q + SPMM_SEG, q1), xt);
     return tot;
@@ -1006,8 +1008,9 @@ __device__ __forceinline__ float2 spmm_row_pair(const int32_t* si, const float* 
     return a;
 }
 
-// W: columns per warp row (TILE, or 8 when at most 8 are real); ACC adds into q (the second and later column slabs)
-template <class T, int W, bool ACC>
+// W: columns per warp row (TILE, or 8 when at most 8 are real); ACC adds into q (the second and later column slabs); SEGS: rows
+// are summed in segments
+template <class T, int W, bool ACC, bool SEGS>
 __global__ void __launch_bounds__(CH_THREADS, 6)
     k_spmm(int64_t n, SpmmItems S, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
            const T* __restrict__ val, const T* __restrict__ p, T* __restrict__ q, int64_t ld, T* __restrict__ lpart,
@@ -1071,7 +1074,7 @@ __global__ void __launch_bounds__(CH_THREADS, 6)
             const int64_t row = r0 + rr;
             const bool on = row_on(ra, row, t);
             const int32_t q0 = sp[rr], q1 = on && t * TILE + col < kcols ? sp[rr + 1] : q0;
-            T acc = spmm_row<T>(si, sv, q0, q1, xt + col);
+            T acc = spmm_row<T, SEGS>(si, sv, q0, q1, xt + col);
             if (!on) continue;
             if (seg) {
                 lpart[(int64_t)c * lld + t * TILE + col] = acc;
@@ -1898,6 +1901,7 @@ struct SpmmPlan {
     unsigned long_blocks = 0;     // x blocks of k_spmm_long for the last slab (p.q partials follow the grid's)
     int nparts = 0;               // partials of p.q per column
     int launches = 0;             // of one product
+    bool segs = false;            // rows (their share of a slab) hold more than SPMM_SEG entries on average
     // Sums of the long rows' segments (both precisions), for `group` tiles at a time: as many as fit half an n x ld block,
     // one at least.  At 1000 entries a row the segments of all columns would be five blocks beside the solve's six.
     double* lpart = nullptr;
@@ -2032,6 +2036,7 @@ static SpmmPlan make_spmm_plan(Context& C, int64_t n, const int64_t* lap_ptr, co
     const int32_t nl = A.items[m - 1].nlong;
     A.long_blocks = nl ? (unsigned)std::min(ceil_div(nl, CH_WARPS), 64) : 0;
     A.nparts = bx + (int)A.long_blocks;
+    A.segs = A.nnz > (int64_t)SPMM_SEG * n * m;
     const int ntiles = (int)(ld / TILE);
     A.group = ntiles;
     if (most_seg) {
@@ -2053,8 +2058,12 @@ static void launch_spmm(Context& C, int64_t n, const SpmmPlan& A, const T* aval,
         const SpmmItems& I = A.items[b];
         const int64_t* ptr = A.ptr + (int64_t)b * n;
         double* part = dot && b == A.nslabs - 1 ? A.part : nullptr;
-        auto kern = narrow ? (b == 0 ? k_spmm<T, NARROW_W, false> : k_spmm<T, NARROW_W, true>)
-                           : (b == 0 ? k_spmm<T, TILE, false> : k_spmm<T, TILE, true>);
+        auto pick = [&](auto segs) {
+            constexpr bool S = decltype(segs)::value;
+            return narrow ? (b == 0 ? k_spmm<T, NARROW_W, false, S> : k_spmm<T, NARROW_W, true, S>)
+                          : (b == 0 ? k_spmm<T, TILE, false, S> : k_spmm<T, TILE, true, S>);
+        };
+        auto kern = A.segs ? pick(std::true_type()) : pick(std::false_type());
         const int ntiles = (int)A.grid.y, group = I.nlong ? A.group : ntiles;
         const int64_t lld = (int64_t)A.group * TILE;
         const unsigned lx = part ? A.long_blocks : (unsigned)std::min(ceil_div(I.nlong, CH_WARPS), 64);

@@ -32,7 +32,7 @@ def test_partial_sums_take_half_a_block_at_most(ssp):
 
 
 @pytest.mark.parametrize("precision", [0, 1])
-@pytest.mark.parametrize("k", [33, 64, 200])
+@pytest.mark.parametrize("k", [5, 33, 64, 200])
 def test_solution_has_the_residual_asked_for(ssp, ctx, k, precision):
     G = _dense(ssp)
     L = ssp.stage_graph(ctx, G)[1]
