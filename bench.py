@@ -121,9 +121,9 @@ def peaks():
 
 
 # DRAM bytes per (Laplacian nonzero, 32-column tile) of one FP64 SpMM launch at ER n=1M, from the ncu
-# capture of a one-tile solve of that graph (profiles/k_chunked_spmm_er_n1M_k32.md: 4.123 GB read + 0.287 GB
+# capture of a one-tile solve of that graph (profiles/k_spmm_er_n1M_k32.md: 4.072 GB read + 0.254 GB
 # written for nnz(L_G) = 21.003M nonzeros x 1 tile); every tile of a full launch does the same work
-SPMM_TRAFFIC_PER_NNZ_TILE = 4.4093e9 / 21.003e6
+SPMM_TRAFFIC_PER_NNZ_TILE = 4.3268e9 / 21.003e6
 SPMM_TILE = 32
 
 

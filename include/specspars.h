@@ -295,8 +295,8 @@ int ssp_shard_finish(ssp_context* ctx, const ssp_csc* graph, const ssp_params* p
  * own stream and workspace, so admitted requests overlap on the device.  A free slot admits the oldest pending
  * request whose estimated device footprint (ssp_request_footprint) fits beside those in flight within
  * hbm_budget_bytes (a younger one may go first while the oldest has waited less than 500 ms; after that the
- * oldest is admitted first); a request whose footprint alone exceeds the budget is refused at submit
- * (SSP_ERR_CAPACITY).  The slot then adds pending requests that can share its run (same epsilon, factor
+ * oldest is admitted first); a request that exceeds the budget alone, without the buffers that a call can do without,
+ * is refused at submit (SSP_ERR_CAPACITY).  The slot then adds pending requests that can share its run (same epsilon, factor
  * seed, precision, PCG options and reweighting, and dense_threshold = 0), up to max_batch
  * and its share of the budget, and runs them with ssp_sparsify_batch; other requests run exactly
  * ssp_sparsify, so their result is the same as a lone call's.  Results are collected once with ssp_wait /

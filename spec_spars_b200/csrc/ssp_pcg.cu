@@ -923,9 +923,10 @@ __global__ void __launch_bounds__(CH_THREADS, MINB)
 // Bound by random 256-byte row gathers through L2 (51 GB in 5.1 ms at ER n = 250,000).  Measured on B200, one FP64 product,
 // with the long rows walked whole and serial last entries -> here: R-MAT n = 24,281, 883K entries, 2693 columns 4.21 ->
 // 1.78 ms; 3-D grid n = 80,840, 1085 columns 1.05 -> 0.58; ER n = 250,000, degree 20, 1194 columns 6.4 -> 5.1; ER n = 1M, 80
-// columns 2.70 -> 2.10.  FP32 (spmm_row_pair) 3.08 -> 2.37 ms at ER n = 229,373, 1185 columns.  Slower: 16-column halves of a
+// columns 2.70 -> 2.10.  FP32 (spmm_row_pair) 2.98 -> 2.45 ms at ER n = 229,373, 1185 columns.  Slower: 16-column halves of a
 // tile, whose gathered rows then fit L2 (2.89 against 2.75 ms at ER n = 1M); FP64 in 16-byte pieces the same way (6.2 ms
-// against 5.06 at ER n = 250,000); FP32 with 3, 5 or 6 pairs in flight (2.67, 2.90, 2.98) and a half-warp per row (3.83).
+// against 5.06 at ER n = 250,000); FP32 with 3, 5 or 6 pairs in flight (2.67, 2.90, 2.98 against 2.37 with one chain a
+// half-warp) and a half-warp per row (3.83).
 // Six resident blocks per SM (five ran slower: FP32 29.7 against 22.6 ms at ER n = 1M, 1327 columns).
 struct SpmmItems {
     const int32_t* chunks = nullptr;  // nchunks + 1 row starts (a row of more than CHUNK_CAP entries is skipped there)
