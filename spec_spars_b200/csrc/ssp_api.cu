@@ -321,7 +321,7 @@ static void sparsify_impl(Context& C, const ssp_csc* graph, const ssp_params* pr
     // one shard of columns per call; otherwise all columns at once, or batches sized after the factorization
     const bool can_batch = !finish_only && !(sh && sh->sq_out);
     const int32_t forced = can_batch ? forced_batch(kl) : 0;
-    const bool batched = can_batch && ((forced > 0 && forced < kl) || !columns_fit(C, G, kl, prm->precision));
+    bool batched = can_batch && ((forced > 0 && forced < kl) || !columns_fit(C, G, kl, prm->precision));
     int32_t kb = kl;
     double* Y = nullptr;
     if (!finish_only && !batched) {
@@ -368,30 +368,49 @@ static void sparsify_impl(Context& C, const ssp_csc* graph, const ssp_params* pr
     const bool fuse = !(fe && fe[0] == '0');
     double* d2 = (finish_only || !fuse) ? nullptr
                  : (sh && sh->sq_out) ? sh->sq_out : C.ws.get_t<double>("sp_d2", G.m + 1);
-    double* d2sum = batched ? C.ws.get_t<double>("sp_d2", G.m + 1) : nullptr;  // batches: their squared sums
-    if (batched) {
-        kb = forced > 0 ? forced : batch_after_factor(C, G, kl, prm->precision);
-        Y = C.ws.get_t<double>("sp_Y", (size_t)n * tile_ld(kb));
-        sketch_device(C, SG, kb, scale, prm->sketch_seed, prm->sketch_uniform, Y, tile_ld(kb), 1, 0);
+    double* d2sum = nullptr;  // batches: their squared sums
+    if (!finish_only && !batched) {
+        try {
+            pcg_device(C, n, G.lap_ptr, G.lap_idx, G.lap_val, F, Y, kb, &Zt, po, rep, nullptr, nullptr, G.lap_eid, d2);
+        } catch (const Error& e) {
+            if (!can_batch || forced > 0 || e.code != SSP_ERR_NOMEM || kl <= SSP_TILE) throw;
+            batched = true;  // all columns at once took more than was expected
+        }
     }
-    if (!finish_only)
-        pcg_device(C, n, G.lap_ptr, G.lap_idx, G.lap_val, F, Y, kb, &Zt, po, rep, nullptr, nullptr, G.lap_eid, d2);
     if (batched) {
-        // the batches' squared diff norms accumulate tile by tile into d2sum: fused, they continue the single
-        // pass's order exactly; from the separate pass, each batch's partial sum is added
+        // The batches' squared diff norms accumulate tile by tile into d2sum: fused, they continue the single
+        // pass's order exactly; from the separate pass, each batch's partial sum is added.  A batch that runs out of memory
+        // leaves them as they were (the final product is the last it does) and is taken again with fewer columns; the first
+        // time, the blocks of earlier calls, which the estimate counts as free whatever their sizes, are given back as well.
+        d2sum = C.ws.get_t<double>("sp_d2", G.m + 1);
         double* part = C.ws.get_t<double>("sp_d2part", G.m + 1);
-        if (!rep.diff_fused) diff_sq_device(C, G.m, G.v1, G.v2, Zt, kb, n, d2sum);
-        for (int32_t c0 = kb; c0 < kl; c0 += kb) {
+        kb = forced > 0 ? forced : batch_after_factor(C, G, kl, prm->precision);
+        bool given_back = false;
+        for (int32_t c0 = 0; c0 < kl;) {
             const int32_t kc = std::min(kb, kl - c0);
-            sketch_device(C, SG, kc, scale, prm->sketch_seed, prm->sketch_uniform, Y, tile_ld(kc), 1, c0);
             PcgReport rb;
-            pcg_device(C, n, G.lap_ptr, G.lap_idx, G.lap_val, F, Y, kc, &Zt, po, rb, nullptr, nullptr, G.lap_eid,
-                       fuse ? d2sum : nullptr, true);
-            if (!rb.diff_fused) {
-                diff_sq_device(C, G.m, G.v1, G.v2, Zt, kc, n, part);
-                add_device(C, G.m, part, d2sum);
+            try {
+                Y = C.ws.get_t<double>("sp_Y", (size_t)n * tile_ld(kc));
+                sketch_device(C, SG, kc, scale, prm->sketch_seed, prm->sketch_uniform, Y, tile_ld(kc), 1, c0);
+                pcg_device(C, n, G.lap_ptr, G.lap_idx, G.lap_val, F, Y, kc, &Zt, po, rb, nullptr, nullptr, G.lap_eid,
+                           fuse ? d2sum : nullptr, c0 > 0);
+            } catch (const Error& e) {
+                if (e.code != SSP_ERR_NOMEM || forced > 0 || (given_back && kc <= SSP_TILE)) throw;
+                if (given_back) kb = std::max<int32_t>(SSP_TILE, kc / 2 / SSP_TILE * SSP_TILE);
+                C.ws.release_prefix("sp_Y");
+                C.ws.release_prefix("pcg");
+                SSP_CUDA(cudaStreamSynchronize(C.stream));
+                if (!given_back) kb = batch_after_factor(C, G, kl, prm->precision);
+                given_back = true;
+                continue;
             }
-            merge_report(rep, rb, c0, kc);
+            if (!rb.diff_fused) {
+                diff_sq_device(C, G.m, G.v1, G.v2, Zt, kc, n, c0 ? part : d2sum);
+                if (c0) add_device(C, G.m, part, d2sum);
+            }
+            if (c0) merge_report(rep, rb, c0, kc);
+            else rep = rb;
+            c0 += kc;
         }
     }
     T.mark();  // 4

@@ -160,6 +160,11 @@ public:
         bufs_[name] = {p, bytes, false};
         return p;
     }
+    // the buffers named p..., for good
+    void release_prefix(const std::string& p) {
+        for (auto it = bufs_.lower_bound(p); it != bufs_.end() && it->first.compare(0, p.size(), p) == 0; it = bufs_.erase(it))
+            cudaFreeAsync(it->second.ptr, stream_);
+    }
     void release() {
         for (auto& kv : bufs_) cudaFreeAsync(kv.second.ptr, stream_);
         bufs_.clear();

@@ -2500,9 +2500,13 @@ void pcg_device(Context& C, int64_t n, const int64_t* lap_ptr, const int32_t* la
     double* z = W.get_t<double>("pcg_z", total);
     double* p = W.get_t<double>("pcg_p", total);
     double* q = W.get_t<double>("pcg_q", total);
+    // (pcg_solve's small buffers, before the optional ones are in use)
+    W.get_t<int32_t>("pcg_loop_it", 1);
     // graphs solved at once (one segment: a single graph)
     SegDev G;
     PcgSegments* segs = opt.segs;
+    if (opt.history || (segs && segs->record_history))
+        W.get_t<double>("pcg_hist", (size_t)opt.max_iters * ((segs ? segs->k.size() : 1) + 1));
     if (segs) {
         const int32_t nseg = (int32_t)segs->k.size();
         SSP_REQUIRE(nseg >= 1 && (int64_t)segs->row0.size() == nseg + 1 && segs->row0.front() == 0 &&
